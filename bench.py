@@ -623,7 +623,7 @@ def run_ours(args) -> None:
         "config": workload_config(n),
         "ms_per_iteration": round(ms_step_max, 5), "word_bytes": word,
         "iteration": "one FP32 PT sweep of the FP32+FP64 defect-correction solve",
-        "roofline": {"bound": "hbm", "kernel": "k_fused_tma (FP32 PT sweep, correction problem)",
+        "roofline": {"bound": "hbm", "kernel": "k_sweep (FP32 PT sweep, correction problem)",
                      "achieved": round(aeff / (out["kernel_ms"] * 1e-3) / 1e9, 3), "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": round(aeff / (out["kernel_ms"] * 1e-3) / 1e9 / pk["hbm_gbs"], 4),
                      "traffic": args.traffic, "peak_source": pk["source"],

@@ -64,6 +64,36 @@ __device__ __forceinline__ CellD<T> cell_strain(const Geo<T>& geo, T d1, T d2, T
     return cell_strain_m<T, G>(cell_metric_t<T, G>(geo, d2, d3, i, j), d1, v1m, v1p, v2m, v2p, v3m, v3p);
 }
 
+// normal-velocity ghost that makes a boundary cell divergence-free (far-field stress faces, the
+// free-surface top): the face normal to axis D on side 0 / 1; the entry of the ghost itself among
+// the six face velocities is not read.  Written with explicit fma, so that the BC kernels and the
+// sweep that evaluates the ghost where it reads it get the same bits.
+__device__ __forceinline__ double gdiv(double a, double b) { return a / b; }
+__device__ __forceinline__ float gdiv(float a, float b) {  // quotient by the reciprocal and one residual step
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    const float q = a * r;
+    return fmaf(fmaf(-b, q, a), r, q);
+}
+template <typename T, int G, int D>
+__device__ __forceinline__ T div_ghost(const CellMetric<T>& m, T d1, int side, T v1m, T v1p, T v2m, T v2p, T v3m, T v3p) {
+    const T h = T(0.5), sgn = side == 0 ? T(-1) : T(1);
+    if (D == 0) {
+        const T vin = side == 0 ? v1p : v1m;
+        const T a = fma(m.a3, v3p - v3m, fma(m.c2, h * (v2m + v2p), vin * fma(h, m.c1, -sgn * d1)));
+        return gdiv(-fma(m.a2, v2p - v2m, a), fma(sgn, d1, h * m.c1));
+    }
+    const T avx = h * (v1m + v1p);
+    if (D == 1) {
+        const T vin = side == 0 ? v2p : v2m;
+        const T a = fma(m.a3, v3p - v3m, fma(m.c1, avx, vin * fma(h, m.c2, -sgn * m.a2)));
+        return gdiv(-fma(d1, v1p - v1m, a), fma(sgn, m.a2, h * m.c2));
+    }
+    const T vin = side == 0 ? v3p : v3m;
+    const T a = fma(m.a2, v2p - v2m, fma(m.c1, avx, fma(m.c2, h * (v2m + v2p), vin * (-sgn * m.a3))));
+    return gdiv(-fma(d1, v1p - v1m, a), sgn * m.a3);
+}
+
 // metric factors of the three edge stencils at index (i, j)
 template <typename T>
 struct EdgeMetric {

@@ -415,29 +415,17 @@ __device__ __forceinline__ void bc_body(const KP<T>& p, const BcStage& st, int h
                 }
                 default: {  // BC_STRESS: normal ghost of V1 (D == 0), V2 (D == 1) or V3 (D == 2) from div V = 0 in the boundary cell
                     const int cellb = side == 0 ? 0 : ext[D] - 2;        // boundary cell index along D
-                    // boundary cell (its tangential velocities: at the ghost, or at the source of its copy)
-                    const int cc = base + (op.kind == BC_STRESS_SRC ? cellb + (side == 0 ? 1 : -1) : cellb) * stride[D];
+                    // tangential velocities of the boundary cell: at the ghost, or at the source of its copy
+                    const int ct = base + (op.kind == BC_STRESS_SRC ? cellb + (side == 0 ? 1 : -1) : cellb) * stride[D];
                     const int i = (D == 0) ? cellb : u;
                     const int j = (D == 1) ? cellb : (du == 1 ? u : v);
                     const CellMetric<T> m = cell_metric<T, G>(p, i, j);
-                    const T sgn = side == 0 ? T(-1) : T(1);
-                    const T avx = (p.V1[cc] + p.V1[cc + 1]) * T(0.5);
-                    const T vin = A[ci];
-                    T A0, B;
-                    if (D == 0) {  // V1 ghost of the free-surface top (or bottom) face
-                        const T avy = (p.V2[cc] + p.V2[cc + sy]) * T(0.5);
-                        A0 = p.d1 * (-sgn) * vin + T(0.5) * m.c1 * vin + m.a2 * (p.V2[cc + sy] - p.V2[cc]) + m.a3 * (p.V3[cc + sz] - p.V3[cc]) +
-                             m.c2 * avy;
-                        B = p.d1 * sgn + T(0.5) * m.c1;
-                    } else if (D == 1) {
-                        A0 = p.d1 * (p.V1[cc + 1] - p.V1[cc]) + m.a3 * (p.V3[cc + sz] - p.V3[cc]) + m.c1 * avx + m.a2 * (-sgn) * vin + m.c2 * T(0.5) * vin;
-                        B = m.a2 * sgn + T(0.5) * m.c2;
-                    } else {
-                        const T avy = (p.V2[cc] + p.V2[cc + sy]) * T(0.5);
-                        A0 = p.d1 * (p.V1[cc + 1] - p.V1[cc]) + m.a2 * (p.V2[cc + sy] - p.V2[cc]) + m.c1 * avx + m.c2 * avy + m.a3 * (-sgn) * vin;
-                        B = m.a3 * sgn;
-                    }
-                    val = -A0 / B;
+                    if (D == 0)
+                        val = div_ghost<T, G, 0>(m, p.d1, side, A[ci], A[ci], p.V2[ct], p.V2[ct + sy], p.V3[ct], p.V3[ct + sz]);
+                    else if (D == 1)
+                        val = div_ghost<T, G, 1>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], A[ci], A[ci], p.V3[ct], p.V3[ct + sz]);
+                    else
+                        val = div_ghost<T, G, 2>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], p.V2[ct], p.V2[ct + sy], A[ci], A[ci]);
                     break;
                 }
             }

@@ -29,7 +29,7 @@
 
 #include "sph_pt.cuh"
 #include "sph_fused.cuh"
-#include "sph_sweep_x2.cuh"
+#include "sph_sweep.cuh"
 #include "sph_adjoint.cuh"
 #include "sph_advect.cuh"
 #include "sph_batch.cuh"
@@ -91,11 +91,13 @@ struct Ctx {
     unsigned long long* hred = nullptr;  // pinned host copy
     std::vector<BcStage> bc;      // BC program: ghost-velocity stages in the reference order (the adjoint transposes these)
     std::vector<BcStage> bc_run;  // the program launched by launch_bc: bc, or an equivalent one with fewer stages
-    // the first stage of bc_run in the homogeneous case as factors of the interior neighbour
-    // (ghost = xg[f] x neighbour on both x1 faces, field f in bit f of xg_mask); 0: not of that form
-    int xg_mask = 0;
-    float xg[3] = {0.f, 0.f, 0.f};
-    bool xg_fuse = true;  // the correction sweep writes those ghosts (SPH_NO_XGHOST=1: the BC stage does)
+    // the homogeneous program in closed form for the correction sweep (SweepOut): set where every
+    // ghost is a multiple of its interior neighbour or divergence-free; SPH_NO_XGHOST=1: not used,
+    // the BC launches follow each sweep
+    bool ghost_fuse = true;
+    int ghost_gmask = 0, ghost_smask = 0;
+    float ghost_gf[9] = {};
+    bool ghost_stored = false;  // the next sweep reads the stored ghosts (after sph_corr_set)
     double cur_n = 1.0;
     double f_scale = 1.0;
     double last_ms = 0.0;
@@ -114,12 +116,11 @@ struct Ctx {
     float* warm_key[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     int warm_len = 0;
     bool use_graphs = true;
-    // TMA tensor maps of the correction sweep, one set per ping-pong arrangement
-    CUtensorMap* d_maps = nullptr;       // [2][TM_COUNT] in device memory
-    float* map_key[2] = {nullptr, nullptr};  // V1 buffer of the arrangement a set was built for
+    // TMA tensor maps of the sweep, one set per arrangement of the ping-pong and η buffers
+    CUtensorMap* d_maps = nullptr;       // [4][SM_COUNT] in device memory
+    float* map_key[4][2] = {};           // V1 and η buffers of the arrangement a set was built for
     int* d_err = nullptr;                // set by a kernel whose bounded wait ran out
     bool use_tma = true;
-    bool use_x2 = false;  // TMA sweep with two points per thread (k_sweep_x2) instead of k_fused_tma
     bool use_pdl = true;  // sweep and BC kernels launched with a programmatic dependency (pdl_enter)
     bool fused = true;   // FP32 sweeps use the fused kernel
     int fused_chunk = 0; // planes per block of the fused sweep (0: chosen by fused_chunk())
@@ -244,32 +245,50 @@ BcStage stage(int dim, std::initializer_list<BcOp> ops) {
     return s;
 }
 
+// the homogeneous form of c.bc in closed form (NEG -1, COPY +1, ZERO / LIN 0, LIN2M -1; STRESS:
+// divergence-free), where the stages run axis by axis and set each ghost once
+void build_ghosts(Ctx& c) {
+    c.ghost_gmask = c.ghost_smask = 0;
+    if (!c.ghost_fuse) return;
+    int gmask = 0, smask = 0, seen = 0, dim = 0;
+    float gf[9] = {};
+    for (const BcStage& st : c.bc) {
+        if (st.dim < dim) return;
+        dim = st.dim;
+        for (int i = 0; i < st.nops; ++i) {
+            const BcOp& op = st.op[i];
+            float f = 0.f;
+            bool free = false;
+            switch (op.kind) {
+                case BC_NEG: case BC_LIN2M: f = -1.f; break;
+                case BC_COPY: f = 1.f; break;
+                case BC_ZERO: case BC_LIN: break;
+                case BC_STRESS: free = true; break;
+                default: return;
+            }
+            if (free && op.field != dim) return;
+            for (int side = 0; side < 2; ++side) {
+                if (op.side >= 0 && op.side != side) continue;
+                const int bit = 1 << (6 * dim + 2 * op.field + side);
+                if (seen & bit) return;
+                seen |= bit;
+                if (free) smask |= 1 << (2 * dim + side);
+                else { gmask |= bit; gf[3 * dim + op.field] = f; }
+            }
+        }
+    }
+    if (seen != (1 << 18) - 1) return;
+    c.ghost_gmask = gmask;
+    c.ghost_smask = smask;
+    for (int i = 0; i < 9; ++i) c.ghost_gf[i] = gf[i];
+}
+
 int build_bc_program(Ctx& c);
 int build_bc(Ctx& c) {
     const int rc = build_bc_program(c);
     if (rc != SPH_OK) return rc;
     if (c.bc_run.empty()) c.bc_run = c.bc;
-    // homogeneous x1-face stage as factors (NEG -1, COPY +1, ZERO / LIN 0, LIN2M -1)
-    c.xg_mask = 0;
-    const BcStage& s0 = c.bc_run[0];
-    int mask = 0;
-    float xg[3] = {0.f, 0.f, 0.f};
-    bool ok = s0.dim == 0 && c.xg_fuse;
-    for (int i = 0; ok && i < s0.nops; ++i) {
-        const BcOp& op = s0.op[i];
-        if (op.field < 0 || op.field > 2 || (mask >> op.field & 1) || op.side >= 0) { ok = false; break; }
-        switch (op.kind) {
-            case BC_NEG: case BC_LIN2M: xg[op.field] = -1.f; break;
-            case BC_COPY: xg[op.field] = 1.f; break;
-            case BC_ZERO: case BC_LIN: xg[op.field] = 0.f; break;
-            default: ok = false;
-        }
-        mask |= 1 << op.field;
-    }
-    if (ok && mask) {
-        c.xg_mask = mask;
-        for (int i = 0; i < 3; ++i) c.xg[i] = xg[i];
-    }
+    build_ghosts(c);
     return SPH_OK;
 }
 
@@ -332,8 +351,8 @@ int build_bc_program(Ctx& c) {
 }
 
 template <typename T, int G>
-void launch_bc(Ctx& c, KP<T>& p, int homog, int first = 0) {
-    for (size_t i = first; i < c.bc_run.size(); ++i) {
+void launch_bc(Ctx& c, KP<T>& p, int homog) {
+    for (size_t i = 0; i < c.bc_run.size(); ++i) {
         const BcStage& st = c.bc_run[i];
         int eu = st.dim == 0 ? c.d.n2 + 1 : c.d.n1 + 1;
         int ev = st.dim == 2 ? c.d.n2 + 1 : c.d.n3 + 1;
@@ -542,65 +561,156 @@ void swap_state(State<float>& s) {
     for (int i = 0; i < 10; ++i) std::swap(s.f[a[i]], s.f[b[i]]);
 }
 
+dim3 sweep_grid(const Dims& d, int chunk) { return dim3((d.n1 + SWX - 1) / SWX, (d.n2 + SWY - 1) / SWY, (d.n3 + chunk - 1) / chunk); }
+
 // x3 chunk lengths picked by sph_autotune, per (geometry, n1, n2, n3), shared by every context
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, int> g_tuned_chunk;
 
 // x3 chunk length of the fused sweep.  Each block marches over one chunk of
-// planes and pays about two planes more than it owns (the halo plane below the
-// chunk and the pipeline fill), while the hardware scheduler balances the SMs
-// only to within one block at the end of the launch.  The time model
-// (k + 2.5) * (blocks / slots + 0.7), slots = resident blocks on the device, picks
-// the chunk among 4..24 planes.  Measured on a GB300, its pick is the fastest
-// chunk at 63^3 and within 1 % of it at 255^3 and 5 % at 127^3, where wave
-// quantisation makes the ranking irregular (sph_autotune measures instead).
+// planes and pays for more planes than it owns (the halo plane below the chunk and
+// the pipeline fill), while the hardware scheduler balances the SMs only to within
+// one block at the end of the launch.  The time model (k + 1.4) * (n / 2 + 0.7), n =
+// blocks on the fullest SM (two are resident), picks the chunk among 1..24 planes; an
+// odd n counts an eighth more, as the last block alone on its SM does not run at twice
+// the speed.
+// Measured on a GB300 (us per sweep, chunks of 1 / 2 / 3 / 4 / 8 / 16 planes): 47 x 31 x 39
+// 7.2 / 8.4 / 10.5 / 13.0 / 22.9 / 42.9, 63^3 17.2 / 17.8 / 16.2 / 16.2 / 28.0 / 52.7,
+// 131 x 117 x 101 80 / 65 / 59 / 58 / 59 / 61, 255^3 - / - / - / - / 345 / 348: the rule's
+// picks (1, 3, 4, 16) are within 2 % of the best.  sph_autotune measures instead.
 int fused_chunk(const Ctx& c) {
     if (c.fused_chunk > 0) return c.fused_chunk;
-    const double xy = (double)((c.d.n1 + FTX - 1) / FTX) * ((c.d.n2 + FTY - 1) / FTY);
-    const double slots = c.fused_slots > 0 ? c.fused_slots : 456.0;
-    int best = 4;
+    const dim3 tiles = sweep_grid(c.d, c.d.n3);
+    const double xy = (double)tiles.x * tiles.y;
+    const double sms = c.fused_slots > 0 ? 0.5 * c.fused_slots : 152.0;
+    int best = 1;
     double best_t = 1e300;
-    for (int k : {4, 6, 8, 12, 16, 24}) {
+    for (int k : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
         const double blocks = xy * ((c.d.n3 + k - 1) / k);
-        const double t = (k + 2.5) * (blocks / slots + 0.7);
+        const int n = (int)std::ceil(blocks / sms);
+        const double t = (k + 1.4) * (0.5 * n + (n & 1 ? 0.125 : 0.0) + 0.7);
         if (t < best_t) { best_t = t; best = k; }
         if (k >= c.d.n3) break;
     }
     return best;
 }
 
-template <int G, int MODE>
-void set_tma_attr() {
-    cudaFuncSetAttribute(k_fused_tma<G, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_tma_smem_bytes());
+// ---------------------------------------------------------------------------
+// TMA tensor maps over the padded box of FP32 fields
+PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {  // looked up once, thread-safe
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+        return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
+    }();
+    return fn;
 }
 
-template <int G, int MODE>
-void set_fused_attr() {
-    cudaFuncSetAttribute(k_fused<G, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes());
+// nf equally spaced fields of the slab from `base` on; boxes of bx x by entries of one plane of all of them
+bool encode_map(const Ctx& c, CUtensorMap* m, const float* base, int nf, unsigned bx, unsigned by) {
+    auto enc = tma_encoder();
+    if (!enc) return false;
+    cuuint64_t gdim[4] = {(cuuint64_t)c.d.px, (cuuint64_t)c.d.py, (cuuint64_t)c.d.pz, (cuuint64_t)nf};
+    cuuint64_t gstr[3] = {(cuuint64_t)c.d.px * 4, (cuuint64_t)c.d.px * c.d.py * 4, (cuuint64_t)c.d.vol * 4};
+    cuuint32_t box[4] = {bx, by, 1, (cuuint32_t)nf};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), gdim, gstr, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// maps of the current buffer arrangement; returns the device pointer of the set or nullptr
+const CUtensorMap* tma_maps(Ctx& c) {
+    if (!c.use_tma) return nullptr;
+    State<float>& t = c.s32;
+    int slot = 0;
+    for (; slot < 4 && c.map_key[slot][0]; ++slot)
+        if (c.map_key[slot][0] == t.f[F_V1] && c.map_key[slot][1] == t.f[F_ETA]) return c.d_maps + slot * SM_COUNT;
+    if (slot == 4) return nullptr;
+    if (!c.d_maps) {
+        if (cudaMalloc((void**)&c.d_maps, sizeof(CUtensorMap) * 4 * SM_COUNT) != cudaSuccess) { c.use_tma = false; return nullptr; }
+    }
+    if (!c.d_err) {
+        if (cudaMalloc((void**)&c.d_err, sizeof(int)) != cudaSuccess) { c.use_tma = false; return nullptr; }
+        cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream);
+    }
+    CUtensorMap h[SM_COUNT];
+    bool ok = encode_map(c, &h[SM_V], t.f[F_V1], 3, SI_X, SI_Y);
+    ok &= encode_map(c, &h[SM_ETA], t.f[F_ETA], 1, SI_X, SI_Y);
+    ok &= encode_map(c, &h[SM_ETASM], t.f[F_ETA_SM], 1, SI_X, SI_Y);
+    ok &= encode_map(c, &h[SM_P], t.f[F_P], 1, SO_X, SO_Y);
+    ok &= encode_map(c, &h[SM_TAU], t.f[F_T11], 6, SO_X, SO_Y);
+    ok &= encode_map(c, &h[SM_RP], t.f[F_RP], 1, SO_X, SO_Y);
+    ok &= encode_map(c, &h[SM_RHO], t.f[F_RHO], 1, SO_X, SO_Y);
+    ok &= encode_map(c, &h[SM_RV], t.f[F_RV1], 3, SWX, SWY);
+    if (!ok || cudaMemcpy(c.d_maps + slot * SM_COUNT, h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess) {
+        c.use_tma = false;
+        return nullptr;
+    }
+    c.map_key[slot][0] = t.f[F_V1];
+    c.map_key[slot][1] = t.f[F_ETA];
+    return c.d_maps + slot * SM_COUNT;
+}
+
+// build the tensor-map sets of all four arrangements (never inside a graph capture)
+void ensure_tma_maps(Ctx& c) {
+    if (!c.use_tma || !c.fused) return;
+    for (int i = 0; i < 4; ++i) {
+        tma_maps(c);
+        swap_state(c.s32);
+        if (i & 1) std::swap(c.s32.f[F_ETA], c.s32.f[F_ETA_OUT]);
+    }
+}
+
+template <int G>
+void set_sweep_attrs() {
+    const int f = (int)fused_smem_bytes(), w = (int)sweep_smem_bytes();
+    cudaFuncSetAttribute(k_fused<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
+    cudaFuncSetAttribute(k_fused<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
+    cudaFuncSetAttribute(k_sweep<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
+    cudaFuncSetAttribute(k_sweep<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
+    cudaFuncSetAttribute(k_sweep_batch<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
 }
 int set_fused_attrs() {
-    set_fused_attr<SPH, 0>(); set_fused_attr<SPH, 1>();
-    set_fused_attr<CYL, 0>(); set_fused_attr<CYL, 1>();
-    set_fused_attr<CART, 0>(); set_fused_attr<CART, 1>();
-    set_tma_attr<SPH, 1>(); set_tma_attr<CYL, 1>(); set_tma_attr<CART, 1>();
-    cudaFuncSetAttribute(k_fused_tma_batch<SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_tma_smem_bytes());
-    cudaFuncSetAttribute(k_fused_tma_batch<CYL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_tma_smem_bytes());
-    cudaFuncSetAttribute(k_fused_tma_batch<CART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_tma_smem_bytes());
-    cudaFuncSetAttribute(k_sweep_x2<SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_x2_smem_bytes());
-    cudaFuncSetAttribute(k_sweep_x2<CYL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_x2_smem_bytes());
-    cudaFuncSetAttribute(k_sweep_x2<CART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_x2_smem_bytes());
+    set_sweep_attrs<SPH>();
+    set_sweep_attrs<CYL>();
+    set_sweep_attrs<CART>();
     CK(cudaGetLastError());
     return SPH_OK;
 }
 
+// output state and ghosts of a sweep of the current arrangement; fill: the sweep of a correction
+// problem that handles the boundary velocities itself
+SweepOut<float> sweep_out(const Ctx& c, const KP<float>& p, bool fill) {
+    const State<float>& t = c.s32;
+    SweepOut<float> o{};
+    o.P = t.f[F_A_P]; o.V1 = t.f[F_A_V1]; o.V2 = t.f[F_A_V2]; o.V3 = t.f[F_A_V3];
+    o.t11 = t.f[F_A_T11]; o.t22 = t.f[F_A_T22]; o.t33 = t.f[F_A_T33]; o.t12 = t.f[F_A_T12]; o.t13 = t.f[F_A_T13]; o.t23 = t.f[F_A_T23];
+    auto pair = [](float x) { return make_float2(x, x); };
+    o.d1 = pair(p.d1); o.d1q = pair(0.25f * p.d1); o.d2 = pair(p.d2); o.gsc = pair(p.gsc); o.kbc = pair(p.kbc); o.nkbc = pair(-p.kbc);
+    o.vp = pair(0.5f * p.vpdt2); o.third = pair(-1.f / 3.f); o.half = pair(-0.5f);
+    if (fill) {
+        o.gmask = c.ghost_gmask;
+        o.smask = c.ghost_stored ? 0 : c.ghost_smask;
+        for (int i = 0; i < 9; ++i) o.gf[i] = c.ghost_gf[i];
+    }
+    return o;
+}
+
+// new state of the arrangement p reads into the other buffer set: the TMA sweep, or the cp.async
+// one where there are no maps; returns whether boundary velocities are done (o.gmask)
 template <int G, int MODE>
-void launch_fused(Ctx& c, KP<float>& p, State<float>& s) {
-    FusedOut<float> o;
-    o.P = s.f[F_A_P]; o.V1 = s.f[F_A_V1]; o.V2 = s.f[F_A_V2]; o.V3 = s.f[F_A_V3];
-    o.t11 = s.f[F_A_T11]; o.t22 = s.f[F_A_T22]; o.t33 = s.f[F_A_T33]; o.t12 = s.f[F_A_T12]; o.t13 = s.f[F_A_T13]; o.t23 = s.f[F_A_T23];
+bool launch_fused(Ctx& c, const KP<float>& p, bool fill) {
     const int kc = fused_chunk(c);
+    if (const CUtensorMap* maps = tma_maps(c)) {
+        launch_pdl(c.use_pdl, k_sweep<G, MODE>, sweep_grid(c.d, kc), dim3(SW_NT, 1, 1), sweep_smem_bytes(), c.stream, p, sweep_out(c, p, fill), kc, maps, c.d_err);
+        return fill;
+    }
     dim3 grid((c.d.n1 + FTX - 1) / FTX, (c.d.n2 + FTY - 1) / FTY, (c.d.n3 + kc - 1) / kc);
-    k_fused<G, MODE><<<grid, dim3(FNT, 1, 1), fused_smem_bytes(), c.stream>>>(p, o, kc);
+    k_fused<G, MODE><<<grid, dim3(FNT, 1, 1), fused_smem_bytes(), c.stream>>>(p, sweep_out(c, p, false), kc);
+    return false;
 }
 
 // one reference iteration with the fused sweep (FP32)
@@ -608,7 +718,7 @@ template <int G>
 void iterate_fused(Ctx& c, State<float>& s) {
     KP<float> p = make_kp<float>(c, s);
     launch_maxloc<float, G>(c, p);
-    launch_fused<G, 0>(c, p, s);
+    launch_fused<G, 0>(c, p, false);
     swap_state(s);
     KP<float> q = make_kp<float>(c, s);
     if (c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) {
@@ -892,77 +1002,12 @@ int prepare_correction(Ctx& c, const double out[7]) {
     CK(cudaGetLastError());
     c.corr_r0 = std::max(out[0], std::max(out[1], out[2]));
     c.corr_ready = true;
+    c.ghost_stored = false;
     c.stale32 = true;  // the FP32 state no longer mirrors the FP64 state
     return SPH_OK;
 }
 
 // ---------------------------------------------------------------------------
-// TMA tensor maps over the padded box of FP32 fields
-PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
-    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {  // looked up once, thread-safe
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-        return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-    }();
-    return fn;
-}
-
-bool encode_map(const Ctx& c, CUtensorMap* m, const float* base, unsigned bx, unsigned by) {
-    auto enc = tma_encoder();
-    if (!enc) return false;
-    cuuint64_t gdim[3] = {(cuuint64_t)c.d.px, (cuuint64_t)c.d.py, (cuuint64_t)c.d.pz};
-    cuuint64_t gstr[2] = {(cuuint64_t)c.d.px * 4, (cuuint64_t)c.d.px * c.d.py * 4};
-    cuuint32_t box[3] = {bx, by, 1};
-    cuuint32_t es[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), gdim, gstr, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// maps of the current buffer arrangement; returns the device pointer of the set or nullptr
-const CUtensorMap* tma_maps(Ctx& c) {
-    if (!c.use_tma) return nullptr;
-    State<float>& t = c.s32;
-    for (int i = 0; i < 2; ++i)
-        if (c.map_key[i] == t.f[F_V1]) return c.d_maps + i * TM_COUNT;
-    if (!c.d_maps) {
-        if (cudaMalloc((void**)&c.d_maps, sizeof(CUtensorMap) * 2 * TM_COUNT) != cudaSuccess) { c.use_tma = false; return nullptr; }
-    }
-    if (!c.d_err) {
-        if (cudaMalloc((void**)&c.d_err, sizeof(int)) != cudaSuccess) { c.use_tma = false; return nullptr; }
-        cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream);
-    }
-    const int slot = c.map_key[0] ? 1 : 0;
-    CUtensorMap h[TM_COUNT];
-    const int in_f[5] = {F_V1, F_V2, F_V3, F_ETA, F_ETA_SM};
-    const int old_f[7] = {F_P, F_T11, F_T22, F_T33, F_T12, F_T13, F_T23};
-    bool ok = true;
-    for (int i = 0; i < 5; ++i) ok &= encode_map(c, &h[TM_V1 + i], t.f[in_f[i]], TIN_X, TIN_Y);
-    for (int i = 0; i < 7; ++i) ok &= encode_map(c, &h[TM_P + i], t.f[old_f[i]], TOLD_X, TOLD_Y);
-    ok &= encode_map(c, &h[TM_RP], t.f[F_RP], TOLD_X, TOLD_Y);
-    ok &= encode_map(c, &h[TM_RHO], t.f[F_RHO], TOLD_X, TOLD_Y);
-    ok &= encode_map(c, &h[TM_RV1], t.f[F_RV1], FTX, FTY);
-    ok &= encode_map(c, &h[TM_RV2], t.f[F_RV2], FTX, FTY);
-    ok &= encode_map(c, &h[TM_RV3], t.f[F_RV3], FTX, FTY);
-    if (!ok || cudaMemcpy(c.d_maps + slot * TM_COUNT, h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess) {
-        c.use_tma = false;
-        return nullptr;
-    }
-    c.map_key[slot] = t.f[F_V1];
-    return c.d_maps + slot * TM_COUNT;
-}
-
-// build the tensor-map sets of both ping-pong arrangements (never inside a graph capture)
-void ensure_tma_maps(Ctx& c) {
-    if (!c.use_tma || !c.fused) return;
-    tma_maps(c);
-    swap_state(c.s32);
-    tma_maps(c);
-    swap_state(c.s32);
-}
-
 // The error word of the TMA sweep kernels: set when a bounded wait on a copy barrier ran
 // out.  The kernel then stopped issuing copies and finished its march on whatever its
 // tiles held, so the FP32 state is suspect and copies may have been in flight when its
@@ -996,47 +1041,38 @@ KP<float> make_kp_corr(Ctx& c) {
     return q;
 }
 
+// whether the correction sweep handles the boundary velocities itself (no BC launches between sweeps)
+bool sweep_fills_ghosts(const Ctx& c) { return c.fused && c.use_tma && c.ghost_gmask != 0; }
+
 // one FP32 sweep of the correction problem (fused or one kernel per step) + homogeneous BCs
 template <int G>
 void correction_sweep(Ctx& c) {
     State<float>& t = c.s32;
     KP<float> q = make_kp_corr(c);
-    int first_bc = 0;
+    bool bc = true;
     if (c.fused) {
-        const CUtensorMap* maps = tma_maps(c);
-        if (maps) {
-            FusedOut<float> o;
-            o.P = t.f[F_A_P]; o.V1 = t.f[F_A_V1]; o.V2 = t.f[F_A_V2]; o.V3 = t.f[F_A_V3];
-            o.t11 = t.f[F_A_T11]; o.t22 = t.f[F_A_T22]; o.t33 = t.f[F_A_T33]; o.t12 = t.f[F_A_T12]; o.t13 = t.f[F_A_T13]; o.t23 = t.f[F_A_T23];
-            o.xg_mask = 0;
-            o.xg[0] = o.xg[1] = o.xg[2] = 0.f;
-            if (!c.use_x2 && c.xg_mask) {  // the sweep writes the x1-face ghosts: the BC launch skips its first stage
-                o.xg_mask = c.xg_mask;
-                for (int i = 0; i < 3; ++i) o.xg[i] = c.xg[i];
-                first_bc = 1;
-            }
-            const int kc = fused_chunk(c);
-            dim3 grid((c.d.n1 + FTX - 1) / FTX, (c.d.n2 + FTY - 1) / FTY, (c.d.n3 + kc - 1) / kc);
-            const bool prof = c.prof_on && 2 * c.prof_next + 1 < c.prof_ev.size();
-            if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next], c.stream);
-            if (c.use_x2)
-                k_sweep_x2<G><<<grid, dim3(X2_NT, 1, 1), sweep_x2_smem_bytes(), c.stream>>>(q, o, kc, maps, c.d_err);
-            else
-                launch_pdl(c.use_pdl, k_fused_tma<G, 1>, grid, dim3(FNT, 1, 1), fused_tma_smem_bytes(), c.stream, q, o, kc, maps, c.d_err);
-            if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next++ + 1], c.stream);
-        } else {
-            const bool prof = c.prof_on && 2 * c.prof_next + 1 < c.prof_ev.size();
-            if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next], c.stream);
-            launch_fused<G, 1>(c, q, t);
-            if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next++ + 1], c.stream);
-        }
+        const bool prof = c.prof_on && 2 * c.prof_next + 1 < c.prof_ev.size();
+        if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next], c.stream);
+        bc = !launch_fused<G, 1>(c, q, sweep_fills_ghosts(c));
+        if (prof) cudaEventRecord(c.prof_ev[2 * c.prof_next++ + 1], c.stream);
         swap_state(t);
+        c.ghost_stored = false;
         q = make_kp_corr(c);
     } else {
         k_stress<float, G, true><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(q);
         k_velocity<float, G, 1><<<grid_vel(c.d), blk2d(), 0, c.stream>>>(q);
     }
-    launch_bc<float, G>(c, q, 1, first_bc);
+    if (bc) launch_bc<float, G>(c, q, 1);
+}
+
+// n sweeps, then the BC program where the sweeps leave ghosts unstored (as a caller reads them)
+template <int G>
+void correction_sweeps(Ctx& c, int n) {
+    for (int i = 0; i < n; ++i) correction_sweep<G>(c);
+    if (sweep_fills_ghosts(c)) {
+        KP<float> q = make_kp_corr(c);
+        launch_bc<float, G>(c, q, 1);
+    }
 }
 
 // run `n` correction sweeps; with graphs enabled and n even, replays a captured
@@ -1045,8 +1081,8 @@ void correction_sweep(Ctx& c) {
 template <int G>
 int run_correction_sweeps(Ctx& c, int n) {
     if (n <= 0) return SPH_OK;
-    if (!c.use_graphs || (n & 1) || n < 8) {
-        for (int i = 0; i < n; ++i) correction_sweep<G>(c);
+    if (!c.use_graphs || (n & 1) || n < 8 || c.ghost_stored) {
+        correction_sweeps<G>(c, n);
         CK(cudaGetLastError());
         return SPH_OK;
     }
@@ -1069,7 +1105,7 @@ int run_correction_sweeps(Ctx& c, int n) {
         CK(cudaStreamSynchronize(c.stream));
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < n; ++i) correction_sweep<G>(c);  // recorded, not run
+        correction_sweeps<G>(c, n);  // recorded, not run
         cudaError_t e = cudaStreamEndCapture(c.stream, &g);
         if (e != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
         e = cudaGraphInstantiate(&c.corr_graph[slot], g, 0);
@@ -1142,6 +1178,7 @@ int run_warm_iterations(Ctx& c, int n) {
     if (slot < 0) {
         slot = c.warm_graph[0] ? 1 : 0;
         if (c.warm_graph[slot]) { cudaGraphExecDestroy(c.warm_graph[slot]); c.warm_graph[slot] = nullptr; }
+        ensure_tma_maps(c);
         CK(cudaStreamSynchronize(c.stream));
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
@@ -1304,10 +1341,9 @@ int batch_nout(const sph_solve_opts& o) { return o.nout > 0 ? o.nout : 100; }
 
 // whether a solve can run in the lockstep batch (else the batch falls back to host threads)
 bool batch_eligible(const Ctx& c, const sph_solve_opts& o) {
-    const int first = c.xg_mask ? 1 : 0;
     return c.prm.precision == SPH_PREC_MIXED && o.criterion == SPH_CRIT_RESIDUAL && !(o.warm_tol > 0.0) &&
-           (c.prm.rheology == SPH_RHEO_LINEAR || c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) && c.fused && c.use_tma && !c.use_x2 &&
-           !c.broken && (batch_nout(o) % 2) == 0 && o.tol > 0.0 && o.maxiter > 0 && (int)c.bc_run.size() - first <= kBatchMaxBc;
+           (c.prm.rheology == SPH_RHEO_LINEAR || c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) && sweep_fills_ghosts(c) &&
+           !c.broken && (batch_nout(o) % 2) == 0 && o.tol > 0.0 && o.maxiter > 0;
 }
 
 // the device entry of a solve whose correction problem has just been prepared
@@ -1319,19 +1355,12 @@ int batch_entry(Ctx& c, BatchSweep& e) {
         const CUtensorMap* maps = tma_maps(c);
         if (!maps || !c.d_err) return fail(SPH_ERR_UNSUPPORTED, "batched sweeps need the TMA sweep");
         e.p[a] = make_kp_corr(c);
-        FusedOut<float>& o = e.o[a];
-        o.P = t.f[F_A_P]; o.V1 = t.f[F_A_V1]; o.V2 = t.f[F_A_V2]; o.V3 = t.f[F_A_V3];
-        o.t11 = t.f[F_A_T11]; o.t22 = t.f[F_A_T22]; o.t33 = t.f[F_A_T33]; o.t12 = t.f[F_A_T12]; o.t13 = t.f[F_A_T13]; o.t23 = t.f[F_A_T23];
-        o.xg_mask = c.xg_mask;
-        for (int i = 0; i < 3; ++i) o.xg[i] = c.xg[i];
+        e.o[a] = sweep_out(c, e.p[a], true);
         e.maps[a] = maps;
         swap_state(t);
     }
     e.err = c.d_err;
     e.kchunk = fused_chunk(c);
-    const int first = c.xg_mask ? 1 : 0;
-    e.nbc = (int)c.bc_run.size() - first;
-    for (int i = 0; i < e.nbc; ++i) e.bc[i] = c.bc_run[first + i];
     return SPH_OK;
 }
 
@@ -1360,6 +1389,12 @@ int batch_end_inner(BatchSolve& b) {
     int rc = check_kernel_flag(c);
     if (rc) return rc;
     if (b.status == SPH_ERR_DIVERGED) { b.st = BatchSolve::DONE; return SPH_OK; }
+    // the ghosts that the batched sweeps leave unstored
+    switch (c.prm.geometry) {
+        case SPH_GEOM_SPHERICAL: correction_sweeps<SPH>(c, 0); break;
+        case SPH_GEOM_CYLINDRICAL: correction_sweeps<CYL>(c, 0); break;
+        default: correction_sweeps<CART>(c, 0); break;
+    }
     if ((rc = apply_correction(c))) return rc;
     ++b.outer;
     b.st = BatchSolve::OUTER;
@@ -1450,10 +1485,10 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
     CK(cudaEventRecord(dev.e0, dev.stream));
     for (BatchSolve& b : bs) { int rc = sync64(*b.c); if (rc) return rc; }
 
-    // work lists: blocks of the member solves' fused sweeps, BC stages and inner tests, per geometry
+    // work lists: blocks of the member solves' fused sweeps and inner tests, per geometry
     std::vector<BatchSweep> host((size_t)n);
     std::vector<int4> items;
-    size_t fz_off[3], fz_n[3], nm_off[3], nm_n[3], bc_off[3][kBatchMaxBc], bc_n[3][kBatchMaxBc];
+    size_t fz_off[3], fz_n[3], nm_off[3], nm_n[3];
     size_t items_cap = 0, members = 0;
     auto build_lists = [&]() -> int {
         items.clear();
@@ -1468,22 +1503,10 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
                 Ctx& c = *bs[i].c;
                 if (c.prm.geometry != g) continue;
                 const int kc = fused_chunk(c);
-                const int gx = (c.d.n1 + FTX - 1) / FTX, gy = (c.d.n2 + FTY - 1) / FTY, gz = (c.d.n3 + kc - 1) / kc;
-                for (int z = 0; z < gz; ++z) for (int y = 0; y < gy; ++y) for (int x = 0; x < gx; ++x) items.push_back(make_int4(i, x, y, z));
+                const dim3 gr = sweep_grid(c.d, kc);
+                for (unsigned z = 0; z < gr.z; ++z) for (unsigned y = 0; y < gr.y; ++y) for (unsigned x = 0; x < gr.x; ++x) items.push_back(make_int4(i, (int)x, (int)y, (int)z));
             }
             fz_n[g] = items.size() - fz_off[g];
-            for (int t = 0; t < kBatchMaxBc; ++t) {
-                bc_off[g][t] = items.size();
-                for (int i : mem) {
-                    Ctx& c = *bs[i].c;
-                    const int first = c.xg_mask ? 1 : 0;
-                    if (c.prm.geometry != g || first + t >= (int)c.bc_run.size()) continue;
-                    const BcStage& st = c.bc_run[first + t];
-                    const int eu = st.dim == 0 ? c.d.n2 + 1 : c.d.n1 + 1, ev = st.dim == 2 ? c.d.n2 + 1 : c.d.n3 + 1;
-                    for (int v = 0; v < (ev + 7) / 8; ++v) for (int u = 0; u < (eu + 31) / 32; ++u) items.push_back(make_int4(i, u, v, 0));
-                }
-                bc_n[g][t] = items.size() - bc_off[g][t];
-            }
             nm_off[g] = items.size();
             for (int i : mem) {
                 Ctx& c = *bs[i].c;
@@ -1527,14 +1550,9 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             // tail of the one before (the kernels wait on it before touching memory)
             const BatchSweep* E = dev.entries;
             const int* act_d = dev.active;
-            if (fz_n[SPH]) launch_pdl(pdl, k_fused_tma_batch<SPH>, dim3((unsigned)fz_n[SPH]), dim3(FNT), fused_tma_smem_bytes(), dev.stream, E, dev.items + fz_off[SPH], act_d, a);
-            if (fz_n[CYL]) launch_pdl(pdl, k_fused_tma_batch<CYL>, dim3((unsigned)fz_n[CYL]), dim3(FNT), fused_tma_smem_bytes(), dev.stream, E, dev.items + fz_off[CYL], act_d, a);
-            if (fz_n[CART]) launch_pdl(pdl, k_fused_tma_batch<CART>, dim3((unsigned)fz_n[CART]), dim3(FNT), fused_tma_smem_bytes(), dev.stream, E, dev.items + fz_off[CART], act_d, a);
-            for (int t = 0; t < kBatchMaxBc; ++t) {
-                if (bc_n[SPH][t]) launch_pdl(pdl, k_bc_batch<SPH>, dim3((unsigned)bc_n[SPH][t]), blk2d(), 0, dev.stream, E, dev.items + bc_off[SPH][t], act_d, a, t);
-                if (bc_n[CYL][t]) launch_pdl(pdl, k_bc_batch<CYL>, dim3((unsigned)bc_n[CYL][t]), blk2d(), 0, dev.stream, E, dev.items + bc_off[CYL][t], act_d, a, t);
-                if (bc_n[CART][t]) launch_pdl(pdl, k_bc_batch<CART>, dim3((unsigned)bc_n[CART][t]), blk2d(), 0, dev.stream, E, dev.items + bc_off[CART][t], act_d, a, t);
-            }
+            if (fz_n[SPH]) launch_pdl(pdl, k_sweep_batch<SPH>, dim3((unsigned)fz_n[SPH]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[SPH], act_d, a);
+            if (fz_n[CYL]) launch_pdl(pdl, k_sweep_batch<CYL>, dim3((unsigned)fz_n[CYL]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[CYL], act_d, a);
+            if (fz_n[CART]) launch_pdl(pdl, k_sweep_batch<CART>, dim3((unsigned)fz_n[CART]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[CART], act_d, a);
         }
         cudaError_t e = cudaStreamEndCapture(dev.stream, &g);
         if (e != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e));
@@ -1760,16 +1778,14 @@ int sph_create(const sph_params* prm, void** out) {
     {
         int dev = 0, sms = 0, per_sm = 0;
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_tma<SPH, 1>, FNT, fused_tma_smem_bytes()) == cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<SPH, 1>, SW_NT, sweep_smem_bytes()) == cudaSuccess)
             c->fused_slots = sms * per_sm;
         cudaGetLastError();
     }
     if (const char* e = std::getenv("SPH_NO_GRAPHS")) c->use_graphs = std::atoi(e) == 0;
     if (const char* e = std::getenv("SPH_NO_TMA")) c->use_tma = std::atoi(e) == 0;
-    if (const char* e = std::getenv("SPH_SWEEP_X2")) c->use_x2 = std::atoi(e) != 0;
-    if (q.bc == SPH_BC_FREE_SURFACE) c->use_x2 = false;  // the paired-FP32 sweep has no free-surface top cell
     if (const char* e = std::getenv("SPH_NO_PDL")) c->use_pdl = std::atoi(e) == 0;
-    if (const char* e = std::getenv("SPH_NO_XGHOST")) c->xg_fuse = std::atoi(e) == 0;
+    if (const char* e = std::getenv("SPH_NO_XGHOST")) c->ghost_fuse = std::atoi(e) == 0;
     if ((rc = build_bc(*c))) return cleanup(rc);
     if ((rc = init_fields(*c))) return cleanup(rc);
     if ((rc = compute_f_scale(*c))) return cleanup(rc);
@@ -2607,6 +2623,7 @@ static int corr_access(void* h, int32_t field, double* host, const double* src, 
     int rc = ensure_correction(*c);
     if (rc) return rc;
     float* dev = c->s32.f[slot];
+    if (src) c->ghost_stored = true;  // the caller's boundary velocities need not satisfy the BCs
     return host ? download_box<float>(*c, dev, e, host) : upload_box<float>(*c, dev, e, src);
 }
 
