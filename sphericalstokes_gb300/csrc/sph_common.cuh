@@ -46,6 +46,7 @@ struct Geo {
     const T* x1c;      // coordinates of the cell centres  [n1], [n2], [n3]
     const T* x2c;
     const T* x3c;
+    const T* pow_tab;  // tables of fast_pow (FP64 state only)
 };
 
 // all fields and scalars one PT kernel may touch
@@ -114,12 +115,6 @@ __device__ __forceinline__ unsigned long long ord_bits(double x) {
     return x != x ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(x);
 }
 __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
-
-// max with NaN propagation (Julia's `max`)
-template <typename T>
-__device__ __forceinline__ T jmax(T a, T b) {
-    return (a != a || b != b) ? (a + b) : (a > b ? a : b);
-}
 
 // metric coefficients of a cell (i, j): divergence and deviatoric normal strain rates
 //   div  = d1*Δ1 + a2*Δ2 + a3*Δ3 + c1*avx(V1) + c2*avy(V2)

@@ -1,0 +1,325 @@
+// PT kernels that march along x3: one thread per (x1, x2) column, a chunk of planes each.
+//
+//   k_cells     compute_P! (WHAT_STRESS), with the strain rates kept for the strain-rate law
+//               (WHAT_STRESS_LAW), the strain rates alone (WHAT_STRAIN) or the viscous stresses
+//               and the divergence of the FP64 residual (WHAT_VISC)
+//   k_nodes     compute_V!: V += avg(DT_R) (momentum) (MODE 0), with the right-hand side of the
+//               correction problem (MODE 1), or the momentum residual itself (MODE 2)
+//   k_edot      strain-rate power law; k_rheo compute_TII! + copy_BC!(τII) + power_law!
+// (SphericalStokes_diapir.jl:155-329)
+//
+// Bound: FP64 instructions (sph_math.cuh).  A thread keeps its (x1, x2) position over the planes, so the
+// metric factors are multiplied out with the spacings once per column (the kernels spent a third of
+// their FP64 instructions on that per point), and the sums of η and ηSM over two cells of a plane serve the
+// edges below and above it.  Columns are numbered along x1 over the whole plane, so that a
+// ragged n1 leaves no idle lanes (an idle lane costs as much FP64 time as a busy one).  Loads are
+// direct: neighbours come from L1, and their issue slots are free beside FP64 at 1/16 of a warp
+// instruction per clock.
+// MARCH_FIGURES
+#pragma once
+#include "sph_math.cuh"
+
+namespace sph {
+
+constexpr int MC_NT = 128;  // threads per block
+
+// planes per thread: enough to pay for the column's coefficients, few enough for an even share of blocks
+// per SM (the FP64 units are the only bound, so the fullest SM ends last)
+inline int march_chunk(long long columns, int planes, int sms, double setup) {
+    const long long cols = (columns + MC_NT - 1) / MC_NT;
+    int best = 1;
+    double best_t = 1e300;
+    for (int k = 1; k <= 16 && k <= planes; ++k) {
+        const long long blocks = cols * ((planes + k - 1) / k);
+        const double t = (double)((blocks + sms - 1) / sms) * (k + setup);
+        if (t < best_t) { best_t = t; best = k; }
+    }
+    return best;
+}
+
+enum CellsWhat { WHAT_STRESS = 0, WHAT_STRESS_LAW, WHAT_STRAIN, WHAT_VISC };
+
+// RHS: continuity right-hand side rP (P -= KBDT (div V + rP))
+template <typename T, int G, int WHAT, bool RHS>
+__global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p, int chunk) {
+    constexpr bool PT = WHAT == WHAT_STRESS || WHAT == WHAT_STRESS_LAW;
+    constexpr bool ETA = WHAT != WHAT_STRAIN;
+    const Dims& d = p.d;
+    const int col = blockIdx.x * MC_NT + threadIdx.x;
+    const int i = col % d.n1, j = col / d.n1;
+    if (j >= d.n2) return;
+    const int sy = d.sy, sz = d.sz;
+    const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
+    const T h = T(0.5);
+    // coefficients of the column: strain rates of the cell (sums of face velocities: halves folded in) and of its edges
+    const CellMetric<T> m = cell_metric<T, G>(p, i, j);
+    const EdgeMetric<T> e = edge_metric<T, G>(p.geo, i, j, d.n1, d.n2);
+    const T a2 = m.a2, a3 = m.a3, e1 = h * m.e1, e2 = h * m.e2, third = T(-1.0 / 3.0);
+    const T e12_2 = e.iRh * p.d2, e12_h = -h * e.iRh;
+    const T e13_3 = G == SPH ? e.iRh * e.iSc1 * p.d3 : p.d3;
+    const T e23_2 = e.iRc1 * p.d2, e23_3 = G == SPH ? e.iRc1 * e.iSh * p.d3 : p.d3, e23_h = -h * e.iRc1 * e.ctH;
+    const bool v12 = i < d.n1 - 1 && j < d.n2 - 1, v13 = i < d.n1 - 1 && j < d.n2 - 2, v23 = i < d.n1 - 2 && j < d.n2 - 1;
+    int c = i + sy * j + sz * k0;
+    // sums over two cells of a plane: X along x1 in row j + 1, Y along x2 in column i + 1
+    T eX = T(0), eY = T(0), sX = T(0), sY = T(0);
+    if (ETA) {
+        const T a = p.eta[c + 1], b = p.eta[c + sy], q = p.eta[c + sy + 1];
+        eX = b + q; eY = a + q;
+    }
+    if (PT) {
+        const T a = p.etaSM[c + 1], b = p.etaSM[c + sy], q = p.etaSM[c + sy + 1];
+        sX = b + q; sY = a + q;
+    }
+    const T gsc4 = T(0.25) * p.gsc;
+    // (entries past the grid are padding of the box: finite, and their results are not stored)
+    for (int k = k0; k < k1; ++k, c += sz) {
+        const int u = c + sz;
+        const T v1p = p.V1[c + 1], v2p = p.V2[c + sy], v3p = p.V3[u];
+        const T D1 = v1p - p.V1[c], D2 = v2p - p.V2[c], D3 = v3p - p.V3[c];
+        T D11 = p.d1 * D1, D22, D33, div;
+        if (G != CART) {
+            const T ex = e1 * (p.V1[c] + v1p);
+            D22 = fma(a2, D2, ex);
+            D33 = G == SPH ? fma(a3, D3, fma(e2, p.V2[c] + v2p, ex)) : a3 * D3;
+            div = D11 + D22 + D33;
+            D11 = fma(div, third, D11); D22 = fma(div, third, D22); D33 = fma(div, third, D33);
+        } else {
+            D22 = a2 * D2; D33 = a3 * D3;
+            div = D11 + D22 + D33;
+        }
+        if (WHAT == WHAT_STRAIN || WHAT == WHAT_STRESS_LAW) p.sDD[c] = h * fma(D11, D11, fma(D22, D22, D33 * D33));
+        if (PT) {
+            const T sm = p.etaSM[c], et = p.eta[c];
+            const T gs = p.gsc * sm, kb = p.kbc * sm, gs2 = gs + gs;
+            const T f = fast_div(et, et + gs);  // 1/(1 + GSDT/η)
+            T Pn = fma(-kb, RHS ? div + p.rP[c] : div, p.P[c]);
+            const T n11 = fma(gs2, D11, p.t11[c]) * f, n22 = fma(gs2, D22, p.t22[c]) * f, n33 = fma(gs2, D33, p.t33[c]) * f;
+            if (p.traction) traction_pressure(j, k, d.n2, d.n3, n22, n33, p.sig2, p.sig3, Pn);
+            if (p.fs && i == d.n1 - 1) Pn = fs_pressure(n11, p.top_load ? p.top_load[c] : T(0), p.fs_kappa, p.V1[c], v1p);
+            p.P[c] = Pn;
+            p.t11[c] = n11; p.t22[c] = n22; p.t33[c] = n33;
+            p.DT_R[c] = fast_div(p.vpdt2, fma(gs, f, kb));
+        } else if (WHAT == WHAT_VISC) {
+            const T x = T(2) * p.eta[c];
+            p.t11[c] = x * D11; p.t22[c] = x * D22; p.t33[c] = x * D33;
+            p.rP[c] = div;
+        }
+        // edges: sums of the plane above
+        T eX0 = T(0), eXn = T(0), eYn = T(0), sX0 = T(0), sXn = T(0), sYn = T(0);
+        if (ETA) {
+            const T a = p.eta[u + 1], b = p.eta[u + sy], q = p.eta[u + sy + 1];
+            eX0 = p.eta[u] + a; eXn = b + q; eYn = a + q;
+        }
+        if (PT) {
+            const T a = p.etaSM[u + 1], b = p.etaSM[u + sy], q = p.etaSM[u + sy + 1];
+            sX0 = p.etaSM[u] + a; sXn = b + q; sYn = a + q;
+        }
+        auto edge = [&](T* t, T* s, T D, T e4, T s4, bool ok) {
+            if (PT) {  // (τ + aG D) aE / (aE + aG), aE = e4 / 4, aG = GSDT s4 / 4
+                const T g = gsc4 * s4;
+                const T v = fma(g, D, t[c]) * fast_div(e4, fma(T(4), g, e4));
+                if (ok) t[c] = v;
+            } else if (WHAT == WHAT_VISC) {
+                if (ok) t[c] = T(0.25) * e4 * D;
+            }
+            if ((WHAT == WHAT_STRAIN || WHAT == WHAT_STRESS_LAW) && ok) s[c] = D;
+        };
+        const T v1a = p.V1[u + 1], v1b = p.V1[u + 1 + sy], v2a = p.V2[u + sy], v2b = p.V2[u + sy + 1];
+        const T v3q = p.V3[u + sy], v3t = p.V3[u + sy + 1], v3s = p.V3[u + 1];
+        {
+            T D = fma(e12_2, v1b - v1a, p.d1 * (v2b - v2a));
+            if (G != CART) D = fma(e12_h, v2a + v2b, D);
+            edge(p.t12, p.s12, D, eX0 + eXn, sX0 + sXn, v12 && k < d.n3 - 2);
+        }
+        {
+            T D = fma(e13_3, v1b - p.V1[c + 1 + sy], p.d1 * (v3t - v3q));
+            if (G == SPH) D = fma(e12_h, v3q + v3t, D);
+            edge(p.t13, p.s13, D, eX + eXn, sX + sXn, v13 && k < d.n3 - 1);
+        }
+        {
+            T D = fma(e23_3, v2b - p.V2[c + 1 + sy], e23_2 * (v3t - v3s));
+            if (G == SPH) D = fma(e23_h, v3s + v3t, D);
+            edge(p.t23, p.s23, D, eY + eYn, sY + sYn, v23 && k < d.n3 - 1);
+        }
+        eX = eXn; eY = eYn; sX = sXn; sY = sYn;
+    }
+}
+
+template <typename T, int G, int MODE>
+__global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p, int chunk) {
+    const Dims& d = p.d;
+    const int col = blockIdx.x * MC_NT + threadIdx.x;
+    const int w = d.n1 - 1;
+    const int I = col % w + 1, J = col / w + 1;
+    if (J > d.n2 - 1) return;
+    const int sy = d.sy, sz = d.sz;
+    const int K0 = blockIdx.y * chunk + 1, K1 = min(K0 + chunk, d.n3);  // K0 .. K1 - 1
+    // the update wants the residual times (DT + DT') / 2: its half is folded into the coefficients
+    const T s = MODE == 2 ? T(1) : T(0.5), h = T(0.5);
+    const MomMetric<T> m = mom_metric<T, G>(p.geo, I, J, d.n1, d.n2);
+    const T c1 = s * p.d1;
+    const T m1_2 = s * m.iR1 * p.d2, m1_3 = s * (G == SPH ? m.iR1 * m.iS1 * p.d3 : p.d3), m1_n = s * (G == SPH ? m.iR1 : h * m.iR1);
+    const T m1_t = s * h * m.iR1 * m.ct1;
+    const T m2_2 = s * m.iR2 * p.d2, m2_3 = s * (G == SPH ? m.iR2 * m.iS2 * p.d3 : p.d3), m2_s = s * (G == SPH ? T(1.5) * m.iR2 : m.iR2);
+    const T m2_n = s * h * m.iR2 * m.ct2;
+    const T m3_3 = s * (G == SPH ? m.iR2 * m.iS3 * p.d3 : p.d3), m3_s = s * (G == SPH ? T(1.5) * m.iR2 : h * m.iR2), m3_n = s * m.iR2 * m.ct3;
+    const T gh = -s * h * p.g;
+    const bool w1 = J <= d.n2 - 2, w2 = I <= d.n1 - 2, w3 = w1 && w2;
+    int c = I + sy * J + sz * K0;
+    // plane K0 - 1: σ33 and DT_R of the cell below, edge stresses
+    T q33 = p.t33[c - sz] - p.P[c - sz], qdt = MODE == 2 ? T(0) : p.DT_R[c - sz];
+    T p13a = p.t13[c - sy - sz], p13b = p.t13[c - 1 - sy - sz], p23 = p.t23[c - 1 - sy - sz];
+    for (int K = K0; K < K1; ++K, c += sz) {
+        const T P = p.P[c];
+        const T s11 = p.t11[c] - P, s22 = p.t22[c] - P, s33 = p.t33[c] - P;
+        const T dt = MODE == 2 ? T(0) : p.DT_R[c];
+        const T t13a = p.t13[c - sy], t13b = p.t13[c - 1 - sy], t23 = p.t23[c - 1 - sy];
+        const T t12b = p.t12[c - 1 - sy - sz], t12c = p.t12[c - sy - sz];
+        const bool kin = K <= d.n3 - 2;
+        auto put = [&](T* V, T* R, T r, T dm) {
+            if (MODE == 2) R[c] = r;
+            else V[c] = fma(MODE == 1 ? fma(h, R[c], r) : r, dm + dt, V[c]);
+        };
+        if (w1 && kin) {  // V1 (I-1/2, J, K), cell m = (I-1, J, K)
+            const T Pm = p.P[c - 1], t12a = p.t12[c - 1 - sz];
+            const T m11 = p.t11[c - 1] - Pm;
+            T r = fma(m1_3, t13b - p13b, fma(m1_2, t12a - t12b, c1 * (s11 - m11)));
+            if (G == SPH) {
+                const T m22 = p.t22[c - 1] - Pm, m33 = p.t33[c - 1] - Pm;
+                r = fma(m1_t, t12a + t12b, fma(m1_n, fma(-h, (m22 + s22) + (m33 + s33), m11 + s11), r));
+            } else if (G == CYL) {
+                r = fma(m1_n, (m11 + s11) - (p.t22[c - 1] - Pm + s22), r);
+            }
+            if (G != CART && MODE != 1) r = fma(gh, p.rho[c - 1] + p.rho[c], r);
+            put(p.V1, p.rV1, r, MODE == 2 ? T(0) : p.DT_R[c - 1]);
+        }
+        if (w2 && kin) {  // V2 (I, J-1/2, K), cell m = (I, J-1, K)
+            const T Pm = p.P[c - sy];
+            const T m22 = p.t22[c - sy] - Pm;
+            T r = fma(m2_3, t23 - p23, fma(m2_2, s22 - m22, c1 * (t12c - t12b)));
+            if (G != CART) r = fma(m2_s, t12c + t12b, r);
+            if (G == SPH) r = fma(m2_n, (m22 + s22) - (p.t33[c - sy] - Pm + s33), r);
+            put(p.V2, p.rV2, r, MODE == 2 ? T(0) : p.DT_R[c - sy]);
+        }
+        if (w3) {  // V3 (I, J, K-1/2), cell m = (I, J, K-1)
+            const T t23a = p.t23[c - 1 - sz];
+            T r = fma(m3_3, s33 - q33, fma(m2_2, t23a - p23, c1 * (p13a - p13b)));
+            if (G != CART) r = fma(m3_s, p13a + p13b, r);
+            if (G == SPH) r = fma(m3_n, t23a + p23, r);
+            if (G == CART && MODE != 1) r = fma(gh, p.rho[c - sz] + p.rho[c], r);
+            put(p.V3, p.rV3, r, qdt);
+        }
+        q33 = s33; qdt = dt; p13a = t13a; p13b = t13b; p23 = t23;
+    }
+}
+
+// strain-rate power law (k_edot_law of sph_pt.cuh is the FP32 one): with x = (ε̇_II / ε̇_bg)^2 of the clamped
+// interior cell, η_t = 2 / (1/η_ini + 1/η_PL) = 2 η_ini / (1 + x^((n-1)/(2n))); RELAXED: η_out = η^(1-relax) η_t^relax
+template <bool RELAXED>
+__global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<double> p, int chunk) {
+    const Dims& d = p.d;
+    const int col = blockIdx.x * MC_NT + threadIdx.x;
+    const int i = col % d.n1, j = col / d.n1;
+    if (j >= d.n2) return;
+    const int sy = d.sy, sz = d.sz;
+    const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
+    const double* tab = p.geo.pow_tab;
+    const double ib2 = 1.0 / (p.edot_bg * p.edot_bg), ex = 0.5 * (p.n_exp - 1.0) / p.n_exp;
+    const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
+    int last = -1;
+    double x = 0.0;
+    for (int k = k0; k < k1; ++k) {
+        const int kc = clampi(k, 1, d.n3 - 2);
+        const int c = i + sy * j + sz * k;
+        if (kc != last) {
+            const int s = s0 + sz * kc, e = s - 1 - sy - sz;
+            const double a = (p.s12[e] + p.s12[e + sy]) + (p.s12[e + 1] + p.s12[e + 1 + sy]);
+            const double b = (p.s13[e] + p.s13[e + 1]) + (p.s13[e + sz] + p.s13[e + 1 + sz]);
+            const double q = (p.s23[e] + p.s23[e + sy]) + (p.s23[e + sz] + p.s23[e + sy + sz]);
+            // (sums of four edges: a quarter of each, squared, times another quarter)
+            x = fma(1.0 / 64.0, fma(a, a, fma(b, b, q * q)), p.sDD[s]);
+            last = kc;
+        }
+        const double ei = p.eta_ini[c];
+        double et = ei;
+        if (!(p.phase && p.phase[c])) et = fast_div(ei + ei, 1.0 + fast_pow(tab, x * ib2, ex));
+        if (RELAXED) {
+            const double eo = p.eta[c];
+            // exact for the half-way mean; else η (η_t/η)^relax
+            et = p.relax == 0.5 ? sqrt(eo * et) : eo * fast_pow(tab, fast_div(et, eo), p.relax);
+        }
+        p.eta_out[c] = et;
+    }
+}
+
+// compute_TII! + copy_BC!(τII) + power_law! (k_rheo_tau of sph_pt.cuh is the FP32 one): with x = (τII / τ_C)^2,
+// η_PL = η_ini x^((1-n)/2), η = 2 / (1/η_ini + 1/η_PL); RELAX: η_PL relaxed in log space
+// (CylindricalStokes_diapir.jl:185-192).  phase == 1 cells are linear.
+template <bool RELAX>
+__global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, double n_exp, int chunk) {
+    const Dims& d = p.d;
+    const int col = blockIdx.x * MC_NT + threadIdx.x;
+    const int i = col % d.n1, j = col / d.n1;
+    if (j >= d.n2) return;
+    const int sy = d.sy, sz = d.sz;
+    const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
+    const double* tab = p.geo.pow_tab;
+    const double ic2 = 1.0 / (p.tau_C * p.tau_C);
+    const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
+    const int rim = (i == 0 || i == d.n1 - 1) + (j == 0 || j == d.n2 - 1);
+    int last = -1;
+    double t2c = 0.0, tiic = 0.0;
+    for (int k = k0; k < k1; ++k) {
+        const int c = i + sy * j + sz * k;
+        double t2, tii;
+        if (faces_only && rim + (k == 0 || k == d.n3 - 1) >= 2) {
+            tii = p.tII[c];  // CartesianStokes_diapir.jl:97-105 never writes edges/corners of τII
+            t2 = tii * tii;
+        } else {
+            const int kc = clampi(k, 1, d.n3 - 2);
+            if (kc != last) {
+                const int s = s0 + sz * kc, e = s - 1 - sy - sz;
+                const double a = (p.t12[e] + p.t12[e + sy]) + (p.t12[e + 1] + p.t12[e + 1 + sy]);
+                const double b = (p.t13[e] + p.t13[e + 1]) + (p.t13[e + sz] + p.t13[e + 1 + sz]);
+                const double q = (p.t23[e] + p.t23[e + sy]) + (p.t23[e + sz] + p.t23[e + sy + sz]);
+                const double x = p.t11[s], y = p.t22[s], z = p.t33[s];
+                t2c = fma(0.5, fma(x, x, fma(y, y, z * z)), 1.0 / 16.0 * fma(a, a, fma(b, b, q * q)));
+                tiic = sqrt(t2c);
+                last = kc;
+            }
+            t2 = t2c;
+            p.tII[c] = tii = tiic;
+        }
+        const double cx = (p.phase && p.phase[c]) ? 0.0 : 0.5 * (n_exp - 1.0);
+        const double ei = p.eta_ini[c], x = t2 * ic2;
+        if (!RELAX) {
+            p.eta[c] = fast_div(ei + ei, 1.0 + fast_pow(tab, x, cx));
+        } else {
+            const double po = p.eta_pl[c];
+            double pl;
+            bool done = false;
+            if (normal_pos(x) && normal_pos(ei) && normal_pos(po)) {
+                // η_PL' = po 2^(relax (log2 ei - log2 po - cx log2 x)), the exponent as a head and a tail
+                double hx, tx, hi, ti, ho, to;
+                log2_parts(tab, x, hx, tx);
+                log2_parts(tab, ei, hi, ti);
+                log2_parts(tab, po, ho, to);
+                const double L = hi - ho, q = cx * hx, s = L - q;
+                const double low = ((ti - to) - fma(cx, tx, fma(cx, hx, -q))) + ((L - s) - q);
+                const double y = p.relax * s;
+                if ((__double2hiint(y) & 0x7fffffff) < 0x408f4000) {  // |y| < 1000
+                    pl = po * exp2_parts(tab, y, fma(p.relax, low, fma(p.relax, s, -y)));
+                    done = true;
+                }
+            }
+            if (!done) {
+                pl = ei * pow(tii / p.tau_C, -2.0 * cx);
+                pl = exp(log(pl) * p.relax + log(po) * (1.0 - p.relax));
+            }
+            p.eta_pl[c] = pl;
+            p.eta[c] = done ? fast_div((ei + ei) * pl, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
+        }
+    }
+}
+
+}  // namespace sph

@@ -1,0 +1,93 @@
+// Arithmetic of the FP64 kernels in few FP64 instructions.
+//
+// GB300 executes about two FP64 operations per SM and clock (1/64 of its FP32 rate), so
+// the FP64 path is bound by the number of FP64 instructions and hardly by anything else.
+#pragma once
+#include <cmath>
+
+#include "sph_core.cuh"
+
+namespace sph {
+
+// a / b in six FP64 operations: PTX's approximate reciprocal (relative error below 2^-20), one
+// third-order Newton (Householder) step r += r (e + e^2), e = 1 - b r, to 2^-60, and Markstein's
+// correction of the quotient by its residual, q += r (a - b q).  At most one unit in the last place from
+// the IEEE quotient for normal operands and quotients (viscosities, steps: no special cases kept).
+__device__ __forceinline__ double fast_div(double a, double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    const double e = fma(-b, r, 1.0);
+    r = fma(r, fma(e, e, e), r);
+    const double q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
+__device__ __forceinline__ float fast_div(float a, float b) { return pdiv(a, b); }
+
+// ---------------------------------------------------------------------------
+// x^c of positive normal numbers, after the table-driven scheme of P. T. P. Tang (ACM TOMS 15-18, 1989-1992):
+// log2 x = E + log2(1/C_i) + log2(1 + r), r = m C_i - 1 with C_i ~ 1/m of the interval of m's leading seven
+// bits, as an exact head and a short tail; c log2 x the same way; 2^y = 2^n 2^(j/64) 2^g.  About 24 FP64
+// operations and an error below 1.1 units in the last place while |c log2 x| < 1000, against some hundred
+// operations of pow().  The tables are made on the host (fill_pow_tables).
+constexpr int kLogN = 128, kExpN = 64;
+constexpr int kPowTab = 3 * kLogN + kExpN;  // doubles: C_i, head, tail of log2(1/C_i); 2^(j/64)
+
+__device__ __forceinline__ bool normal_pos(double x) { return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u; }
+
+// log2 of a positive normal x: head (a multiple of 2^-40: sums of a few heads are exact) and tail
+__device__ __forceinline__ void log2_parts(const double* __restrict__ tab, double x, double& head, double& tail) {
+    const int hi = __double2hiint(x);
+    const int i = (hi >> 13) & (kLogN - 1);
+    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
+    const double r = fma(m, __ldg(tab + i), -1.0);  // |r| < 2^-8
+    // log2(1 + r) = sum (-1)^(k+1) r^k / (k ln 2), to r^6: the next term is below 2^-58
+    double p = -0.2404491734814939;
+    p = fma(p, r, 0.28853900817779266);
+    p = fma(p, r, -0.36067376022224085);
+    p = fma(p, r, 0.4808983469629878);
+    p = fma(p, r, -0.7213475204444817);
+    p = fma(p, r, 1.4426950408889634);
+    tail = fma(p, r, __ldg(tab + 2 * kLogN + i));
+    head = (double)((hi >> 20) - 1023) + __ldg(tab + kLogN + i);
+}
+// 2^(y + t), |y| < 1000, t a small correction
+__device__ __forceinline__ double exp2_parts(const double* __restrict__ tab, double y, double t) {
+    const double big = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer in the low word
+    const double s = fma(y, (double)kExpN, big);
+    const int n = __double2loint(s);
+    const double g = fma(s - big, -1.0 / kExpN, y) + t;  // |g| <= 2^-7
+    // 2^g - 1 = sum (g ln 2)^k / k!, to g^6: the next term is below 2^-66
+    double p = 0.0001540353039338161;
+    p = fma(p, g, 0.0013333558146428443);
+    p = fma(p, g, 0.009618129107628477);
+    p = fma(p, g, 0.05550410866482158);
+    p = fma(p, g, 0.24022650695910072);
+    p = fma(p, g, 0.6931471805599453);
+    const double T = __ldg(tab + 3 * kLogN + (n & (kExpN - 1)));
+    const double v = fma(T * g, p, T);
+    return __hiloint2double(__double2hiint(v) + ((n >> 6) << 20), __double2loint(v));
+}
+__device__ __forceinline__ double fast_pow(const double* __restrict__ tab, double x, double c) {
+    if (normal_pos(x)) {
+        double h, t;
+        log2_parts(tab, x, h, t);
+        const double y = c * h;
+        if ((__double2hiint(y) & 0x7fffffff) < 0x408f4000)  // |y| < 1000
+            return exp2_parts(tab, y, fma(c, t, fma(c, h, -y)));
+    }
+    return pow(x, c);
+}
+
+inline void fill_pow_tables(double* tab) {
+    for (int i = 0; i < kLogN; ++i) {
+        const double C = (double)(float)(1.0 / (1.0 + (i + 0.5) / kLogN));
+        const long double L = -std::log2((long double)C), u = 1099511627776.0L;  // 2^40
+        const double head = (double)(std::nearbyint(L * u) / u);
+        tab[i] = C;
+        tab[kLogN + i] = head;
+        tab[2 * kLogN + i] = (double)(L - (long double)head);
+    }
+    for (int j = 0; j < kExpN; ++j) tab[3 * kLogN + j] = (double)std::exp2((long double)j / kExpN);
+}
+
+}  // namespace sph

@@ -3,10 +3,10 @@
 // These are the building blocks of one PT iteration in the reference's order
 // (SphericalStokes_diapir.jl:413-425):
 //   k_maxloc   maxloc! + copy_BC!(ηSM)          :149-152, :102-124
-//   k_stress   compute_P!                        :155-241
-//   k_rheo_tau compute_TII! + copy_BC!(τII) + power_law!   :243-265
-//   k_strain / k_edot_law   strain-rate power law (not in the reference)
-//   k_velocity compute_V!                        :267-329
+//   k_cells    compute_P!                        :155-241   (sph_march.cuh)
+//   k_rheo_tau compute_TII! + copy_BC!(τII) + power_law!   :243-265 (FP64: k_rheo, sph_march.cuh)
+//   k_edot_law strain-rate power law (not in the reference; FP64: k_edot, sph_march.cuh)
+//   k_nodes    compute_V!                        :267-329   (sph_march.cuh)
 //   k_bc       BC_R! / BC_θ! / BC_φ! and the cyl/cart BC kernels
 // All three coordinate systems share the kernels; the metric terms come from
 // the template parameter G and the 1D tables in Geo.  The FP32 fused sweep in
@@ -21,6 +21,22 @@ namespace sph {
 // of the clamped interior cell (copy_bc_r!, copy_bc_θ!, copy_bc_φ! in that
 // order leave exactly that).  faces_only: CartesianStokes_diapir.jl:97-105
 // copies only face interiors and edges/corners keep η (ηSM .= η before maxloc!).
+//
+// The maximum is taken on integers in the numbers' order (a comparison in FP64 would cost FP64
+// issue, three of them per jmax): the bits of x with the magnitude of a negative x flipped, every
+// NaN above +inf, so that it propagates as in Julia's maximum.
+__device__ __forceinline__ long long order_bits(double x) {
+    const long long b = __double_as_longlong(x);
+    if ((b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) return 0x7fffffffffffffffLL;
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double from_order(long long b, double) { return __longlong_as_double(b ^ ((b >> 63) & 0x7fffffffffffffffLL)); }
+__device__ __forceinline__ int order_bits(float x) {
+    const int b = __float_as_int(x);
+    if ((b & 0x7fffffff) > 0x7f800000) return 0x7fffffff;
+    return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float from_order(int b, float) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); }
 template <typename T>
 __global__ void k_maxloc(KP<T> p, int faces_only) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
@@ -32,59 +48,10 @@ __global__ void k_maxloc(KP<T> p, int faces_only) {
     const int a = clampi(i, 1, d.n1 - 2), b = clampi(j, 1, d.n2 - 2), e = clampi(k, 1, d.n3 - 2);
     const int s = a + d.sy * b + d.sz * e;
     const T* E = p.eta;
-    p.etaSM[c] = jmax(jmax(jmax(jmax(E[s - 1], E[s + 1]), E[s]), jmax(E[s - d.sy], E[s + d.sy])), jmax(E[s - d.sz], E[s + d.sz]));
-}
-
-// ---------------------------------------------------------------------------
-// compute_P!: pressure, normal deviatoric stresses and DT_R at cells, shear
-// stresses at edges.  RHS: continuity right-hand side rP (correction problem:
-// P -= KBDT*(div δV + div V_fp64)).
-template <typename T, int G, bool RHS>
-__global__ void __launch_bounds__(256) k_stress(KP<T> p) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const Dims& d = p.d;
-    if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;
-    const int sy = d.sy, sz = d.sz;
-    const int c = i + sy * j + sz * k;
-    {
-        const CellD<T> D = cell_strain<T, G>(p.geo, p.d1, p.d2, p.d3, i, j, p.V1[c], p.V1[c + 1], p.V2[c], p.V2[c + sy], p.V3[c], p.V3[c + sz]);
-        const T sm = p.etaSM[c], e = p.eta[c];
-        const T gs = p.gsc * sm, kb = p.kbc * sm;
-        const T f = pdiv(e, e + gs);  // 1/(1 + GSDT/η)
-        T dv = D.div;
-        if (RHS) dv += p.rP[c];
-        T Pn = p.P[c] - kb * dv;
-        const T n11 = (p.t11[c] + T(2) * gs * D.D11) * f;
-        const T n22 = (p.t22[c] + T(2) * gs * D.D22) * f, n33 = (p.t33[c] + T(2) * gs * D.D33) * f;
-        if (p.traction) traction_pressure(j, k, d.n2, d.n3, n22, n33, p.sig2, p.sig3, Pn);
-        if (p.fs && i == d.n1 - 1) Pn = fs_pressure(n11, p.top_load ? p.top_load[c] : T(0), p.fs_kappa, p.V1[c], p.V1[c + 1]);
-        p.P[c] = Pn;
-        p.t11[c] = n11;
-        p.t22[c] = n22;
-        p.t33[c] = n33;
-        p.DT_R[c] = pdiv(p.vpdt2, kb + gs * f);
-    }
-    // τ12 at (i+1/2, j+1/2, k+1): cells (i|i+1, j|j+1, k+1)
-    if (i < d.n1 - 1 && j < d.n2 - 1 && k < d.n3 - 2) {
-        const int q = c + sz;
-        const T D = edge12<T, G>(p.geo, p.d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]);
-        p.t12[c] = edge_update(p.t12[c], p.gsc, p.etaSM[q] + p.etaSM[q + sy] + p.etaSM[q + 1] + p.etaSM[q + 1 + sy],
-                               p.eta[q] + p.eta[q + sy] + p.eta[q + 1] + p.eta[q + 1 + sy], D);
-    }
-    // τ13 at (i+1/2, j+1, k+1/2): cells (i|i+1, j+1, k|k+1)
-    if (i < d.n1 - 1 && j < d.n2 - 2 && k < d.n3 - 1) {
-        const int q = c + sy;
-        const T D = edge13<T, G>(p.geo, p.d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]);
-        p.t13[c] = edge_update(p.t13[c], p.gsc, p.etaSM[q] + p.etaSM[q + sz] + p.etaSM[q + 1] + p.etaSM[q + 1 + sz],
-                               p.eta[q] + p.eta[q + sz] + p.eta[q + 1] + p.eta[q + 1 + sz], D);
-    }
-    // τ23 at (i+1, j+1/2, k+1/2): cells (i+1, j|j+1, k|k+1)
-    if (i < d.n1 - 2 && j < d.n2 - 1 && k < d.n3 - 1) {
-        const int q = c + 1;
-        const T D = edge23<T, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]);
-        p.t23[c] = edge_update(p.t23[c], p.gsc, p.etaSM[q] + p.etaSM[q + sz] + p.etaSM[q + sy] + p.etaSM[q + sy + sz],
-                               p.eta[q] + p.eta[q + sz] + p.eta[q + sy] + p.eta[q + sy + sz], D);
-    }
+    auto m = order_bits(E[s]);
+    const int off[6] = {-1, 1, -d.sy, d.sy, -d.sz, d.sz};
+    for (int q = 0; q < 6; ++q) m = max(m, order_bits(E[s + off[q]]));
+    p.etaSM[c] = from_order(m, T(0));
 }
 
 // ---------------------------------------------------------------------------
@@ -159,35 +126,6 @@ __global__ void k_rheo_tau(KP<T> p, int faces_only, T n_exp) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// strain rates of the current velocities (as compute_P! forms them):
-// sDD = 0.5*(D11^2 + D22^2 + D33^2) at cells, s12/s13/s23 = engineering shear
-// strain rates at the edges.
-template <typename T, int G>
-__global__ void __launch_bounds__(256) k_strain(KP<T> p) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const Dims& d = p.d;
-    if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;
-    const int sy = d.sy, sz = d.sz;
-    const int c = i + sy * j + sz * k;
-    {
-        const CellD<T> D = cell_strain<T, G>(p.geo, p.d1, p.d2, p.d3, i, j, p.V1[c], p.V1[c + 1], p.V2[c], p.V2[c + sy], p.V3[c], p.V3[c + sz]);
-        p.sDD[c] = T(0.5) * (D.D11 * D.D11 + D.D22 * D.D22 + D.D33 * D.D33);
-    }
-    if (i < d.n1 - 1 && j < d.n2 - 1 && k < d.n3 - 2) {
-        const int q = c + sz;
-        p.s12[c] = edge12<T, G>(p.geo, p.d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]);
-    }
-    if (i < d.n1 - 1 && j < d.n2 - 2 && k < d.n3 - 1) {
-        const int q = c + sy;
-        p.s13[c] = edge13<T, G>(p.geo, p.d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]);
-    }
-    if (i < d.n1 - 2 && j < d.n2 - 1 && k < d.n3 - 1) {
-        const int q = c + 1;
-        p.s23[c] = edge23<T, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]);
-    }
-}
-
 // strain-rate power law (not in the reference): the invariant of the clamped
 // interior cell (as copy_BC! does for τII), η_t = 2/(1/η_ini + 1/η_PL),
 // η_PL = η_ini (edot_II/edot_bg)^((1-n)/n); RELAXED: η_out = η^(1-relax) η_t^relax.
@@ -258,31 +196,6 @@ __device__ __forceinline__ void momentum(const KP<T>& p, int I, int J, int K, T 
     }
 }
 
-// MODE 0: V += dV*avg(DT_R) with the ρg body force (reference compute_V!)
-// MODE 1: V += (dV + rV)*avg(DT_R), no gravity (correction problem)
-// MODE 2: rV = dV with gravity (residual evaluation, V unchanged)
-template <typename T, int G, int MODE>
-__global__ void __launch_bounds__(256) k_velocity(KP<T> p) {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x + 1, J = blockIdx.y * blockDim.y + threadIdx.y + 1, K = blockIdx.z + 1;
-    const Dims& d = p.d;
-    if (I > d.n1 - 1 || J > d.n2 - 1 || K > d.n3 - 1) return;
-    const int sy = d.sy, sz = d.sz;
-    const int c = I + sy * J + sz * K;
-    T dv[3];
-    bool ok[3];
-    momentum<T, G, MODE != 1, MODE == 1>(p, I, J, K, dv, ok);
-    const T h = T(0.5);
-    if (MODE == 2) {
-        if (ok[0]) p.rV1[c] = dv[0];
-        if (ok[1]) p.rV2[c] = dv[1];
-        if (ok[2]) p.rV3[c] = dv[2];
-    } else {
-        if (ok[0]) p.V1[c] = p.V1[c] + dv[0] * ((p.DT_R[c - 1] + p.DT_R[c]) * h);
-        if (ok[1]) p.V2[c] = p.V2[c] + dv[1] * ((p.DT_R[c - sy] + p.DT_R[c]) * h);
-        if (ok[2]) p.V3[c] = p.V3[c] + dv[2] * ((p.DT_R[c - sz] + p.DT_R[c]) * h);
-    }
-}
-
 // max |dV + rV| of the correction problem over the velocity nodes of block (bx, by, bz) into
 // *red (inner stopping test); 32 x 8 threads, the body of k_velocity_norm and of its batched
 // launch over many grids
@@ -315,40 +228,6 @@ __device__ __forceinline__ void velocity_norm_body(const KP<T>& p, int bx, int b
 template <typename T, int G>
 __global__ void __launch_bounds__(256) k_velocity_norm(KP<T> p) {
     velocity_norm_body<T, G>(p, blockIdx.x, blockIdx.y, blockIdx.z, p.red);
-}
-
-// viscous stresses of the current velocities: τ_ii = 2 η D_ii at cells,
-// τ_ij = avg4(η) D_ij at edges (the PT stress update's fixed point), and
-// rP = div V.  Used by the FP64 residual.
-template <typename T, int G>
-__global__ void __launch_bounds__(256) k_tau_visc(KP<T> p) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const Dims& d = p.d;
-    if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;
-    const int sy = d.sy, sz = d.sz;
-    const int c = i + sy * j + sz * k;
-    const T q4 = T(0.25);
-    {
-        const CellD<T> D = cell_strain<T, G>(p.geo, p.d1, p.d2, p.d3, i, j, p.V1[c], p.V1[c + 1], p.V2[c], p.V2[c + sy], p.V3[c], p.V3[c + sz]);
-        const T e2 = T(2) * p.eta[c];
-        p.t11[c] = e2 * D.D11; p.t22[c] = e2 * D.D22; p.t33[c] = e2 * D.D33;
-        p.rP[c] = D.div;
-    }
-    if (i < d.n1 - 1 && j < d.n2 - 1 && k < d.n3 - 2) {
-        const int q = c + sz;
-        const T aE = (p.eta[q] + p.eta[q + sy] + p.eta[q + 1] + p.eta[q + 1 + sy]) * q4;
-        p.t12[c] = aE * edge12<T, G>(p.geo, p.d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]);
-    }
-    if (i < d.n1 - 1 && j < d.n2 - 2 && k < d.n3 - 1) {
-        const int q = c + sy;
-        const T aE = (p.eta[q] + p.eta[q + sz] + p.eta[q + 1] + p.eta[q + 1 + sz]) * q4;
-        p.t13[c] = aE * edge13<T, G>(p.geo, p.d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]);
-    }
-    if (i < d.n1 - 2 && j < d.n2 - 1 && k < d.n3 - 1) {
-        const int q = c + 1;
-        const T aE = (p.eta[q] + p.eta[q + sz] + p.eta[q + sy] + p.eta[q + sy + sz]) * q4;
-        p.t23[c] = aE * edge23<T, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]);
-    }
 }
 
 // ---------------------------------------------------------------------------

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "sph_pt.cuh"
+#include "sph_march.cuh"
 #include "sph_fused.cuh"
 #include "sph_sweep.cuh"
 #include "sph_adjoint.cuh"
@@ -124,6 +125,7 @@ struct Ctx {
     bool use_pdl = true;  // sweep and BC kernels launched with a programmatic dependency (pdl_enter)
     bool fused = true;   // FP32 sweeps use the fused kernel
     int fused_chunk = 0; // planes per block of the fused sweep (0: chosen by fused_chunk())
+    int sms = 152;
     int fused_slots = 0; // resident blocks of the fused TMA sweep on the device (SMs x blocks per SM)
     double* adj = nullptr;  // adjoint arrays (AJ_COUNT slots of the box), allocated on first use
     // per-launch timing of the fused sweep kernel (sph_sweep_profile): event pairs
@@ -371,7 +373,8 @@ int alloc_state(Ctx& c, State<T>& s) {
     for (int i = 0; i < F_NSLOTS; ++i) s.f[i] = s.slab + (long long)i * vol;
     // tables: invRc[n1] invRh[n1] invSinC[n2] invSinH[n2] cotC[n2] cotH[n2] x1c[n1] x2c[n2] x3c[n3]
     const int n1 = c.d.n1, n2 = c.d.n2, n3 = c.d.n3;
-    size_t nt = 3 * (size_t)n1 + 4 * (size_t)n2 + (size_t)n2 + (size_t)n3;
+    const bool fp64 = sizeof(T) == 8;
+    size_t nt = 3 * (size_t)n1 + 4 * (size_t)n2 + (size_t)n2 + (size_t)n3 + (fp64 ? kPowTab : 0);
     std::vector<T> h(nt, T(1));
     T* w = h.data();
     T* invRc = w; w += n1;
@@ -383,6 +386,7 @@ int alloc_state(Ctx& c, State<T>& s) {
     T* x1c = w; w += n1;
     T* x2c = w; w += n2;
     T* x3c = w; w += n3;
+    if (fp64) fill_pow_tables(reinterpret_cast<double*>(w));
     for (int i = 0; i < n1; ++i) {
         x1c[i] = T(c.hx1[i]);
         invRc[i] = T(1.0 / c.hx1[i]);
@@ -411,6 +415,7 @@ int alloc_state(Ctx& c, State<T>& s) {
     s.geo.x1c = t; t += n1;
     s.geo.x2c = t; t += n2;
     s.geo.x3c = t; t += n3;
+    s.geo.pow_tab = fp64 ? t : nullptr;
     CK(cudaStreamSynchronize(c.stream));
     return SPH_OK;
 }
@@ -510,6 +515,41 @@ int sync64(Ctx& c) {
 }
 
 // ---------------------------------------------------------------------------
+// launches of the marching kernels (sph_march.cuh).  set-up of a column in planes of the march
+template <typename T, int G, int WHAT, bool RHS = false>
+void launch_cells(Ctx& c, const KP<T>& p) {
+    const long long cols = (long long)c.d.n1 * c.d.n2;
+    const int k = march_chunk(cols, c.d.n3, c.sms, 0.4);
+    k_cells<T, G, WHAT, RHS><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+}
+template <typename T, int G, int MODE>
+void launch_nodes(Ctx& c, const KP<T>& p) {
+    const long long cols = (long long)(c.d.n1 - 1) * (c.d.n2 - 1);
+    const int k = march_chunk(cols, c.d.n3 - 1, c.sms, 0.5);
+    k_nodes<T, G, MODE><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 - 1 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+}
+template <typename T, bool RELAXED>
+void launch_edot(Ctx& c, const KP<T>& p) {
+    if constexpr (sizeof(T) == 8) {
+        const long long cols = (long long)c.d.n1 * c.d.n2;
+        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1);
+        k_edot<RELAXED><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+    } else {
+        k_edot_law<T, RELAXED><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
+    }
+}
+template <typename T, bool RELAX>
+void launch_tau_law(Ctx& c, const KP<T>& p, int faces_only) {
+    if constexpr (sizeof(T) == 8) {
+        const long long cols = (long long)c.d.n1 * c.d.n2;
+        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1);
+        k_rheo<RELAX><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, faces_only, c.cur_n, k);
+    } else {
+        k_rheo_tau<T, RELAX><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
+    }
+}
+
+// ---------------------------------------------------------------------------
 // one reference PT iteration on state s
 // ηSM: `etasm_passes` applications of the 7-point max filter (maxloc! + copy_BC!);
 // intermediate passes go through the η_out scratch field, the last one into ηSM
@@ -528,17 +568,18 @@ void launch_maxloc(Ctx& c, KP<T>& p) {
     }
 }
 
+// strains: the strain rates are in their fields already (WHAT_STRESS_LAW)
 template <typename T, int G>
-void launch_rheology(Ctx& c, State<T>& s, KP<T>& p) {
+void launch_rheology(Ctx& c, State<T>& s, KP<T>& p, bool strains = false) {
     const int rh = c.prm.rheology;
     const int faces_only = (G == CART);
     if (rh == SPH_RHEO_TAU_POWER) {
-        k_rheo_tau<T, 0><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
+        launch_tau_law<T, false>(c, p, faces_only);
     } else if (rh == SPH_RHEO_TAU_POWER_RELAX) {
-        if (c.cur_n > 1.0) k_rheo_tau<T, 1><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
+        if (c.cur_n > 1.0) launch_tau_law<T, true>(c, p, faces_only);
     } else if (rh == SPH_RHEO_EDOT_POWER_RELAX) {
-        k_strain<T, G><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
-        k_edot_law<T, true><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
+        if (!strains) launch_cells<T, G, WHAT_STRAIN>(c, p);
+        launch_edot<T, true>(c, p);
         std::swap(s.f[F_ETA], s.f[F_ETA_OUT]);
         p.eta = s.f[F_ETA]; p.eta_out = s.f[F_ETA_OUT];
     }
@@ -548,9 +589,11 @@ template <typename T, int G>
 void iterate_one(Ctx& c, State<T>& s) {
     KP<T> p = make_kp<T>(c, s);
     launch_maxloc<T, G>(c, p);
-    k_stress<T, G, false><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
-    launch_rheology<T, G>(c, s, p);
-    k_velocity<T, G, 0><<<grid_vel(c.d), blk2d(), 0, c.stream>>>(p);
+    const bool law = c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX;
+    if (law) launch_cells<T, G, WHAT_STRESS_LAW>(c, p);
+    else launch_cells<T, G, WHAT_STRESS>(c, p);
+    launch_rheology<T, G>(c, s, p, law);
+    launch_nodes<T, G, 0>(c, p);
     launch_bc<T, G>(c, p, 0);
 }
 
@@ -817,19 +860,19 @@ int residual64_g(Ctx& c, double out[7], bool eta_from_law) {
     KP<double> p = make_kp<double>(c, s);
     const double* eta_eff = s.f[F_ETA];
     if (eta_from_law) {
-        k_strain<double, G><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
-        k_edot_law<double, false><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
+        launch_cells<double, G, WHAT_STRAIN>(c, p);
+        launch_edot<double, false>(c, p);
         eta_eff = s.f[F_ETA_OUT];
     }
     KP<double> r = p;
     r.eta = const_cast<double*>(eta_eff);
     r.t11 = s.f[F_Q11]; r.t22 = s.f[F_Q22]; r.t33 = s.f[F_Q33]; r.t12 = s.f[F_Q12]; r.t13 = s.f[F_Q13]; r.t23 = s.f[F_Q23];
-    k_tau_visc<double, G><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(r);
+    launch_cells<double, G, WHAT_VISC>(c, r);
     if (r.traction || r.fs) {
         k_traction_pressure<double><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(r, s.f[F_PRES]);
         r.P = s.f[F_PRES];
     }
-    k_velocity<double, G, 2><<<grid_vel(c.d), blk2d(), 0, c.stream>>>(r);
+    launch_nodes<double, G, 2>(c, r);
     CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
     launch_maxabs<double>(c, s.f[F_RV1], nullptr, 0);
     launch_maxabs<double>(c, s.f[F_RV2], nullptr, 1);
@@ -975,8 +1018,8 @@ int outer_residual(Ctx& c, double out[7]) {
     KP<double> p = make_kp<double>(c, s);
     const long long vol = c.d.vol;
     if (c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) {
-        k_strain<double, G><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
-        k_edot_law<double, false><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
+        launch_cells<double, G, WHAT_STRAIN>(c, p);
+        launch_edot<double, false>(c, p);
         CK(cudaMemcpyAsync(s.f[F_ETA], s.f[F_ETA_OUT], sizeof(double) * vol, cudaMemcpyDeviceToDevice, c.stream));
     }
     launch_bc<double, G>(c, p, 0);
@@ -1059,8 +1102,8 @@ void correction_sweep(Ctx& c) {
         c.ghost_stored = false;
         q = make_kp_corr(c);
     } else {
-        k_stress<float, G, true><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(q);
-        k_velocity<float, G, 1><<<grid_vel(c.d), blk2d(), 0, c.stream>>>(q);
+        launch_cells<float, G, WHAT_STRESS, true>(c, q);
+        launch_nodes<float, G, 1>(c, q);
     }
     if (bc) launch_bc<float, G>(c, q, 1);
 }
@@ -1780,6 +1823,7 @@ int sph_create(const sph_params* prm, void** out) {
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<SPH, 1>, SW_NT, sweep_smem_bytes()) == cudaSuccess)
             c->fused_slots = sms * per_sm;
+        if (sms > 0) c->sms = sms;
         cudaGetLastError();
     }
     if (const char* e = std::getenv("SPH_NO_GRAPHS")) c->use_graphs = std::atoi(e) == 0;
@@ -2027,8 +2071,8 @@ static KP<double> adj_kp(Ctx* c) {
     KP<double> p = make_kp<double>(*c, s);
     double* eta = adj_slot(c, AJ_ETA);
     if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) {
-        k_strain<double, G><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p);
-        k_edot_law<double, false><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p);
+        launch_cells<double, G, WHAT_STRAIN>(*c, p);
+        launch_edot<double, false>(*c, p);
         cudaMemcpyAsync(eta, s.f[F_ETA_OUT], sizeof(double) * c->d.vol, cudaMemcpyDeviceToDevice, c->stream);
     } else {
         cudaMemcpyAsync(eta, s.f[F_ETA], sizeof(double) * c->d.vol, cudaMemcpyDeviceToDevice, c->stream);
@@ -2675,17 +2719,17 @@ int sph_run_kernel(void* h, int32_t kernel) {
             if (G == SPH) launch_maxloc<double, SPH>(*c, p); else if (G == CYL) launch_maxloc<double, CYL>(*c, p); else launch_maxloc<double, CART>(*c, p);
             break;
         case SPH_K_COMPUTE_P:
-            if (G == SPH) k_stress<double, SPH, false><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p);
-            else if (G == CYL) k_stress<double, CYL, false><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p);
-            else k_stress<double, CART, false><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p);
+            if (G == SPH) launch_cells<double, SPH, WHAT_STRESS>(*c, p);
+            else if (G == CYL) launch_cells<double, CYL, WHAT_STRESS>(*c, p);
+            else launch_cells<double, CART, WHAT_STRESS>(*c, p);
             break;
         case SPH_K_RHEOLOGY:
             if (G == SPH) launch_rheology<double, SPH>(*c, s, p); else if (G == CYL) launch_rheology<double, CYL>(*c, s, p); else launch_rheology<double, CART>(*c, s, p);
             break;
         case SPH_K_COMPUTE_V:
-            if (G == SPH) k_velocity<double, SPH, 0><<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p);
-            else if (G == CYL) k_velocity<double, CYL, 0><<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p);
-            else k_velocity<double, CART, 0><<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p);
+            if (G == SPH) launch_nodes<double, SPH, 0>(*c, p);
+            else if (G == CYL) launch_nodes<double, CYL, 0>(*c, p);
+            else launch_nodes<double, CART, 0>(*c, p);
             break;
         case SPH_K_BC:
             if (G == SPH) launch_bc<double, SPH>(*c, p, 0); else if (G == CYL) launch_bc<double, CYL>(*c, p, 0); else launch_bc<double, CART>(*c, p, 0);
