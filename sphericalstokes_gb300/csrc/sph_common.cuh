@@ -64,6 +64,7 @@ struct KP {
     T kbc, gsc, vpdt2;                 // KBDT = kbc*ηSM, GSDT = gsc*ηSM, vpdt^2
     T g;
     T tau_C, n_exp, relax, edot_bg;
+    T law_i2, law_ex;                  // FP64 laws: 1/ε̇_bg², (n-1)/(2n) or 1/τ_C², (n-1)/2
     T sig2, sig3;                      // prescribed total normal stress on x2 / x3 faces
     int traction;                      // 1: boundary cells on x2/x3 faces take P = τ_nn - σ_bc
     int fs;                            // 1: top cells (i = n1-1) take the free-surface pressure (fs_pressure)

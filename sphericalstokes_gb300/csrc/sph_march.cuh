@@ -15,7 +15,10 @@
 // ragged n1 leaves no idle lanes (an idle lane costs as much FP64 time as a busy one).  Loads are
 // direct: neighbours come from L1, and their issue slots are free beside FP64 at 1/16 of a warp
 // instruction per clock.
-// MARCH_FIGURES
+// Measured on a GB300, 127^3 sector, strain-rate law, us (FP64 operations per cell): k_cells with the strain
+// rates kept 379 (97), k_edot 208 (54), k_nodes 205 (52), each with the FP64 units 86 - 88 % busy; one
+// point per thread, with separate strain-rate kernel and CUDA's pow, exp and log: compute_P! 537, strain rates 223,
+// law 642, compute_V! 310.  An iteration 838 (2071); Cartesian 207^3, relaxed stress law 3390 (7030).
 #pragma once
 #include "sph_math.cuh"
 
@@ -55,9 +58,11 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
     const CellMetric<T> m = cell_metric<T, G>(p, i, j);
     const EdgeMetric<T> e = edge_metric<T, G>(p.geo, i, j, d.n1, d.n2);
     const T a2 = m.a2, a3 = m.a3, e1 = h * m.e1, e2 = h * m.e2, third = T(-1.0 / 3.0);
-    const T e12_2 = e.iRh * p.d2, e12_h = -h * e.iRh;
-    const T e13_3 = G == SPH ? e.iRh * e.iSc1 * p.d3 : p.d3;
-    const T e23_2 = e.iRc1 * p.d2, e23_3 = G == SPH ? e.iRc1 * e.iSh * p.d3 : p.d3, e23_h = -h * e.iRc1 * e.ctH;
+    // (a difference and the sum of the same two values, d Δ + h (v + v'), as (d + h) Δ + 2 h v: one operation less)
+    const T e12_2 = e.iRh * p.d2, e1_d = G != CART ? p.d1 - h * e.iRh : p.d1, e1_v = -e.iRh;
+    const T e13_3 = G == SPH ? e.iRh * e.iSc1 * p.d3 : p.d3, e13_d = G == SPH ? e1_d : p.d1;
+    const T e23_2 = G == SPH ? e.iRc1 * p.d2 - h * e.iRc1 * e.ctH : e.iRc1 * p.d2, e23_v = -e.iRc1 * e.ctH;
+    const T e23_3 = G == SPH ? e.iRc1 * e.iSh * p.d3 : p.d3;
     const bool v12 = i < d.n1 - 1 && j < d.n2 - 1, v13 = i < d.n1 - 1 && j < d.n2 - 2, v23 = i < d.n1 - 2 && j < d.n2 - 1;
     int c = i + sy * j + sz * k0;
     // sums over two cells of a plane: X along x1 in row j + 1, Y along x2 in column i + 1
@@ -91,14 +96,14 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
         if (PT) {
             const T sm = p.etaSM[c], et = p.eta[c];
             const T gs = p.gsc * sm, kb = p.kbc * sm, gs2 = gs + gs;
-            const T f = fast_div(et, et + gs);  // 1/(1 + GSDT/η)
+            const T f = near_div(et, et + gs);  // 1/(1 + GSDT/η)
             T Pn = fma(-kb, RHS ? div + p.rP[c] : div, p.P[c]);
             const T n11 = fma(gs2, D11, p.t11[c]) * f, n22 = fma(gs2, D22, p.t22[c]) * f, n33 = fma(gs2, D33, p.t33[c]) * f;
             if (p.traction) traction_pressure(j, k, d.n2, d.n3, n22, n33, p.sig2, p.sig3, Pn);
             if (p.fs && i == d.n1 - 1) Pn = fs_pressure(n11, p.top_load ? p.top_load[c] : T(0), p.fs_kappa, p.V1[c], v1p);
             p.P[c] = Pn;
             p.t11[c] = n11; p.t22[c] = n22; p.t33[c] = n33;
-            p.DT_R[c] = fast_div(p.vpdt2, fma(gs, f, kb));
+            p.DT_R[c] = near_div(p.vpdt2, fma(gs, f, kb));
         } else if (WHAT == WHAT_VISC) {
             const T x = T(2) * p.eta[c];
             p.t11[c] = x * D11; p.t22[c] = x * D22; p.t33[c] = x * D33;
@@ -117,7 +122,7 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
         auto edge = [&](T* t, T* s, T D, T e4, T s4, bool ok) {
             if (PT) {  // (τ + aG D) aE / (aE + aG), aE = e4 / 4, aG = GSDT s4 / 4
                 const T g = gsc4 * s4;
-                const T v = fma(g, D, t[c]) * fast_div(e4, fma(T(4), g, e4));
+                const T v = fma(g, D, t[c]) * near_div(e4, fma(T(4), g, e4));
                 if (ok) t[c] = v;
             } else if (WHAT == WHAT_VISC) {
                 if (ok) t[c] = T(0.25) * e4 * D;
@@ -127,18 +132,18 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
         const T v1a = p.V1[u + 1], v1b = p.V1[u + 1 + sy], v2a = p.V2[u + sy], v2b = p.V2[u + sy + 1];
         const T v3q = p.V3[u + sy], v3t = p.V3[u + sy + 1], v3s = p.V3[u + 1];
         {
-            T D = fma(e12_2, v1b - v1a, p.d1 * (v2b - v2a));
-            if (G != CART) D = fma(e12_h, v2a + v2b, D);
+            T D = fma(e12_2, v1b - v1a, e1_d * (v2b - v2a));
+            if (G != CART) D = fma(e1_v, v2a, D);
             edge(p.t12, p.s12, D, eX0 + eXn, sX0 + sXn, v12 && k < d.n3 - 2);
         }
         {
-            T D = fma(e13_3, v1b - p.V1[c + 1 + sy], p.d1 * (v3t - v3q));
-            if (G == SPH) D = fma(e12_h, v3q + v3t, D);
+            T D = fma(e13_3, v1b - p.V1[c + 1 + sy], e13_d * (v3t - v3q));
+            if (G == SPH) D = fma(e1_v, v3q, D);
             edge(p.t13, p.s13, D, eX + eXn, sX + sXn, v13 && k < d.n3 - 1);
         }
         {
             T D = fma(e23_3, v2b - p.V2[c + 1 + sy], e23_2 * (v3t - v3s));
-            if (G == SPH) D = fma(e23_h, v3s + v3t, D);
+            if (G == SPH) D = fma(e23_v, v3s, D);
             edge(p.t23, p.s23, D, eY + eYn, sY + sYn, v23 && k < d.n3 - 1);
         }
         eX = eXn; eY = eYn; sX = sXn; sY = sYn;
@@ -157,12 +162,15 @@ __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p
     // the update wants the residual times (DT + DT') / 2: its half is folded into the coefficients
     const T s = MODE == 2 ? T(1) : T(0.5), h = T(0.5);
     const MomMetric<T> m = mom_metric<T, G>(p.geo, I, J, d.n1, d.n2);
+    // coefficients of differences, and of the lower value where its sum with the upper one enters too:
+    // d Δ + h (v + v') = (d + h) Δ + 2 h v
     const T c1 = s * p.d1;
-    const T m1_2 = s * m.iR1 * p.d2, m1_3 = s * (G == SPH ? m.iR1 * m.iS1 * p.d3 : p.d3), m1_n = s * (G == SPH ? m.iR1 : h * m.iR1);
-    const T m1_t = s * h * m.iR1 * m.ct1;
-    const T m2_2 = s * m.iR2 * p.d2, m2_3 = s * (G == SPH ? m.iR2 * m.iS2 * p.d3 : p.d3), m2_s = s * (G == SPH ? T(1.5) * m.iR2 : m.iR2);
-    const T m2_n = s * h * m.iR2 * m.ct2;
-    const T m3_3 = s * (G == SPH ? m.iR2 * m.iS3 * p.d3 : p.d3), m3_s = s * (G == SPH ? T(1.5) * m.iR2 : h * m.iR2), m3_n = s * m.iR2 * m.ct3;
+    const T m1_n = s * (G == SPH ? m.iR1 : h * m.iR1), m1_t = G == SPH ? s * h * m.iR1 * m.ct1 : T(0);
+    const T m1_1 = G == CART ? c1 : c1 + m1_n, m1_2 = s * m.iR1 * p.d2 + m1_t, m1_3 = s * (G == SPH ? m.iR1 * m.iS1 * p.d3 : p.d3);
+    const T m2_s = G == CART ? T(0) : s * (G == SPH ? T(1.5) * m.iR2 : m.iR2), m2_n = G == SPH ? s * h * m.iR2 * m.ct2 : T(0);
+    const T m2_1 = c1 + m2_s, m2_2 = s * m.iR2 * p.d2 + m2_n, m2_3 = s * (G == SPH ? m.iR2 * m.iS2 * p.d3 : p.d3);
+    const T m3_s = G == CART ? T(0) : s * (G == SPH ? T(1.5) * m.iR2 : h * m.iR2), m3_n = G == SPH ? s * m.iR2 * m.ct3 : T(0);
+    const T m3_1 = c1 + m3_s, m3_2 = s * m.iR2 * p.d2 + m3_n, m3_3 = s * (G == SPH ? m.iR2 * m.iS3 * p.d3 : p.d3);
     const T gh = -s * h * p.g;
     const bool w1 = J <= d.n2 - 2, w2 = I <= d.n1 - 2, w3 = w1 && w2;
     int c = I + sy * J + sz * K0;
@@ -183,12 +191,12 @@ __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p
         if (w1 && kin) {  // V1 (I-1/2, J, K), cell m = (I-1, J, K)
             const T Pm = p.P[c - 1], t12a = p.t12[c - 1 - sz];
             const T m11 = p.t11[c - 1] - Pm;
-            T r = fma(m1_3, t13b - p13b, fma(m1_2, t12a - t12b, c1 * (s11 - m11)));
+            T r = fma(m1_3, t13b - p13b, fma(m1_2, t12a - t12b, m1_1 * (s11 - m11)));
             if (G == SPH) {
                 const T m22 = p.t22[c - 1] - Pm, m33 = p.t33[c - 1] - Pm;
-                r = fma(m1_t, t12a + t12b, fma(m1_n, fma(-h, (m22 + s22) + (m33 + s33), m11 + s11), r));
+                r = fma(T(2) * m1_t, t12b, fma(m1_n, fma(-h, (m22 + s22) + (m33 + s33), m11 + m11), r));
             } else if (G == CYL) {
-                r = fma(m1_n, (m11 + s11) - (p.t22[c - 1] - Pm + s22), r);
+                r = fma(m1_n, (m11 + m11) - (p.t22[c - 1] - Pm + s22), r);
             }
             if (G != CART && MODE != 1) r = fma(gh, p.rho[c - 1] + p.rho[c], r);
             put(p.V1, p.rV1, r, MODE == 2 ? T(0) : p.DT_R[c - 1]);
@@ -196,16 +204,16 @@ __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p
         if (w2 && kin) {  // V2 (I, J-1/2, K), cell m = (I, J-1, K)
             const T Pm = p.P[c - sy];
             const T m22 = p.t22[c - sy] - Pm;
-            T r = fma(m2_3, t23 - p23, fma(m2_2, s22 - m22, c1 * (t12c - t12b)));
-            if (G != CART) r = fma(m2_s, t12c + t12b, r);
-            if (G == SPH) r = fma(m2_n, (m22 + s22) - (p.t33[c - sy] - Pm + s33), r);
+            T r = fma(m2_3, t23 - p23, fma(m2_2, s22 - m22, m2_1 * (t12c - t12b)));
+            if (G != CART) r = fma(T(2) * m2_s, t12b, r);
+            if (G == SPH) r = fma(m2_n, (m22 + m22) - (p.t33[c - sy] - Pm + s33), r);
             put(p.V2, p.rV2, r, MODE == 2 ? T(0) : p.DT_R[c - sy]);
         }
         if (w3) {  // V3 (I, J, K-1/2), cell m = (I, J, K-1)
             const T t23a = p.t23[c - 1 - sz];
-            T r = fma(m3_3, s33 - q33, fma(m2_2, t23a - p23, c1 * (p13a - p13b)));
-            if (G != CART) r = fma(m3_s, p13a + p13b, r);
-            if (G == SPH) r = fma(m3_n, t23a + p23, r);
+            T r = fma(m3_3, s33 - q33, fma(m3_2, t23a - p23, m3_1 * (p13a - p13b)));
+            if (G != CART) r = fma(T(2) * m3_s, p13b, r);
+            if (G == SPH) r = fma(T(2) * m3_n, p23, r);
             if (G == CART && MODE != 1) r = fma(gh, p.rho[c - sz] + p.rho[c], r);
             put(p.V3, p.rV3, r, qdt);
         }
@@ -224,29 +232,30 @@ __global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<doubl
     const int sy = d.sy, sz = d.sz;
     const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
     const double* tab = p.geo.pow_tab;
-    const double ib2 = 1.0 / (p.edot_bg * p.edot_bg), ex = 0.5 * (p.n_exp - 1.0) / p.n_exp;
     const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
     int last = -1;
-    double x = 0.0;
+    double x = 0.0, b0 = 0.0, q0 = 0.0;  // the invariant squared; sums of the edges below the next plane
     for (int k = k0; k < k1; ++k) {
         const int kc = clampi(k, 1, d.n3 - 2);
         const int c = i + sy * j + sz * k;
         if (kc != last) {
             const int s = s0 + sz * kc, e = s - 1 - sy - sz;
+            if (last < 0) { b0 = p.s13[e] + p.s13[e + 1]; q0 = p.s23[e] + p.s23[e + sy]; }
             const double a = (p.s12[e] + p.s12[e + sy]) + (p.s12[e + 1] + p.s12[e + 1 + sy]);
-            const double b = (p.s13[e] + p.s13[e + 1]) + (p.s13[e + sz] + p.s13[e + 1 + sz]);
-            const double q = (p.s23[e] + p.s23[e + sy]) + (p.s23[e + sz] + p.s23[e + sy + sz]);
+            const double b1 = p.s13[e + sz] + p.s13[e + 1 + sz], q1 = p.s23[e + sz] + p.s23[e + sy + sz];
+            const double b = b0 + b1, q = q0 + q1;
+            b0 = b1; q0 = q1;
             // (sums of four edges: a quarter of each, squared, times another quarter)
             x = fma(1.0 / 64.0, fma(a, a, fma(b, b, q * q)), p.sDD[s]);
             last = kc;
         }
         const double ei = p.eta_ini[c];
         double et = ei;
-        if (!(p.phase && p.phase[c])) et = fast_div(ei + ei, 1.0 + fast_pow(tab, x * ib2, ex));
+        if (!(p.phase && p.phase[c])) et = fast_div(ei + ei, 1.0 + fast_pow(tab, x * p.law_i2, p.law_ex));
         if (RELAXED) {
             const double eo = p.eta[c];
             // exact for the half-way mean; else η (η_t/η)^relax
-            et = p.relax == 0.5 ? sqrt(eo * et) : eo * fast_pow(tab, fast_div(et, eo), p.relax);
+            et = p.relax == 0.5 ? fast_sqrt(eo * et) : eo * fast_pow(tab, fast_div(et, eo), p.relax);
         }
         p.eta_out[c] = et;
     }
@@ -256,7 +265,7 @@ __global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<doubl
 // η_PL = η_ini x^((1-n)/2), η = 2 / (1/η_ini + 1/η_PL); RELAX: η_PL relaxed in log space
 // (CylindricalStokes_diapir.jl:185-192).  phase == 1 cells are linear.
 template <bool RELAX>
-__global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, double n_exp, int chunk) {
+__global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, int chunk) {
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -264,11 +273,10 @@ __global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<doubl
     const int sy = d.sy, sz = d.sz;
     const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
     const double* tab = p.geo.pow_tab;
-    const double ic2 = 1.0 / (p.tau_C * p.tau_C);
     const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
     const int rim = (i == 0 || i == d.n1 - 1) + (j == 0 || j == d.n2 - 1);
     int last = -1;
-    double t2c = 0.0, tiic = 0.0;
+    double t2c = 0.0, tiic = 0.0, b0 = 0.0, q0 = 0.0;
     for (int k = k0; k < k1; ++k) {
         const int c = i + sy * j + sz * k;
         double t2, tii;
@@ -279,19 +287,21 @@ __global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<doubl
             const int kc = clampi(k, 1, d.n3 - 2);
             if (kc != last) {
                 const int s = s0 + sz * kc, e = s - 1 - sy - sz;
+                if (last < 0) { b0 = p.t13[e] + p.t13[e + 1]; q0 = p.t23[e] + p.t23[e + sy]; }
                 const double a = (p.t12[e] + p.t12[e + sy]) + (p.t12[e + 1] + p.t12[e + 1 + sy]);
-                const double b = (p.t13[e] + p.t13[e + 1]) + (p.t13[e + sz] + p.t13[e + 1 + sz]);
-                const double q = (p.t23[e] + p.t23[e + sy]) + (p.t23[e + sz] + p.t23[e + sy + sz]);
+                const double b1 = p.t13[e + sz] + p.t13[e + 1 + sz], q1 = p.t23[e + sz] + p.t23[e + sy + sz];
+                const double b = b0 + b1, q = q0 + q1;
+                b0 = b1; q0 = q1;
                 const double x = p.t11[s], y = p.t22[s], z = p.t33[s];
                 t2c = fma(0.5, fma(x, x, fma(y, y, z * z)), 1.0 / 16.0 * fma(a, a, fma(b, b, q * q)));
-                tiic = sqrt(t2c);
+                tiic = fast_sqrt(t2c);
                 last = kc;
             }
             t2 = t2c;
             p.tII[c] = tii = tiic;
         }
-        const double cx = (p.phase && p.phase[c]) ? 0.0 : 0.5 * (n_exp - 1.0);
-        const double ei = p.eta_ini[c], x = t2 * ic2;
+        const double cx = (p.phase && p.phase[c]) ? 0.0 : p.law_ex;
+        const double ei = p.eta_ini[c], x = t2 * p.law_i2;
         if (!RELAX) {
             p.eta[c] = fast_div(ei + ei, 1.0 + fast_pow(tab, x, cx));
         } else {
@@ -317,7 +327,8 @@ __global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<doubl
                 pl = exp(log(pl) * p.relax + log(po) * (1.0 - p.relax));
             }
             p.eta_pl[c] = pl;
-            p.eta[c] = done ? fast_div((ei + ei) * pl, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
+            const double num = (ei + ei) * pl;
+            p.eta[c] = done && normal_pos(num) ? fast_div(num, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
         }
     }
 }

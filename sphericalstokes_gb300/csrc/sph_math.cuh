@@ -9,19 +9,36 @@
 
 namespace sph {
 
-// a / b in six FP64 operations: PTX's approximate reciprocal (relative error below 2^-20), one
-// third-order Newton (Householder) step r += r (e + e^2), e = 1 - b r, to 2^-60, and Markstein's
-// correction of the quotient by its residual, q += r (a - b q).  At most one unit in the last place from
-// the IEEE quotient for normal operands and quotients (viscosities, steps: no special cases kept).
-__device__ __forceinline__ double fast_div(double a, double b) {
+// a / b in five FP64 operations: PTX's approximate reciprocal r (relative error below 2^-20), the
+// quotient a r, and two corrections by its residual, q += r (a - b q), each of which multiplies the error
+// by that of r: to 2^-40, then below 2^-60 (Newton's iteration for the quotient, Markstein's last step).  At
+// most one unit in the last place from the IEEE quotient.  near_div: b and the quotient well inside the range
+// of normal numbers (sums of viscosities; a zero or infinite b gives NaN).  fast_div: any operands, those out
+// of the middle of the range (integer tests, no FP64 issue) by the IEEE division.
+__device__ __forceinline__ double near_div(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    const double e = fma(-b, r, 1.0);
-    r = fma(r, fma(e, e, e), r);
     const double q = a * r;
-    return fma(fma(-b, q, a), r, q);
+    const double q1 = fma(fma(-b, q, a), r, q);
+    return fma(fma(-b, q1, a), r, q1);
 }
-__device__ __forceinline__ float fast_div(float a, float b) { return pdiv(a, b); }
+__device__ __forceinline__ double fast_div(double a, double b) {
+    if ((__double2hiint(a) & 0x7fffffff) >= 0x7ff00000 || (unsigned)(__double2hiint(b) & 0x7fffffff) - 0x00300000u >= 0x7fa00000u) return a / b;
+    return near_div(a, b);
+}
+__device__ __forceinline__ float near_div(float a, float b) { return pdiv(a, b); }
+
+// square root of a positive normal x in seven FP64 operations: the approximate reciprocal root, one
+// coupled (Goldschmidt) step for the root and half its reciprocal, and the residual correction; others by sqrt()
+__device__ __forceinline__ double fast_sqrt(double x) {
+    if (!((unsigned)__double2hiint(x) - 0x00200000u < 0x7fc00000u)) return sqrt(x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double g = x * y, h = 0.5 * y;
+    const double e = fma(-g, h, 0.5);
+    const double g1 = fma(g, e, g);
+    return fma(fma(-g1, g1, x), fma(h, e, h), g1);
+}
 
 // ---------------------------------------------------------------------------
 // x^c of positive normal numbers, after the table-driven scheme of P. T. P. Tang (ACM TOMS 15-18, 1989-1992):

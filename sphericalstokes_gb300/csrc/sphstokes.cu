@@ -202,6 +202,9 @@ KP<T> make_kp(Ctx& c, State<T>& s) {
     p.vpdt2 = T(q.vpdt * q.vpdt);
     p.g = T(q.g);
     p.tau_C = T(q.tau_C); p.n_exp = T(c.cur_n); p.relax = T(q.relax); p.edot_bg = T(q.edot_bg);
+    const bool ed = q.rheology == SPH_RHEO_EDOT_POWER_RELAX;
+    p.law_i2 = T(ed ? 1.0 / (q.edot_bg * q.edot_bg) : 1.0 / (q.tau_C * q.tau_C));
+    p.law_ex = T(0.5 * (c.cur_n - 1.0) / (ed ? c.cur_n : 1.0));
     p.sig2 = T(q.sig_bc[1]); p.sig3 = T(q.sig_bc[2]);
     p.traction = q.bc == SPH_BC_STRESS ? 1 : 0;
     p.fs = q.bc == SPH_BC_FREE_SURFACE ? 1 : 0;
@@ -543,7 +546,7 @@ void launch_tau_law(Ctx& c, const KP<T>& p, int faces_only) {
     if constexpr (sizeof(T) == 8) {
         const long long cols = (long long)c.d.n1 * c.d.n2;
         const int k = march_chunk(cols, c.d.n3, c.sms, 0.1);
-        k_rheo<RELAX><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, faces_only, c.cur_n, k);
+        k_rheo<RELAX><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, faces_only, k);
     } else {
         k_rheo_tau<T, RELAX><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
     }
