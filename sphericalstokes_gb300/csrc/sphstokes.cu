@@ -2034,9 +2034,12 @@ static int write_file(const std::string& path, const void* data, size_t bytes) {
 // ---------------------------------------------------------------------------
 // adjoint of the FP64 residual (sph_adjoint.cuh)
 enum AdjSlot {
-    AJ_LV1, AJ_LV2, AJ_LV3, AJ_LP, AJ_S11, AJ_S22, AJ_S33, AJ_T12, AJ_T13, AJ_T23,
-    AJ_V1, AJ_V2, AJ_V3, AJ_P, AJ_GETA, AJ_GRHO, AJ_B1, AJ_B2, AJ_B3, AJ_BP, AJ_R1, AJ_R2, AJ_R3, AJ_RP, AJ_ETA,
-    AJ_GEI, AJ_GN, AJ_M11, AJ_M22, AJ_M33, AJ_M12, AJ_M13, AJ_M23, AJ_COUNT
+    AJ_LV1, AJ_LV2, AJ_LV3, AJ_LP, AJ_V1, AJ_V2, AJ_V3, AJ_P, AJ_GETA, AJ_GRHO, AJ_B1, AJ_B2, AJ_B3, AJ_BP, AJ_R1, AJ_R2, AJ_R3, AJ_RP, AJ_ETA,
+    AJ_GEI, AJ_GN, AJ_M11, AJ_M22, AJ_M33, AJ_M12, AJ_M13, AJ_M23,  // memory of the transposed PT
+    AJ_D11, AJ_D22, AJ_D33, AJ_E12, AJ_E13, AJ_E23,                 // adjoints of the strain rates (no memory)
+    AJ_X12, AJ_X13, AJ_X23, AJ_Q12, AJ_Q13, AJ_Q23, AJ_O1, AJ_O2, AJ_O3, AJ_O4, AJ_O5, AJ_GW,
+    AJ_FC, AJ_WC, AJ_F12, AJ_F13, AJ_F23, AJ_W12, AJ_W13, AJ_W23, AJ_C11, AJ_C22, AJ_C33, AJ_G12, AJ_G13, AJ_G23,
+    AJ_LW, AJ_LR, AJ_LA, AJ_LB, AJ_LC, AJ_COUNT
 };
 
 static int adj_alloc(Ctx* c) {
@@ -2088,40 +2091,81 @@ static KP<double> adj_kp(Ctx* c) {
     return p;
 }
 
-static Adj adj_ptrs(Ctx* c) {
+// mem: the iteration of the transposed solve (adjoints of the strain rates are the memory)
+static Adj adj_ptrs(Ctx* c, bool mem) {
+    auto s = [&](int i) { return adj_slot(c, i); };
     Adj a;
-    a.lV1 = adj_slot(c, AJ_LV1); a.lV2 = adj_slot(c, AJ_LV2); a.lV3 = adj_slot(c, AJ_LV3); a.lP = adj_slot(c, AJ_LP);
-    a.aS11 = adj_slot(c, AJ_S11); a.aS22 = adj_slot(c, AJ_S22); a.aS33 = adj_slot(c, AJ_S33);
-    a.aT12 = adj_slot(c, AJ_T12); a.aT13 = adj_slot(c, AJ_T13); a.aT23 = adj_slot(c, AJ_T23);
-    a.aV1 = adj_slot(c, AJ_V1); a.aV2 = adj_slot(c, AJ_V2); a.aV3 = adj_slot(c, AJ_V3); a.aP = adj_slot(c, AJ_P);
-    a.gEta = adj_slot(c, AJ_GETA); a.gRho = adj_slot(c, AJ_GRHO);
+    a.lV1 = s(AJ_LV1); a.lV2 = s(AJ_LV2); a.lV3 = s(AJ_LV3); a.lP = s(AJ_LP); a.bP = s(AJ_BP);
+    const int d = mem ? AJ_M11 : AJ_D11;
+    a.d11 = s(d); a.d22 = s(d + 1); a.d33 = s(d + 2); a.e12 = s(d + 3); a.e13 = s(d + 4); a.e23 = s(d + 5);
+    a.x12 = s(AJ_X12); a.x13 = s(AJ_X13); a.x23 = s(AJ_X23); a.q12 = s(AJ_Q12); a.q13 = s(AJ_Q13); a.q23 = s(AJ_Q23);
+    a.E1 = s(AJ_O1); a.M1 = s(AJ_O2); a.E2 = s(AJ_O3); a.M2 = s(AJ_O4); a.E3 = s(AJ_O5);
+    a.aV1 = s(AJ_V1); a.aV2 = s(AJ_V2); a.aV3 = s(AJ_V3); a.aP = s(AJ_P);
+    a.gEta = s(AJ_GETA); a.gRho = s(AJ_GRHO); a.gW = s(AJ_GW);
+    a.fc = s(AJ_FC); a.wc = s(AJ_WC);
+    a.f12 = s(AJ_F12); a.f13 = s(AJ_F13); a.f23 = s(AJ_F23); a.w12 = s(AJ_W12); a.w13 = s(AJ_W13); a.w23 = s(AJ_W23);
+    a.c11 = s(AJ_C11); a.c22 = s(AJ_C22); a.c33 = s(AJ_C33); a.g12 = s(AJ_G12); a.g13 = s(AJ_G13); a.g23 = s(AJ_G23);
+    a.lw = s(AJ_LW); a.lr = s(AJ_LR); a.la = s(AJ_LA); a.lb = s(AJ_LB); a.lc = s(AJ_LC);
     return a;
+}
+
+static dim3 adj_cells(const Ctx* c, int chunk) {
+    return dim3((unsigned)(((long long)c->d.n1 * c->d.n2 + MC_NT - 1) / MC_NT), (c->d.n3 + chunk - 1) / chunk);
+}
+
+// the transposed homogeneous BC program on the velocity adjoints
+template <int G>
+static void adj_bc(Ctx* c, const KP<double>& p, const Adj& a) {
+    KP<double> hp = p;
+    hp.sig2 = 0.0; hp.sig3 = 0.0;
+    for (auto st = c->bc.rbegin(); st != c->bc.rend(); ++st) {
+        int eu = st->dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
+        int ev = st->dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
+        dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
+        k_bc_adjoint<G><<<g, blk2d(), 0, c->stream>>>(hp, a, *st);
+    }
+}
+
+// the fixed factors of the state behind p (after adj_kp)
+template <int G>
+static void adj_setup(Ctx* c, const KP<double>& p) {
+    const Adj a = adj_ptrs(c, false);
+    if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) k_adj_setup<G, true><<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a);
+    else k_adj_setup<G, false><<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a);
+}
+
+// λ_V, λ_P -> adjoints of V (all entries); MEM: one update of the memory and of λ_P on the way
+template <int G, bool MEM>
+static void adj_rows(Ctx* c, const KP<double>& p, const Adj& a) {
+    const bool law = c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX;
+    const long long cols = (long long)c->d.n1 * c->d.n2;
+    const int ks = march_chunk(cols, c->d.n3, c->sms, 0.6), kl = march_chunk(cols, c->d.n3, c->sms, 0.2);
+    if (law) k_adj_stress<G, MEM, true><<<adj_cells(c, ks), MC_NT, 0, c->stream>>>(p, a, ks);
+    else k_adj_stress<G, MEM, false><<<adj_cells(c, ks), MC_NT, 0, c->stream>>>(p, a, ks);
+    if (law) {
+        k_adj_eta<true><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
+        k_adj_law<G><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
+    } else if (!MEM) {
+        k_adj_eta<false><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
+    }
+    const long long nodes = (long long)(c->d.n1 + 1) * (c->d.n2 + 1);
+    const int kn = march_chunk(nodes, c->d.n3 + 1, c->sms, 0.6);
+    const dim3 gn((unsigned)((nodes + MC_NT - 1) / MC_NT), (c->d.n3 + 1 + kn - 1) / kn);
+    if (law) k_adj_strain<G><<<gn, MC_NT, 0, c->stream>>>(p, a, a.x12, a.x13, a.x23, kn);
+    else k_adj_strain<G><<<gn, MC_NT, 0, c->stream>>>(p, a, a.e12, a.e13, a.e23, kn);
 }
 
 // Aᵀ λ (λ in the AJ_L* slots) into AJ_V*, AJ_P, with ∂R/∂η, ∂R/∂ρ contractions; with_bc: the
 // transposed homogeneous BC program (interior-unknown form)
 template <int G>
 static int adj_apply(Ctx* c, KP<double>& p, bool with_bc) {
-    Adj a = adj_ptrs(c);
-    CK(cudaMemsetAsync(adj_slot(c, AJ_S11), 0, sizeof(double) * c->d.vol * (AJ_GRHO - AJ_S11 + 1), c->stream));
-    k_vjp_momentum<G><<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p, a);
-    k_vjp_pressure<<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a);
-    k_vjp_strain<G><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a);
-    if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX)  // the law's dependence on V (Newton form) and its η_ini, n chain
-        k_vjp_law<G, true><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_GEI), adj_slot(c, AJ_GN));
+    const Adj a = adj_ptrs(c, false);
+    adj_rows<G, false>(c, p, a);
+    if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX)
+        k_adj_law_params<<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a, adj_slot(c, AJ_GEI), adj_slot(c, AJ_GN));
     else
         CK(cudaMemcpyAsync(adj_slot(c, AJ_GEI), adj_slot(c, AJ_GETA), sizeof(double) * c->d.vol, cudaMemcpyDeviceToDevice, c->stream));
-    if (with_bc) {
-        KP<double> hp = p;
-        hp.sig2 = 0.0; hp.sig3 = 0.0;
-        for (auto it = c->bc.rbegin(); it != c->bc.rend(); ++it) {
-            const BcStage& st = *it;
-            int eu = st.dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
-            int ev = st.dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
-            dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
-            k_bc_adjoint<G><<<g, blk2d(), 0, c->stream>>>(hp, a, st);
-        }
-    }
+    if (with_bc) adj_bc<G>(c, p, a);
     CK(cudaGetLastError());
     return SPH_OK;
 }
@@ -2129,7 +2173,8 @@ static int adj_apply(Ctx* c, KP<double>& p, bool with_bc) {
 template <int G>
 static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf) {
     KP<double> p = adj_kp<G>(c);
-    Adj a = adj_ptrs(c);
+    adj_setup<G>(c, p);
+    const Adj a = adj_ptrs(c, true);
     const int nout = o.nout > 0 ? o.nout : 100;
     // max|b|
     CK(cudaMemsetAsync(c->red, 0, sizeof(unsigned long long) * kRedSlots, c->stream));
@@ -2139,33 +2184,15 @@ static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf)
     double bmax = 0.0;
     for (int s = 0; s < 4; ++s) bmax = std::max(bmax, slot_val(*c, s));
     if (bmax == 0.0) bmax = 1.0;
-    for (int s = AJ_M11; s <= AJ_M23; ++s) CK(cudaMemsetAsync(adj_slot(c, s), 0, sizeof(double) * c->d.vol, c->stream));
-    const bool law = c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX;
+    CK(cudaMemsetAsync(adj_slot(c, AJ_M11), 0, sizeof(double) * c->d.vol * (AJ_M23 - AJ_M11 + 1), c->stream));
     dim3 gu((c->d.n1 + 1 + 31) / 32, (c->d.n2 + 1 + 7) / 8, c->d.n3 + 1);
     int64_t it = 0;
     double err = 1.0;
     int status = SPH_ERR_NOT_CONVERGED;
     while (it < o.maxiter) {
         ++it;
-        // M_τᵀ λ_V (σ adjoints -> τ adjoints) and M_Pᵀ λ_V
-        CK(cudaMemsetAsync(adj_slot(c, AJ_S11), 0, sizeof(double) * c->d.vol * (AJ_GRHO - AJ_S11 + 1), c->stream));
-        k_vjp_momentum<G><<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p, a);
-        k_vjp_pressure<<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a);
-        k_adj_pressure_update<<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_LP), adj_slot(c, AJ_BP));
-        k_adj_memory<<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_M11), adj_slot(c, AJ_M22), adj_slot(c, AJ_M33),
-                                                                  adj_slot(c, AJ_M12), adj_slot(c, AJ_M13), adj_slot(c, AJ_M23));
-        k_vjp_strain<G><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a);  // Eᵀ μ + Dᵀ λ_P
-        if (law) k_vjp_law<G, true><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_GEI), adj_slot(c, AJ_GN));
-        {
-            KP<double> hp = p;
-            hp.sig2 = 0.0; hp.sig3 = 0.0;
-            for (auto st = c->bc.rbegin(); st != c->bc.rend(); ++st) {
-                int eu = st->dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
-                int ev = st->dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
-                dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
-                k_bc_adjoint<G><<<g, blk2d(), 0, c->stream>>>(hp, a, *st);
-            }
-        }
+        adj_rows<G, true>(c, p, a);  // M_τᵀ λ_V, M_Pᵀ λ_V, Eᵀ μ + Dᵀ λ_P
+        adj_bc<G>(c, p, a);
         k_adj_velocity_update<<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_LV1), adj_slot(c, AJ_LV2), adj_slot(c, AJ_LV3),
                                                                          adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3));
         if (it % nout) continue;
@@ -2353,9 +2380,9 @@ int sph_residual_vjp(void* h, const double* lV1, const double* lV2, const double
         return rc;
     const int G = c->prm.geometry;
     const bool bc = (flags & 1) != 0;
-    if (G == SPH) { KP<double> p = adj_kp<SPH>(c); rc = adj_apply<SPH>(c, p, bc); }
-    else if (G == CYL) { KP<double> p = adj_kp<CYL>(c); rc = adj_apply<CYL>(c, p, bc); }
-    else { KP<double> p = adj_kp<CART>(c); rc = adj_apply<CART>(c, p, bc); }
+    if (G == SPH) { KP<double> p = adj_kp<SPH>(c); adj_setup<SPH>(c, p); rc = adj_apply<SPH>(c, p, bc); }
+    else if (G == CYL) { KP<double> p = adj_kp<CYL>(c); adj_setup<CYL>(c, p); rc = adj_apply<CYL>(c, p, bc); }
+    else { KP<double> p = adj_kp<CART>(c); adj_setup<CART>(c, p); rc = adj_apply<CART>(c, p, bc); }
     if (rc) return rc;
     if ((rc = adj_download(c, AJ_V1, SPH_FIELD_V1, aV1)) || (rc = adj_download(c, AJ_V2, SPH_FIELD_V2, aV2)) ||
         (rc = adj_download(c, AJ_V3, SPH_FIELD_V3, aV3)) || (rc = adj_download(c, AJ_P, SPH_FIELD_P, aP)) ||
@@ -2435,16 +2462,11 @@ int sph_bc_vjp(void* h, double* aV1, double* aV2, double* aV3) {
         return rc;
     KP<double> p = make_kp<double>(*c, c->s64);
     p.sig2 = 0.0; p.sig3 = 0.0;
-    Adj a = adj_ptrs(c);
+    const Adj a = adj_ptrs(c, false);
     const int G = c->prm.geometry;
-    for (auto st = c->bc.rbegin(); st != c->bc.rend(); ++st) {
-        int eu = st->dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
-        int ev = st->dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
-        dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
-        if (G == SPH) k_bc_adjoint<SPH><<<g, blk2d(), 0, c->stream>>>(p, a, *st);
-        else if (G == CYL) k_bc_adjoint<CYL><<<g, blk2d(), 0, c->stream>>>(p, a, *st);
-        else k_bc_adjoint<CART><<<g, blk2d(), 0, c->stream>>>(p, a, *st);
-    }
+    if (G == SPH) adj_bc<SPH>(c, p, a);
+    else if (G == CYL) adj_bc<CYL>(c, p, a);
+    else adj_bc<CART>(c, p, a);
     CK(cudaGetLastError());
     if ((rc = adj_download(c, AJ_V1, SPH_FIELD_V1, aV1)) || (rc = adj_download(c, AJ_V2, SPH_FIELD_V2, aV2)) ||
         (rc = adj_download(c, AJ_V3, SPH_FIELD_V3, aV3)))
