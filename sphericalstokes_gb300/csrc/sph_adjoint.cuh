@@ -19,9 +19,11 @@
 // derivative) are made once by k_adj_setup.
 //   k_adj_stress   λ_V -> adjoint of σ, τ (cells, edges), of P; MEM: μ and λ_P updated
 //   k_adj_eta      per cell λᵀ ∂R/∂η (and, for the law, that times dη_t/dε̇)
-//   k_adj_law      the law's dependence on V added to the adjoints of the strain rates
+//   k_adj_collect, k_adj_law   the law's dependence on V added to the adjoints of the strain rates
 //   k_adj_strain   adjoints of strain rates and div V -> V (all entries)
-// ADJOINT_FIGURES
+// Measured on a GB300, 63^3 sector under the strain-rate law: 125 us per transposed iteration (820 with
+// scatters by FP64 atomics and coefficients evaluated as stencils of unit vectors), the FP64 units 63 - 78 %
+// busy in the cell and node kernels; the rest is the five BC stages and launches.
 #pragma once
 #include "sph_march.cuh"
 #include "sph_pt.cuh"
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(MC_NT) k_adj_setup(const __grid_constant__ KP<
 // the adjoints of the strain rates themselves, of P and ρ.  LAW: k_adj_law finishes the cells.
 template <int G, bool MEM, bool LAW>
 __global__ void __launch_bounds__(MC_NT) k_adj_stress(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -208,6 +211,7 @@ __global__ void __launch_bounds__(MC_NT) k_adj_stress(const __grid_constant__ KP
 // λᵀ ∂R/∂η per cell: the cell's own part and its twelve edges'; times the law's derivative for k_adj_law
 template <bool LAW>
 __global__ void __launch_bounds__(MC_NT) k_adj_eta(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -228,10 +232,25 @@ __global__ void __launch_bounds__(MC_NT) k_adj_eta(const __grid_constant__ KP<do
     }
 }
 
-// The law: η of a cell follows ε̇ of its clamped interior cell s, so s collects gW of the cells clamped to it and
-// passes it on to the strain rates that form ε̇(s)
+// The law: η of a cell follows ε̇ of its clamped interior cell s.  First the interior cells next to the
+// boundary collect gW of the boundary cells clamped to them, in place (boundary cells are only read) ...
+__global__ void __launch_bounds__(256) k_adj_collect(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a) {
+    pdl_enter_small();
+    const Dims& d = p.d;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y, z = blockIdx.z;
+    const int n1 = d.n1, n2 = d.n2, n3 = d.n3, sy = d.sy, sz = d.sz;
+    if (x < 1 || y < 1 || z < 1 || x > n1 - 2 || y > n2 - 2 || z > n3 - 2) return;
+    if (x != 1 && y != 1 && z != 1 && x != n1 - 2 && y != n2 - 2 && z != n3 - 2) return;
+    double h = 0.0;
+    for (int dz = (z == 1 ? -1 : 0); dz <= (z == n3 - 2 ? 1 : 0); ++dz)
+        for (int dy = (y == 1 ? -1 : 0); dy <= (y == n2 - 2 ? 1 : 0); ++dy)
+            for (int dx = (x == 1 ? -1 : 0); dx <= (x == n1 - 2 ? 1 : 0); ++dx) h += a.gW[x + dx + sy * (y + dy) + sz * (z + dz)];
+    a.gW[x + sy * y + sz * z] = h;
+}
+// ... then s passes it on to the strain rates that form ε̇(s) (the factors of boundary cells are zero)
 template <int G>
 __global__ void __launch_bounds__(MC_NT) k_adj_law(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -240,30 +259,18 @@ __global__ void __launch_bounds__(MC_NT) k_adj_law(const __grid_constant__ KP<do
     const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, n3);
     const CellMetric<double> m = cell_metric<double, G>(p, i, j);
     const bool e12 = i < n1 - 1 && j < n2 - 1, e13 = i < n1 - 1 && j < n2 - 2, e23 = i < n1 - 2 && j < n2 - 1;
-    const bool edge_col = i <= 2 || j <= 2 || i >= n1 - 3 || j >= n2 - 3;
-    auto collect = [&](int x, int y, int z) {
-        if (x < 1 || y < 1 || z < 1 || x > n1 - 2 || y > n2 - 2 || z > n3 - 2) return 0.0;
-        double h = 0.0;
-        for (int dz = (z == 1 ? -1 : 0); dz <= (z == n3 - 2 ? 1 : 0); ++dz)
-            for (int dy = (y == 1 ? -1 : 0); dy <= (y == n2 - 2 ? 1 : 0); ++dy)
-                for (int dx = (x == 1 ? -1 : 0); dx <= (x == n1 - 2 ? 1 : 0); ++dx) h += a.gW[x + dx + sy * (y + dy) + sz * (z + dz)];
-        return h;
-    };
     for (int k = k0; k < k1; ++k) {
-        const int c = i + sy * j + sz * k;
-        const bool plain = !edge_col && k > 2 && k < n3 - 3;  // the cell and its upper neighbours: interior, nothing clamped to them
-        auto H = [&](int x, int y, int z) { return plain ? a.gW[c + x + sy * y + sz * z] : collect(i + x, j + y, k + z); };
-        const double h = H(0, 0, 0) * a.lr[c];
+        const int c = i + sy * j + sz * k, q = c + sz;
+        const double *H = a.gW;
+        const double h = H[c] * a.lr[c];
         cell_out<G>(m, p.d1, a, c, fma(h, a.c11[c], a.d11[c]), fma(h, a.c22[c], a.d22[c]), fma(h, a.c33[c], a.d33[c]), a.lP[c]);
-        const int q = c + sz;
-        const double H111 = H(1, 1, 1);
-        const int q111 = q + sy + 1;
+        const int o = sy + 1;
         if (e12 && k < n3 - 2)
-            a.x12[c] = a.e12[c] + (fma(H(0, 0, 1), a.la[q], H(1, 0, 1) * a.la[q + 1]) + fma(H(0, 1, 1), a.la[q + sy], H111 * a.la[q111]));
+            a.x12[c] = a.e12[c] + (fma(H[q], a.la[q], H[q + 1] * a.la[q + 1]) + fma(H[q + sy], a.la[q + sy], H[q + o] * a.la[q + o]));
         if (e13 && k < n3 - 1)
-            a.x13[c] = a.e13[c] + (fma(H(0, 1, 0), a.lb[c + sy], H(1, 1, 0) * a.lb[c + sy + 1]) + fma(H(0, 1, 1), a.lb[q + sy], H111 * a.lb[q111]));
+            a.x13[c] = a.e13[c] + (fma(H[c + sy], a.lb[c + sy], H[c + o] * a.lb[c + o]) + fma(H[q + sy], a.lb[q + sy], H[q + o] * a.lb[q + o]));
         if (e23 && k < n3 - 1)
-            a.x23[c] = a.e23[c] + (fma(H(1, 0, 0), a.lc[c + 1], H(1, 1, 0) * a.lc[c + 1 + sy]) + fma(H(1, 0, 1), a.lc[q + 1], H111 * a.lc[q111]));
+            a.x23[c] = a.e23[c] + (fma(H[c + 1], a.lc[c + 1], H[c + o] * a.lc[c + o]) + fma(H[q + 1], a.lc[q + 1], H[q + o] * a.lc[q + o]));
     }
 }
 
@@ -271,6 +278,7 @@ __global__ void __launch_bounds__(MC_NT) k_adj_law(const __grid_constant__ KP<do
 template <int G>
 __global__ void __launch_bounds__(MC_NT) k_adj_strain(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, const double* __restrict__ X12,
                                                       const double* __restrict__ X13, const double* __restrict__ X23, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int w = d.n1 + 1;
@@ -360,69 +368,53 @@ __global__ void __launch_bounds__(MC_NT) k_adj_law_params(const __grid_constant_
     gN[c] = ed > 0.0 ? -g * et * et * log(ed / p.edot_bg) / (2.0 * pl * n * n) : 0.0;
 }
 
-// normal-velocity ghost of the far-field-stress BC (k_bc, BC_STRESS) as a function of its
-// inputs: V1 at the boundary cell's two r-faces, the other tangential component's two
-// faces, and the normal component one node inside (vin)
-template <int G>
-__device__ __forceinline__ double stress_ghost(const KP<double>& p, int D, int side, int i, int j, double v1a, double v1b, double wa,
-                                               double wb, double vin) {
-    const CellMetric<double> m = cell_metric<double, G>(p, i, j);
-    const double sgn = side == 0 ? -1.0 : 1.0;
-    const double avx = (v1a + v1b) * 0.5;
-    double A0, B;
-    if (D == 1) {  // wa, wb = V3 at cc, cc + sz
-        A0 = p.d1 * (v1b - v1a) + m.a3 * (wb - wa) + m.c1 * avx + m.a2 * (-sgn) * vin + m.c2 * 0.5 * vin;
-        B = m.a2 * sgn + 0.5 * m.c2;
-    } else {  // wa, wb = V2 at cc, cc + sy
-        const double avy = (wa + wb) * 0.5;
-        A0 = p.d1 * (v1b - v1a) + m.a2 * (wb - wa) + m.c1 * avx + m.c2 * avy + m.a3 * (-sgn) * vin;
-        B = m.a3 * sgn;
-    }
-    return -A0 / B;
-}
-
-// transpose of one homogeneous BC stage on the velocity adjoints: each boundary entry's
-// adjoint goes back to the entries its value was computed from, then is cleared
-template <int G>
-__global__ void k_bc_adjoint(KP<double> p, Adj a, BcStage st) {
+// transpose of one homogeneous BC stage (faces normal to axis D) on the velocity adjoints: each boundary
+// entry's adjoint goes back to the entries its value was computed from, then is cleared
+template <int G, int D>
+__global__ void k_bc_adjoint(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, const __grid_constant__ BcStage st) {
+    pdl_enter_small();
     const int u = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y * blockDim.y + threadIdx.y;
     const Dims& d = p.d;
-    const int D = st.dim;
     const int sy = d.sy, sz = d.sz;
+    const int step = D == 0 ? 1 : (D == 1 ? sy : sz);
+    const int base = D == 0 ? u * sy + v * sz : (D == 1 ? u + v * sz : u + v * sy);
     for (int o = st.nops - 1; o >= 0; --o) {
-        const BcOp op = st.op[o];
-        const int f = op.field;
-        int ext[3] = {d.n1 + (f == 0), d.n2 + (f == 1), d.n3 + (f == 2)};
-        const int du = D == 0 ? 1 : 0, dv = D == 2 ? 1 : 2;
-        if (u >= ext[du] || v >= ext[dv]) continue;
+        const int f = st.op[o].field, kind = st.op[o].kind;
+        const int e0 = d.n1 + (f == 0), e1 = d.n2 + (f == 1), e2 = d.n3 + (f == 2);
+        if (u >= (D == 0 ? e1 : e0) || v >= (D == 2 ? e1 : e2)) continue;
+        const int ext = D == 0 ? e0 : (D == 1 ? e1 : e2);
         double* A = f == 0 ? a.aV1 : (f == 1 ? a.aV2 : a.aV3);
-        const int stride[3] = {1, sy, sz};
-        const int base = u * stride[du] + v * stride[dv];
         for (int side = 1; side >= 0; --side) {
-            const int b = side == 0 ? 0 : ext[D] - 1;
-            const int in = side == 0 ? 1 : ext[D] - 2;
-            const int cb = base + b * stride[D], ci = base + in * stride[D];
+            const int b = side == 0 ? 0 : ext - 1, in = side == 0 ? 1 : ext - 2;
+            const int cb = base + b * step, ci = base + in * step;
             const double g = A[cb];
             A[cb] = 0.0;
             if (g == 0.0) continue;
-            switch (op.kind) {
-                case BC_NEG: atomicAdd(A + ci, -g); break;
-                case BC_COPY: atomicAdd(A + ci, g); break;
-                case BC_LIN2M: atomicAdd(A + ci, -g); break;  // homogeneous form: -A[in]
+            switch (kind) {
+                // (one face point per source: no other thread of the stage adds to it)
+                case BC_NEG: A[ci] -= g; break;
+                case BC_COPY: A[ci] += g; break;
+                case BC_LIN2M: A[ci] -= g; break;  // homogeneous form: -A[in]
                 case BC_ZERO:
                 case BC_LIN: break;                              // constants: no dependence
-                default: {                                       // BC_STRESS
-                    const int cellb = side == 0 ? 0 : ext[D] - 2;
-                    const int cc = base + cellb * stride[D];
-                    const int i = (D == 0) ? cellb : u;
-                    const int j = (D == 1) ? cellb : (du == 1 ? u : v);
-                    const int wstep = D == 1 ? sz : sy;
-                    double* W = D == 1 ? a.aV3 : a.aV2;
-                    double* dst[5] = {a.aV1 + cc, a.aV1 + cc + 1, W + cc, W + cc + wstep, A + ci};
-                    for (int q = 0; q < 5; ++q) {
-                        const double cf = stress_ghost<G>(p, D, side, i, j, q == 0 ? 1.0 : 0.0, q == 1 ? 1.0 : 0.0, q == 2 ? 1.0 : 0.0,
-                                                          q == 3 ? 1.0 : 0.0, q == 4 ? 1.0 : 0.0);
-                        atomicAdd(dst[q], g * cf);
+                default: {  // BC_STRESS on the x2 / x3 faces (div_ghost, D = 1, 2): linear in V1 at the cell's two x1
+                            // faces, the other tangential component and the normal one inside
+                    if (D == 0) break;
+                    const int cell = side == 0 ? 0 : ext - 2, cc = base + cell * step;
+                    const int i = u, j = D == 1 ? cell : v;
+                    const CellMetric<double> m = cell_metric<double, G>(p, i, j);
+                    const double sgn = side == 0 ? -1.0 : 1.0, hc1 = 0.5 * m.c1, hc2 = 0.5 * m.c2;
+                    const double s = -g / (D == 1 ? fma(sgn, m.a2, hc2) : sgn * m.a3);
+                    atomicAdd(a.aV1 + cc, s * (hc1 - p.d1));
+                    atomicAdd(a.aV1 + cc + 1, s * (hc1 + p.d1));
+                    if (D == 1) {
+                        atomicAdd(a.aV3 + cc, -s * m.a3);
+                        atomicAdd(a.aV3 + cc + sz, s * m.a3);
+                        atomicAdd(A + ci, s * (hc2 - sgn * m.a2));
+                    } else {
+                        atomicAdd(a.aV2 + cc, s * (hc2 - m.a2));
+                        atomicAdd(a.aV2 + cc + sy, s * (hc2 + m.a2));
+                        atomicAdd(A + ci, -s * sgn * m.a3);
                     }
                     break;
                 }
@@ -443,8 +435,9 @@ __global__ void __launch_bounds__(256) k_pt_dtr(KP<double> p) {
 }
 
 // λ_V of the transposed PT: λ_V += avg(DT_R) (Eᵀ μ + Dᵀ λ_P - b_V) at interior nodes
-__global__ void __launch_bounds__(256) k_adj_velocity_update(KP<double> p, Adj a, double* lV1, double* lV2, double* lV3,
+__global__ void __launch_bounds__(256) k_adj_velocity_update(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, double* lV1, double* lV2, double* lV3,
                                                              const double* bV1, const double* bV2, const double* bV3) {
+    pdl_enter_small();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z + 1;
     const Dims& d = p.d;
     if (i > d.n1 - 1 || j > d.n2 - 1 || k > d.n3 - 1) return;

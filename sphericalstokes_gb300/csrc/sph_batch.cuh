@@ -2,10 +2,9 @@
 //
 // A batch of mixed-precision solves advances in lockstep: every solve whose
 // correction problem is being iterated runs the same number of FP32 sweeps per
-// round.  One sweep of all of them is one launch of k_sweep_batch per
-// geometry over a work list of (solve, tile x, tile y, x3 chunk) items — the
-// blocks each solve's own k_sweep launch would have; the sweeps handle the
-// boundary velocities themselves (SweepOut::gmask, smask), and a round of sweeps
+// round.  One sweep of all of them is one launch of k_sweep_batch over a work
+// list of (solve, tile x, tile y, x3 chunk) items; the sweeps handle the boundary
+// velocities themselves (SweepOut::gmask, smask), and a round of sweeps
 // is replayed from one CUDA graph.  The kernels run the single-grid bodies
 // (sweep_body, velocity_norm_body), so each solve computes exactly what it
 // computes alone.
@@ -25,13 +24,15 @@ struct BatchSweep {
     SweepOut<float> o[2];          // outputs of a sweep reading arrangement a (the other buffer set)
     const CUtensorMap* maps[2];    // TMA maps of the arrangement a sweep reads
     int* err;                      // the solve's bounded-wait error word
-    int kchunk;                    // x3 planes per block
+    int geom;
 };
 
-// one correction sweep of every active solve of geometry G (items: x = solve, y, z, w = tile x, y, chunk)
-template <int G>
+// one correction sweep of every active solve (items: x = solve, y, z, w = tile x, y, chunk; kchunk: planes per
+// block of each solve).  All geometries in one launch: a block runs the body of its own, and the
+// blocks of a small batch fill the SMs together (12 grids of 31 .. 47 cells a side, 600 sweeps with the
+// FP64 steps and copies: 50.8 ms with a launch per geometry and each solve's own chunk, 39.2 ms).
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __restrict__ b, const int4* __restrict__ items,
-                                                             const int* __restrict__ active, int a) {
+                                                          const int* __restrict__ active, const int* __restrict__ kchunk, int a) {
     pdl_wait();  // as k_sweep: no early release of the next grid
     const int4 it = items[blockIdx.x];
     if (!active[it.x]) return;  // whole block: no barrier is reached
@@ -45,17 +46,22 @@ __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __re
     copy(&p, &s.p[a], sizeof(p));
     copy(&o, &s.o[a], sizeof(o));
     __syncthreads();
-    sweep_body<G, 1>(p, o, s.kchunk, s.maps[a], s.err, it.y, it.z, it.w);
+    const int kc = kchunk[it.x];
+    if (s.geom == SPH) sweep_body<SPH, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
+    else if (s.geom == CYL) sweep_body<CYL, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
+    else sweep_body<CART, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
 }
 
-// inner stopping test of every active solve of geometry G: max |dV + rV| of arrangement 0 into
-// red[solve]; items: x = solve, y, z, w = velocity-node block; 32 x 8 threads
-template <int G>
+// inner stopping test of every active solve: max |dV + rV| of arrangement 0 into red[solve];
+// items: x = solve, y, z, w = velocity-node block; 32 x 8 threads
 __global__ void __launch_bounds__(256) k_velocity_norm_batch(const BatchSweep* __restrict__ b, const int4* __restrict__ items,
                                                              const int* __restrict__ active, unsigned long long* __restrict__ red) {
     const int4 it = items[blockIdx.x];
     if (!active[it.x]) return;
-    velocity_norm_body<float, G>(b[it.x].p[0], it.y, it.z, it.w, red + it.x);
+    const BatchSweep& s = b[it.x];
+    if (s.geom == SPH) velocity_norm_body<float, SPH>(s.p[0], it.y, it.z, it.w, red + it.x);
+    else if (s.geom == CYL) velocity_norm_body<float, CYL>(s.p[0], it.y, it.z, it.w, red + it.x);
+    else velocity_norm_body<float, CART>(s.p[0], it.y, it.z, it.w, red + it.x);
 }
 
 }  // namespace sph

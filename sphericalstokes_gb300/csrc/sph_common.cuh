@@ -83,6 +83,14 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// The same where the next grid is large and bound by its fullest SM: released early only from a grid of a
+// few blocks, as blocks placed beside running ones are spread unevenly over the SMs (spherical 63^3, FP64: 194 us
+// an iteration with early release throughout, 125 with this).
+__device__ __forceinline__ void pdl_enter_small() {
+    pdl_wait();
+    if (gridDim.x * gridDim.y * gridDim.z <= 64u) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __host__ __device__ inline int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 // pressure of a boundary cell under the far-field normal-stress BC: the total

@@ -26,15 +26,17 @@ namespace sph {
 
 constexpr int MC_NT = 128;  // threads per block
 
-// planes per thread: enough to pay for the column's coefficients, few enough for an even share of blocks
-// per SM (the FP64 units are the only bound, so the fullest SM ends last)
-inline int march_chunk(long long columns, int planes, int sms, double setup) {
+// planes per thread: enough to pay for the column's coefficients (`setup`, in planes), few enough for an even
+// share of blocks per SM (the FP64 units are the only bound, so the fullest SM ends last) and for `need`
+// blocks per SM, below which the loads of a plane are not hidden behind its FP64 instructions
+inline int march_chunk(long long columns, int planes, int sms, double setup, double need) {
     const long long cols = (columns + MC_NT - 1) / MC_NT;
     int best = 1;
     double best_t = 1e300;
     for (int k = 1; k <= 16 && k <= planes; ++k) {
         const long long blocks = cols * ((planes + k - 1) / k);
-        const double t = (double)((blocks + sms - 1) / sms) * (k + setup);
+        const double n = (double)((blocks + sms - 1) / sms);
+        const double t = (n > need ? n : need) * (k + setup);
         if (t < best_t) { best_t = t; best = k; }
     }
     return best;
@@ -47,6 +49,7 @@ template <typename T, int G, int WHAT, bool RHS>
 __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p, int chunk) {
     constexpr bool PT = WHAT == WHAT_STRESS || WHAT == WHAT_STRESS_LAW;
     constexpr bool ETA = WHAT != WHAT_STRAIN;
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -152,6 +155,7 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
 
 template <typename T, int G, int MODE>
 __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int w = d.n1 - 1;
@@ -225,6 +229,7 @@ __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p
 // interior cell, η_t = 2 / (1/η_ini + 1/η_PL) = 2 η_ini / (1 + x^((n-1)/(2n))); RELAXED: η_out = η^(1-relax) η_t^relax
 template <bool RELAXED>
 __global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<double> p, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
@@ -266,6 +271,7 @@ __global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<doubl
 // (CylindricalStokes_diapir.jl:185-192).  phase == 1 cells are linear.
 template <bool RELAX>
 __global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, int chunk) {
+    pdl_enter_small();
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;

@@ -39,6 +39,7 @@ __device__ __forceinline__ int order_bits(float x) {
 __device__ __forceinline__ float from_order(int b, float) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); }
 template <typename T>
 __global__ void k_maxloc(KP<T> p, int faces_only) {
+    pdl_enter_small();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     const Dims& d = p.d;
     if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;

@@ -522,21 +522,21 @@ int sync64(Ctx& c) {
 template <typename T, int G, int WHAT, bool RHS = false>
 void launch_cells(Ctx& c, const KP<T>& p) {
     const long long cols = (long long)c.d.n1 * c.d.n2;
-    const int k = march_chunk(cols, c.d.n3, c.sms, 0.4);
-    k_cells<T, G, WHAT, RHS><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+    const int k = march_chunk(cols, c.d.n3, c.sms, 0.4, 2.0);
+    launch_pdl(c.use_pdl, k_cells<T, G, WHAT, RHS>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, k);
 }
 template <typename T, int G, int MODE>
 void launch_nodes(Ctx& c, const KP<T>& p) {
     const long long cols = (long long)(c.d.n1 - 1) * (c.d.n2 - 1);
-    const int k = march_chunk(cols, c.d.n3 - 1, c.sms, 0.5);
-    k_nodes<T, G, MODE><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 - 1 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+    const int k = march_chunk(cols, c.d.n3 - 1, c.sms, 0.8, 3.0);
+    launch_pdl(c.use_pdl, k_nodes<T, G, MODE>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 - 1 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, k);
 }
 template <typename T, bool RELAXED>
 void launch_edot(Ctx& c, const KP<T>& p) {
     if constexpr (sizeof(T) == 8) {
         const long long cols = (long long)c.d.n1 * c.d.n2;
-        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1);
-        k_edot<RELAXED><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, k);
+        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1, 3.0);
+        launch_pdl(c.use_pdl, k_edot<RELAXED>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, k);
     } else {
         k_edot_law<T, RELAXED><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
     }
@@ -545,8 +545,8 @@ template <typename T, bool RELAX>
 void launch_tau_law(Ctx& c, const KP<T>& p, int faces_only) {
     if constexpr (sizeof(T) == 8) {
         const long long cols = (long long)c.d.n1 * c.d.n2;
-        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1);
-        k_rheo<RELAX><<<dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), MC_NT, 0, c.stream>>>(p, faces_only, k);
+        const int k = march_chunk(cols, c.d.n3, c.sms, 0.1, 3.0);
+        launch_pdl(c.use_pdl, k_rheo<RELAX>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, faces_only, k);
     } else {
         k_rheo_tau<T, RELAX><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
     }
@@ -566,7 +566,7 @@ void launch_maxloc(Ctx& c, KP<T>& p) {
         T* dst = last ? p.etaSM : (((passes - 1 - i) & 1) ? p.eta_out : p.etaSM);
         q.eta = src;
         q.etaSM = dst;
-        k_maxloc<T><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(q, G == CART);
+        launch_pdl(c.use_pdl, k_maxloc<T>, grid_cells(c.d), blk2d(), 0, c.stream, q, (int)(G == CART));
         src = dst;
     }
 }
@@ -624,21 +624,28 @@ std::map<std::tuple<int, int, int, int>, int> g_tuned_chunk;
 // 7.2 / 8.4 / 10.5 / 13.0 / 22.9 / 42.9, 63^3 17.2 / 17.8 / 16.2 / 16.2 / 28.0 / 52.7,
 // 131 x 117 x 101 80 / 65 / 59 / 58 / 59 / 61, 255^3 - / - / - / - / 345 / 348: the rule's
 // picks (1, 3, 4, 16) are within 2 % of the best.  sph_autotune measures instead.
-int fused_chunk(const Ctx& c) {
-    if (c.fused_chunk > 0) return c.fused_chunk;
-    const dim3 tiles = sweep_grid(c.d, c.d.n3);
-    const double xy = (double)tiles.x * tiles.y;
-    const double sms = c.fused_slots > 0 ? 0.5 * c.fused_slots : 152.0;
-    int best = 1;
+// tiles: (tiles in x1 and x2, planes) of each grid of the launch
+int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
+    int best = 1, planes = 0;
+    for (const auto& t : tiles) planes = std::max(planes, t.second);
     double best_t = 1e300;
     for (int k : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
-        const double blocks = xy * ((c.d.n3 + k - 1) / k);
-        const int n = (int)std::ceil(blocks / sms);
+        long long blocks = 0;
+        for (const auto& t : tiles) blocks += t.first * ((t.second + k - 1) / k);
+        const int n = (int)((blocks + sms - 1) / sms);
         const double t = (k + 1.4) * (0.5 * n + (n & 1 ? 0.125 : 0.0) + 0.7);
         if (t < best_t) { best_t = t; best = k; }
-        if (k >= c.d.n3) break;
+        if (k >= planes) break;
     }
     return best;
+}
+long long sweep_tiles(const Dims& d) {
+    const dim3 t = sweep_grid(d, d.n3);
+    return (long long)t.x * t.y;
+}
+int fused_chunk(const Ctx& c) {
+    if (c.fused_chunk > 0) return c.fused_chunk;
+    return chunk_rule({{sweep_tiles(c.d), c.d.n3}}, c.sms);
 }
 
 // ---------------------------------------------------------------------------
@@ -717,12 +724,12 @@ void set_sweep_attrs() {
     cudaFuncSetAttribute(k_fused<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
     cudaFuncSetAttribute(k_sweep<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
     cudaFuncSetAttribute(k_sweep<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
-    cudaFuncSetAttribute(k_sweep_batch<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
 }
 int set_fused_attrs() {
     set_sweep_attrs<SPH>();
     set_sweep_attrs<CYL>();
     set_sweep_attrs<CART>();
+    cudaFuncSetAttribute(k_sweep_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem_bytes());
     CK(cudaGetLastError());
     return SPH_OK;
 }
@@ -1406,7 +1413,7 @@ int batch_entry(Ctx& c, BatchSweep& e) {
         swap_state(t);
     }
     e.err = c.d_err;
-    e.kchunk = fused_chunk(c);
+    e.geom = c.prm.geometry;
     return SPH_OK;
 }
 
@@ -1486,6 +1493,7 @@ struct BatchDev {
     int* active = nullptr;
     unsigned long long* red = nullptr;
     int4* items = nullptr;
+    int* kchunk = nullptr;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1496,6 +1504,7 @@ struct BatchDev {
         if (active) cudaFree(active);
         if (red) cudaFree(red);
         if (items) cudaFree(items);
+        if (kchunk) cudaFree(kchunk);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (stream) cudaStreamDestroy(stream);
@@ -1531,38 +1540,37 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
     CK(cudaEventRecord(dev.e0, dev.stream));
     for (BatchSolve& b : bs) { int rc = sync64(*b.c); if (rc) return rc; }
 
-    // work lists: blocks of the member solves' fused sweeps and inner tests, per geometry
+    // work lists: blocks of the member solves' fused sweeps and inner tests.  The chunk of planes per
+    // block comes from all members' blocks together, unless a solve has its own (sph_autotune).
     std::vector<BatchSweep> host((size_t)n);
     std::vector<int4> items;
-    size_t fz_off[3], fz_n[3], nm_off[3], nm_n[3];
+    std::vector<int> kchunk((size_t)n, 1);
+    size_t fz_n = 0, nm_off = 0, nm_n = 0;
     size_t items_cap = 0, members = 0;
     auto build_lists = [&]() -> int {
         items.clear();
-        members = 0;
         std::vector<int> mem;
-        for (int32_t i = 0; i < n; ++i)
-            if (bs[i].st != BatchSolve::DONE) mem.push_back(i);
-        members = mem.size();
-        for (int g = 0; g < 3; ++g) {
-            fz_off[g] = items.size();
-            for (int i : mem) {
-                Ctx& c = *bs[i].c;
-                if (c.prm.geometry != g) continue;
-                const int kc = fused_chunk(c);
-                const dim3 gr = sweep_grid(c.d, kc);
-                for (unsigned z = 0; z < gr.z; ++z) for (unsigned y = 0; y < gr.y; ++y) for (unsigned x = 0; x < gr.x; ++x) items.push_back(make_int4(i, (int)x, (int)y, (int)z));
-            }
-            fz_n[g] = items.size() - fz_off[g];
-            nm_off[g] = items.size();
-            for (int i : mem) {
-                Ctx& c = *bs[i].c;
-                if (c.prm.geometry != g) continue;
-                const dim3 gv = grid_vel(c.d);
-                for (unsigned z = 0; z < gv.z; ++z) for (unsigned y = 0; y < gv.y; ++y) for (unsigned x = 0; x < gv.x; ++x)
-                    items.push_back(make_int4(i, (int)x, (int)y, (int)z));
-            }
-            nm_n[g] = items.size() - nm_off[g];
+        std::vector<std::pair<long long, int>> tiles;
+        for (int32_t i = 0; i < n; ++i) {
+            if (bs[i].st == BatchSolve::DONE) continue;
+            mem.push_back(i);
+            tiles.push_back({sweep_tiles(bs[i].c->d), bs[i].c->d.n3});
         }
+        members = mem.size();
+        const int common = chunk_rule(tiles, bs[0].c->sms);
+        for (int i : mem) {
+            Ctx& c = *bs[i].c;
+            kchunk[i] = c.fused_chunk > 0 ? c.fused_chunk : common;
+            const dim3 gr = sweep_grid(c.d, kchunk[i]);
+            for (unsigned z = 0; z < gr.z; ++z) for (unsigned y = 0; y < gr.y; ++y) for (unsigned x = 0; x < gr.x; ++x) items.push_back(make_int4(i, (int)x, (int)y, (int)z));
+        }
+        fz_n = nm_off = items.size();
+        for (int i : mem) {
+            const dim3 gv = grid_vel(bs[i].c->d);
+            for (unsigned z = 0; z < gv.z; ++z) for (unsigned y = 0; y < gv.y; ++y) for (unsigned x = 0; x < gv.x; ++x)
+                items.push_back(make_int4(i, (int)x, (int)y, (int)z));
+        }
+        nm_n = items.size() - nm_off;
         if (items.size() > items_cap) {
             CK(cudaStreamSynchronize(dev.stream));
             if (dev.items) cudaFree(dev.items);
@@ -1574,11 +1582,12 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             items_cap = items.size();
         }
         CK(cudaMemcpyAsync(dev.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, dev.stream));
+        CK(cudaMemcpyAsync(dev.kchunk, kchunk.data(), sizeof(int) * n, cudaMemcpyHostToDevice, dev.stream));
         CK(cudaStreamSynchronize(dev.stream));  // the host list is rebuilt in place next time
         return SPH_OK;
     };
     if (cudaMalloc((void**)&dev.entries, sizeof(BatchSweep) * n) != cudaSuccess || cudaMalloc((void**)&dev.active, sizeof(int) * n) != cudaSuccess ||
-        cudaMalloc((void**)&dev.red, sizeof(unsigned long long) * n) != cudaSuccess) {
+        cudaMalloc((void**)&dev.red, sizeof(unsigned long long) * n) != cudaSuccess || cudaMalloc((void**)&dev.kchunk, sizeof(int) * n) != cudaSuccess) {
         cudaGetLastError();
         return fail(SPH_ERR_NOMEM, "batched solve: device work lists");
     }
@@ -1596,9 +1605,8 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             // tail of the one before (the kernels wait on it before touching memory)
             const BatchSweep* E = dev.entries;
             const int* act_d = dev.active;
-            if (fz_n[SPH]) launch_pdl(pdl, k_sweep_batch<SPH>, dim3((unsigned)fz_n[SPH]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[SPH], act_d, a);
-            if (fz_n[CYL]) launch_pdl(pdl, k_sweep_batch<CYL>, dim3((unsigned)fz_n[CYL]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[CYL], act_d, a);
-            if (fz_n[CART]) launch_pdl(pdl, k_sweep_batch<CART>, dim3((unsigned)fz_n[CART]), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items + fz_off[CART], act_d, a);
+            const int* kc_d = dev.kchunk;
+            launch_pdl(pdl, k_sweep_batch, dim3((unsigned)fz_n), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items, act_d, kc_d, a);
         }
         cudaError_t e = cudaStreamEndCapture(dev.stream, &g);
         if (e != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e));
@@ -1653,9 +1661,7 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
         CK(cudaMemcpyAsync(dev.active, act.data(), sizeof(int) * n, cudaMemcpyHostToDevice, dev.stream));
         CK(cudaGraphLaunch(dev.graph, dev.stream));
         CK(cudaMemsetAsync(dev.red, 0, sizeof(unsigned long long) * n, dev.stream));
-        if (nm_n[SPH]) k_velocity_norm_batch<SPH><<<(unsigned)nm_n[SPH], blk2d(), 0, dev.stream>>>(dev.entries, dev.items + nm_off[SPH], dev.active, dev.red);
-        if (nm_n[CYL]) k_velocity_norm_batch<CYL><<<(unsigned)nm_n[CYL], blk2d(), 0, dev.stream>>>(dev.entries, dev.items + nm_off[CYL], dev.active, dev.red);
-        if (nm_n[CART]) k_velocity_norm_batch<CART><<<(unsigned)nm_n[CART], blk2d(), 0, dev.stream>>>(dev.entries, dev.items + nm_off[CART], dev.active, dev.red);
+        k_velocity_norm_batch<<<(unsigned)nm_n, blk2d(), 0, dev.stream>>>(dev.entries, dev.items + nm_off, dev.active, dev.red);
         CK(cudaGetLastError());
         std::vector<unsigned long long> red((size_t)n);
         CK(cudaMemcpyAsync(red.data(), dev.red, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, dev.stream));
@@ -2122,7 +2128,8 @@ static void adj_bc(Ctx* c, const KP<double>& p, const Adj& a) {
         int eu = st->dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
         int ev = st->dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
         dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
-        k_bc_adjoint<G><<<g, blk2d(), 0, c->stream>>>(hp, a, *st);
+        auto k = st->dim == 0 ? k_bc_adjoint<G, 0> : (st->dim == 1 ? k_bc_adjoint<G, 1> : k_bc_adjoint<G, 2>);
+        launch_pdl(c->use_pdl, k, g, blk2d(), 0, c->stream, hp, a, *st);
     }
 }
 
@@ -2139,20 +2146,22 @@ template <int G, bool MEM>
 static void adj_rows(Ctx* c, const KP<double>& p, const Adj& a) {
     const bool law = c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX;
     const long long cols = (long long)c->d.n1 * c->d.n2;
-    const int ks = march_chunk(cols, c->d.n3, c->sms, 0.6), kl = march_chunk(cols, c->d.n3, c->sms, 0.2);
-    if (law) k_adj_stress<G, MEM, true><<<adj_cells(c, ks), MC_NT, 0, c->stream>>>(p, a, ks);
-    else k_adj_stress<G, MEM, false><<<adj_cells(c, ks), MC_NT, 0, c->stream>>>(p, a, ks);
+    const int ks = march_chunk(cols, c->d.n3, c->sms, 0.6, 6.0), kl = march_chunk(cols, c->d.n3, c->sms, 0.2, 8.0);
+    const dim3 nt(MC_NT);
+    if (law) launch_pdl(c->use_pdl, k_adj_stress<G, MEM, true>, adj_cells(c, ks), nt, 0, c->stream, p, a, ks);
+    else launch_pdl(c->use_pdl, k_adj_stress<G, MEM, false>, adj_cells(c, ks), nt, 0, c->stream, p, a, ks);
     if (law) {
-        k_adj_eta<true><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
-        k_adj_law<G><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
+        launch_pdl(c->use_pdl, k_adj_eta<true>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
+        launch_pdl(c->use_pdl, k_adj_collect, grid_cells(c->d), blk2d(), 0, c->stream, p, a);
+        launch_pdl(c->use_pdl, k_adj_law<G>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
     } else if (!MEM) {
-        k_adj_eta<false><<<adj_cells(c, kl), MC_NT, 0, c->stream>>>(p, a, kl);
+        launch_pdl(c->use_pdl, k_adj_eta<false>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
     }
     const long long nodes = (long long)(c->d.n1 + 1) * (c->d.n2 + 1);
-    const int kn = march_chunk(nodes, c->d.n3 + 1, c->sms, 0.6);
+    const int kn = march_chunk(nodes, c->d.n3 + 1, c->sms, 0.6, 8.0);
     const dim3 gn((unsigned)((nodes + MC_NT - 1) / MC_NT), (c->d.n3 + 1 + kn - 1) / kn);
-    if (law) k_adj_strain<G><<<gn, MC_NT, 0, c->stream>>>(p, a, a.x12, a.x13, a.x23, kn);
-    else k_adj_strain<G><<<gn, MC_NT, 0, c->stream>>>(p, a, a.e12, a.e13, a.e23, kn);
+    const double *x12 = law ? a.x12 : a.e12, *x13 = law ? a.x13 : a.e13, *x23 = law ? a.x23 : a.e23;
+    launch_pdl(c->use_pdl, k_adj_strain<G>, gn, nt, 0, c->stream, p, a, x12, x13, x23, kn);
 }
 
 // Aᵀ λ (λ in the AJ_L* slots) into AJ_V*, AJ_P, with ∂R/∂η, ∂R/∂ρ contractions; with_bc: the
@@ -2193,8 +2202,8 @@ static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf)
         ++it;
         adj_rows<G, true>(c, p, a);  // M_τᵀ λ_V, M_Pᵀ λ_V, Eᵀ μ + Dᵀ λ_P
         adj_bc<G>(c, p, a);
-        k_adj_velocity_update<<<grid_vel(c->d), blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_LV1), adj_slot(c, AJ_LV2), adj_slot(c, AJ_LV3),
-                                                                         adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3));
+        launch_pdl(c->use_pdl, k_adj_velocity_update, grid_vel(c->d), blk2d(), 0, c->stream, p, a, adj_slot(c, AJ_LV1), adj_slot(c, AJ_LV2),
+                   adj_slot(c, AJ_LV3), adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3));
         if (it % nout) continue;
         // convergence: the transposed residual Aᵀλ - b of the current λ
         if ((rc = adj_apply<G>(c, p, true))) return rc;
