@@ -29,13 +29,19 @@
 // * 14 rows, because 7 warps of owned points and one of halo points (31 pairs) make four
 //   warps per scheduler at two blocks per SM, which leaves 128 registers to each thread:
 //   16 rows need a ninth warp, five warps on some schedulers, 96 registers and spills.
+// * Uniform paths.  Faces, masks and ghosts are bits set once per pair; a warp whose points
+//   are all inside takes the path without masks (a vote at the start of the block), ghosts on
+//   x1 travel with the pair's own store, and the divergence-free x2 ghosts and the loaded x2
+//   faces are paired arithmetic: no plane diverges except the first and last of the grid and
+//   the rows on an x1 face with such a ghost.
 // Measured on a GB300, us per sweep with its boundary velocities (before: one cell per
 // thread, 32 x 8 tiles, 30 warps per SM, x2 / x3 ghosts by two to four BC launches):
-// 255^3 349 (375; 4.9 TB/s of the algorithmic bytes, 0.74 of the copy rate),
-// 511 x 255 x 255 with a free surface 643 (732), 131 x 117 x 101 58.3 (65.0),
-// 63^3 16.2 (19.1), 47 x 31 x 39 Cartesian 7.2 (14.5).  At 255^3 351 warp instructions
-// per 32 cells (608) at 15.6 warps per SM: what remains is latency, block-barrier waits
-// (2.2 stalls per issue) and dependent arithmetic (1.6).
+// 255^3 304 (375; 5.7 TB/s of the algorithmic bytes, 0.85 of the copy rate),
+// 511 x 255 x 255 with a free surface 608 (732), 131 x 117 x 101 45.2 (65.0),
+// 63^3 12.7 (19.1), 47 x 31 x 39 Cartesian 6.3 (14.5).  At 255^3 300 warp instructions
+// per 32 cells (608).  The same copies and stores without the arithmetic take 285 us
+// (the tiles' halos and 10 + 10 streams cost 10 % of the copy rate): memory bound there.  The
+// smallest grids are one wave of blocks: the latency of a few planes and the launch.
 //
 // Thread roles (8 warps): warp w < 7, lane l: row b = 2w + l/16 + 1, points
 // a = 2(l%16) + 1, +2, i.e. cells (x0 + 2(l%16) + {0,1}, y0 + b - 1), and the
@@ -345,39 +351,51 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
     const int I = x, J = y;  // velocity nodes (I, J), (I + 1, J) of the owned points
     const int gxy = x + d.sy * y;
     // what holds for this pair's points whatever the plane, one bit each (point l: bit + l)
-    enum { IN_ = 0, E12_ = 2, E13_ = 4, E23_ = 6, N1_ = 8, N2_ = 10, N3_ = 12,  // inside the grid: cells, edges, V1..V3 nodes
-           FULL = 14,     // all of the first eight
-           SPECIAL = 15,  // a boundary cell whose P or ghosts need more than the plain update
-           XLO = 16,      // the pair's first point is the low x1 ghost
-           XH1 = 17, XH2 = 19,  // the high x1 ghost of V1 / V2, V3 follows point l
-           XFACE = 21, YFACE = 22,
-           VFULL = 23 };  // every node of the pair inside the grid, none next to an x1 or x2 face  // ghosts on x1 / on x2 faces to store
+    enum { IN_ = 0, E12_ = 2, E13_ = 4, E23_ = 6,  // inside the grid: cells, edges
+           M_ = 8,        // entries of V1 (+2: V2, +4: V3) this pair writes: nodes, and x1 ghosts within the pair
+           X_ = 14,       // V1 (+1, +2): the high x1 ghost follows the pair's second point
+           XLO = 17,      // the pair's first point is the low x1 ghost
+           XH1 = 18, XH2 = 19,  // the pair's second point is the high x1 ghost of V1 / of V2 and V3
+           SPECIAL = 20,  // a cell on an x1 face with a divergence-free ghost or the free-surface pressure
+           GY_ = 21,      // V1 (+1, +2) has an x2 ghost next to this row
+           YS = 24, YT = 25 };  // a cell on an x2 face with a divergence-free ghost / a prescribed normal stress
     unsigned fl = 0;
     {
         const bool in[2] = {in0, in1};
         const bool nrow = !halo && J >= 1 && J <= n2 - 1;
-        const bool yf = y == 0 || y == n2 - 1;
         for (int l = 0; l < 2; ++l) {
             const int xl = x + l;
-            const bool node = nrow && xl >= 1 && xl <= n1 - 1;
             fl |= (in[l] ? 1u : 0u) << (IN_ + l);
             fl |= (in[l] && xl < n1 - 1 && y < n2 - 1 ? 1u : 0u) << (E12_ + l);
             fl |= (in[l] && xl < n1 - 1 && y < n2 - 2 ? 1u : 0u) << (E13_ + l);
             fl |= (in[l] && xl < n1 - 2 && y < n2 - 1 ? 1u : 0u) << (E23_ + l);
-            fl |= (node && J <= n2 - 2 ? 1u : 0u) << (N1_ + l);
-            fl |= (node && xl <= n1 - 2 ? 1u : 0u) << (N2_ + l);
-            fl |= (node && xl <= n1 - 2 && J <= n2 - 2 ? 1u : 0u) << (N3_ + l);
-            fl |= (xl == n1 - 1 ? 1u : 0u) << (XH1 + l);
-            fl |= (xl == n1 - 2 ? 1u : 0u) << (XH2 + l);
         }
-        if ((fl & 255u) == 255u) fl |= 1u << FULL;
-        if (yin && (((p.traction || (o.smask & 12)) && yf) || ((p.fs || (o.smask & 3)) && (x <= 0 || x + 1 >= n1 - 1)))) fl |= 1u << SPECIAL;
+        for (int f = 0; f < 3; ++f) {
+            const int lastI = f == 0 ? n1 - 1 : n1 - 2, lastJ = f == 1 ? n2 - 1 : n2 - 2;
+            const bool row = nrow && J <= lastJ;
+            const bool lo = MODE == 1 && (o.gmask >> (2 * f) & 1), hi = MODE == 1 && (o.gmask >> (2 * f) & 2);
+            const bool a0 = row && (I >= 1 ? I <= lastI : I == 0 && lo);
+            const bool a1 = row && I + 1 >= 1 && (I + 1 <= lastI || (I == lastI && hi));
+            fl |= (a0 ? 1u : 0u) << (M_ + 2 * f) | (a1 ? 1u : 0u) << (M_ + 2 * f + 1);
+            fl |= (row && I + 1 == lastI && hi ? 1u : 0u) << (X_ + f);
+            fl |= (row && o.gmask && (J == 1 ? o.gmask >> (6 + 2 * f) & 1 : J == lastJ && (o.gmask >> (7 + 2 * f) & 1)) ? 1u : 0u) << (GY_ + f);
+        }
         if (I == 0) fl |= 1u << XLO;
-        if (nrow && (o.gmask & 63) && (fl & (31u << XLO))) fl |= 1u << XFACE;
-        if (nrow && (o.gmask >> 6) && (J == 1 || J >= n2 - 2)) fl |= 1u << YFACE;
-        if ((fl >> N1_ & 63u) == 63u && !(fl & (3u << XFACE))) fl |= 1u << VFULL;
+        if (I == n1 - 1) fl |= 1u << XH1;
+        if (I == n1 - 2) fl |= 1u << XH2;
+        const bool yf = y == 0 || y == n2 - 1;
+        if (yin && (p.fs || (o.smask & 3)) && (x <= 0 || x + 1 >= n1 - 1)) fl |= 1u << SPECIAL;
+        if (yin && o.smask & (y == 0 ? 4 : (y == n2 - 1 ? 8 : 0))) fl |= 1u << YS;
+        if (yin && p.traction && yf) fl |= 1u << YT;
     }
+    // whole warps without masks: every cell and edge inside, every node written and no ghost
+    const bool wcells = __all_sync(0xffffffffu, (fl & 255u) == 255u);
+    constexpr unsigned kStage1Bits = 1u << SPECIAL | 1u << YS | 1u << YT;  // (of no concern to the nodes)
+    const bool wnodes = __all_sync(0xffffffffu, ((fl & ~kStage1Bits) >> M_) == 63u);
     auto has = [&](int bit) { return (fl >> bit & 1u) != 0u; };
+    // a warp whose two rows lie past the grid (the last tile of a ragged n2) only keeps the barriers: no
+    // valid point reads its rows
+    const bool busy = halo || y0 + 2 * warp < n2;
 
     // Spherical: four momentum coefficients wait in shared memory, for registers (spilled ones go to
     // L2, as the shared memory of two blocks leaves almost no L1)
@@ -408,8 +426,8 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
     auto rare = [](bool c) { return __builtin_expect(c, 0) != 0; };
 
     // stresses of plane k from the values n brings along from plane k; leaves those of plane k + 1
-    // in m.  inner: 1 <= k <= n3 - 3 (every x3 condition holds, no x3 face)
-    auto stage1 = [&](auto par, int k, bool own, bool inner, const float* A, const float* B, const Carry& n, Carry& m) {
+    // in m
+    auto stage1 = [&](auto par, int k, bool own, const float* A, const float* B, const Carry& n, Carry& m) {
         constexpr int so = decltype(par)::value;  // parity of k - k0: slots
         const float *A2 = A + SI_N, *B2 = B + SI_N, *A3 = A2 + SI_N, *B3 = B2 + SI_N;  // V2, V3 of planes k, k + 1
         auto ld2 = [&](const float* T, int db) { return make_float2(T[iin + db * SI_X + 1], T[iin + db * SI_X + 2]); };
@@ -418,7 +436,19 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
         {
             ov1 = ldP(A, 0); ov2 = ldP(A2, 0); ov3 = ldP(A3, 0);
             float2 a1 = ov1, b1 = ldS(A, 0, a1), a2 = ov2, b2 = ldP(A2, 1), a3 = ov3, b3 = ldP(B3, 0);
-            if (rare(MODE == 1 && o.smask && (has(SPECIAL) || k == 0 || k == n3 - 1))) {
+            const bool zface = k == 0 || k == n3 - 1;
+            if (MODE == 1 && has(YS) && !zface && !has(SPECIAL)) {  // div_ghost<D = 1> of both points
+                const bool low = y == 0;
+                const float sg = low ? -1.f : 1.f;
+                const float2 hh = dup(0.5f), c1 = mul2(C.e1, dup(G == SPH ? 4.f : 2.f)), c2 = add2(C.e2, C.e2);
+                const float2 avx = mul2(hh, add2(a1, b1)), vin = low ? b2 : a2;
+                const float2 t = fma2(C.a3, sub2(b3, a3), fma2(c1, avx, mul2(vin, fma2(hh, c2, mul2(dup(-sg), C.a2)))));
+                const float2 num = mul2(fma2(o.d1, sub2(b1, a1), t), dup(-1.f)), den = fma2(dup(sg), C.a2, mul2(hh, c2));
+                const float2 rc = make_float2(rcp_approx(den.x), rcp_approx(den.y)), q = mul2(num, rc);
+                const float2 g = fma2(fma2(mul2(den, dup(-1.f)), q, num), rc, q);
+                if (low) a2 = g;
+                else b2 = g;
+            } else if (rare(MODE == 1 && o.smask && (has(SPECIAL) || zface))) {
 #pragma unroll 1
                 for (int l = 0; l < 2; ++l) {
                     if (!has(IN_ + l)) continue;
@@ -454,7 +484,9 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
             v11 = mul2(fma2(gs2, D11, old(S.tau[so], 0)), f);
             v22 = mul2(fma2(gs2, D22, old(S.tau[so], 1)), f);
             v33 = mul2(fma2(gs2, D33, old(S.tau[so], 2)), f);
-            if (rare(has(SPECIAL) || (p.traction && (k == 0 || k == n3 - 1)))) {
+            if (has(YT) && !zface) {
+                vP = sub2(v22, dup(p.sig2));
+            } else if (rare(has(SPECIAL) || (p.traction && zface))) {
 #pragma unroll 1
                 for (int l = 0; l < 2; ++l) {
                     if (!has(IN_ + l)) continue;
@@ -467,7 +499,6 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
             }
             vdt = div2(o.vp, fma2(gs, f, kb));
         }
-        asm volatile("" ::: "memory");  // loads stay in their block: hoisted ones cost registers that spill
         auto sums = [&](const float* A, float2& P, float2& X0, float2& X, float2& Y) {
             P = ldP(A, 0);
             const float2 s = ldS(A, 0, P), q = ldP(A, 1), t = ldS(A, 1, q);
@@ -489,7 +520,6 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
             if (G != CART) D = fma2(C.e12_h, add2(b2Q, b2T), D);
             v12 = edge(old(S.tau[so], 3), add2(sX0, m.sX), add2(eX0, m.eX), D);
         }
-        asm volatile("" ::: "memory");
         {
             float2 D = fma2(C.e13_d3, sub2(b1T, ld2(A, 1)), mul2(o.d1q, sub2(b3T, b3Q)));
             if (G == SPH) D = fma2(C.e12_h, add2(b3Q, b3T), D);
@@ -504,26 +534,19 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
 
         const bool k12 = k < n3 - 2, k1x = k < n3 - 1;
         const unsigned gb = 4u * (unsigned)(gxy + d.sz * k);  // byte offset (owned points only: >= 0)
-        if (own) {
-            if (!rare(!(has(FULL) && inner))) {
-                st_pair(o.P, gb, vP); st_pair(o.t11, gb, v11); st_pair(o.t22, gb, v22); st_pair(o.t33, gb, v33);
-                st_pair(o.t12, gb, v12); st_pair(o.t13, gb, v13); st_pair(o.t23, gb, v23);
-            } else {
-                const bool i0 = has(IN_), i1 = has(IN_ + 1);
-                st_pair(o.P, gb, vP, i0, i1); st_pair(o.t11, gb, v11, i0, i1);
-                st_pair(o.t22, gb, v22, i0, i1); st_pair(o.t33, gb, v33, i0, i1);
-                if (k12) st_pair(o.t12, gb, v12, has(E12_), has(E12_ + 1));
-                if (k1x) { st_pair(o.t13, gb, v13, has(E13_), has(E13_ + 1)); st_pair(o.t23, gb, v23, has(E23_), has(E23_ + 1)); }
-            }
-        }
         float2 o33 = sub2(v33, vP);
         o11 = sub2(v11, vP); o22 = sub2(v22, vP);
-        if (rare(!has(FULL) || !inner)) {  // points outside the grid: zero
+        if (!(wcells && k12)) {  // zero outside the grid (a pair's first point is inside where its second is)
             const bool i0 = has(IN_), i1 = has(IN_ + 1);
+            vP = keep2(vP, i0, i1); v11 = keep2(v11, i0, i1); v22 = keep2(v22, i0, i1); v33 = keep2(v33, i0, i1);
             o11 = keep2(o11, i0, i1); o22 = keep2(o22, i0, i1); o33 = keep2(o33, i0, i1); vdt = keep2(vdt, i0, i1);
             v12 = keep2(v12, has(E12_) && k12, has(E12_ + 1) && k12);
             v13 = keep2(v13, has(E13_) && k1x, has(E13_ + 1) && k1x);
             v23 = keep2(v23, has(E23_) && k1x, has(E23_ + 1) && k1x);
+        }
+        if (own && has(IN_)) {  // (zeros where the second point, or an edge of the first, is padding)
+            st_pair(o.P, gb, vP); st_pair(o.t11, gb, v11); st_pair(o.t22, gb, v22); st_pair(o.t33, gb, v33);
+            st_pair(o.t12, gb, v12); st_pair(o.t13, gb, v13); st_pair(o.t23, gb, v23);
         }
         m.s33 = o33; m.dt = vdt; m.t12 = v12.x; m.u23 = v23.x;
         auto put = [&](float* W, float2 v) { *reinterpret_cast<float2*>(W + ist) = v; };
@@ -534,7 +557,7 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
 
     // velocities of plane K at the nodes (I, J), (I + 1, J) from the stresses of planes K-1 and K
     // (n, m: what stage 1 of plane K took and left)
-    auto velocity = [&](auto par, int K, bool own, bool inner, const Carry& n, Carry& m) {
+    auto velocity = [&](auto par, int K, bool own, const Carry& n, Carry& m) {
         constexpr int so = decltype(par)::value;
         const float *E12p = S.e[1 - so][0] + ist, *E13p = S.e[1 - so][1] + ist, *E23p = S.e[1 - so][2] + ist;
         const float *E13 = S.e[so][1] + ist - SR_X, *E23 = S.e[so][2] + ist - SR_X;
@@ -546,36 +569,10 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
             const float2 b12 = *reinterpret_cast<const float2*>(E12p - SR_X);               // τ12 (I, J-1, K-1)
             const float2 t12a = make_float2(E12p[-1], n.t12), t12b = make_float2(E12p[-SR_X - 1], b12.x);
             const float *Q11 = S.q[0] + ist, *Q22 = S.q[1] + ist, *Q33 = S.q[2] + ist, *QDT = S.q[3] + ist;
-            asm volatile("" ::: "memory");
-            // nodes next to the grid's faces: masked stores, and with MODE 1 the ghosts of the x1, x2
-            // and x3 faces (a ghost's own ghosts on edges and corners among them)
-            const bool plain = has(VFULL) && inner && K > 1;
-            auto put = [&](float* A, int f, float2 v, bool m0, bool m1, int high, int lastJ, int lastK) {
-                auto row = [&](unsigned at, float2 w) {
-                    st_pair(A, at, w, m0, m1);
-                    if (MODE == 1 && has(XFACE) && (m0 || m1)) {
-                        if (has(XLO) && (o.gmask >> (2 * f) & 1)) st_at(A, at, o.gf[f] * w.y);
-                        if ((fl >> high & 3u) && (o.gmask >> (2 * f) & 2)) st_at(A, at + (has(high) ? 4u : 8u), o.gf[f] * (has(high) ? w.x : w.y));
-                    }
-                };
-                if (!rare(!plain)) { st_pair(A, gb, v); return; }
-                // bit 0: the x2 ghost, bit 1: the x3 ghost next to these nodes
-                int q = 0;
-                if (MODE == 1 && (J == 1 || J == lastJ)) q |= o.gmask >> (6 + 2 * f + (J == 1 ? 0 : 1)) & 1;
-                if (MODE == 1 && (K == 1 || K == lastK)) q |= (o.gmask >> (12 + 2 * f + (K == 1 ? 0 : 1)) & 1) << 1;
-                const unsigned oy = (unsigned)(J == 1 ? -4 * d.sy : 4 * d.sy), oz = (unsigned)(K == 1 ? -4 * d.sz : 4 * d.sz);
-#pragma unroll 1
-                for (int i = 0; i < (MODE == 1 ? 4 : 1); ++i) {
-                    if ((i & q) != i) continue;
-                    float2 w = v;
-                    if (i & 1) w = mul2(w, dup(o.gf[3 + f]));
-                    if (i & 2) w = mul2(w, dup(o.gf[6 + f]));
-                    row(gb + (i & 1 ? oy : 0u) + (i & 2 ? oz : 0u), w);
-                }
-            };
             const float* R = MODE == 1 ? S.rv[so] + (b - 1) * SWX + (a - 1) : S.rp[so] + iold;
             auto rv = [&](int f) { return *reinterpret_cast<const float2*>(R + f * SV_N); };
             const float2 gh = dup(-0.5f * p.g), rc = MODE == 0 ? rv(0) : dup(0.f);
+            float2 u1, u2, u3;
             {  // V1 (I-1/2, J, K), cell m = (I-1, J, K)
                 const float2 m11 = make_float2(Q11[-1], o11.x);
                 float2 r1 = fma2(coef(0, C.m1_d3), sub2(c13, p13), mul2(o.d1, sub2(o11, m11)));
@@ -595,10 +592,8 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
                 }
                 if (MODE == 1) r1 = add2(r1, rv(0));
                 else if (G != CART) r1 = fma2(gh, add2(make_float2(R[-1], rc.x), rc), r1);
-                const float2 v = fma2(r1, add2(make_float2(QDT[-1], odt.x), odt), ov1);
-                if (K <= n3 - 2) put(o.V1, 0, v, has(N1_), has(N1_ + 1), XH1, n2 - 2, n3 - 2);
+                u1 = fma2(r1, add2(make_float2(QDT[-1], odt.x), odt), ov1);
             }
-            asm volatile("" ::: "memory");
             {  // V2 (I, J-1/2, K), cell m = (I, J-1, K)
                 const float2 m22 = *reinterpret_cast<const float2*>(Q22 - SR_X);
                 float2 r2 = fma2(coef(2, C.m2_d3), sub2(c23, p23), fma2(C.a2, sub2(o22, m22), mul2(o.d1, sub2(b12, t12b))));
@@ -608,10 +603,8 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
                     r2 = fma2(coef(3, C.m2_n), sub2(add2(m22, o22), add2(m33, o33)), r2);
                 }
                 if (MODE == 1) r2 = add2(r2, rv(1));
-                const float2 v = fma2(r2, add2(*reinterpret_cast<const float2*>(QDT - SR_X), odt), ov2);
-                if (K <= n3 - 2) put(o.V2, 1, v, has(N2_), has(N2_ + 1), XH2, n2 - 1, n3 - 2);
+                u2 = fma2(r2, add2(*reinterpret_cast<const float2*>(QDT - SR_X), odt), ov2);
             }
-            asm volatile("" ::: "memory");
             {  // V3 (I, J, K-1/2), cell m = (I, J, K-1)
                 const float2 t13a = *reinterpret_cast<const float2*>(E13p - SR_X), t23a = make_float2(E23p[-1], n.u23);
                 float2 r3 = fma2(C.a3, sub2(o33, n.s33), fma2(C.a2, sub2(t23a, p23), mul2(o.d1, sub2(t13a, p13))));
@@ -623,12 +616,44 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
                 if (MODE == 1) {
                     r3 = add2(r3, rv(2));
                 } else if (G == CART) {  // ρ of plane K-1: its slot is being refilled
-                    const float2 rm = make_float2(has(N3_) ? p.rho[gxy + d.sz * (K - 1)] : 0.f, has(N3_ + 1) ? p.rho[gxy + d.sz * (K - 1) + 1] : 0.f);
+                    const float2 rm = make_float2(has(M_ + 4) ? p.rho[gxy + d.sz * (K - 1)] : 0.f, has(M_ + 5) ? p.rho[gxy + d.sz * (K - 1) + 1] : 0.f);
                     r3 = fma2(gh, add2(rm, rc), r3);
                 }
-                const float2 v = fma2(r3, add2(n.dt, odt), ov3);
-                put(o.V3, 2, v, has(N3_), has(N3_ + 1), XH2, n2 - 2, n3 - 1);
+                u3 = fma2(r3, add2(n.dt, odt), ov3);
             }
+            if (wnodes && K > 1 && K <= n3 - 3) {
+                st_pair(o.V1, gb, u1); st_pair(o.V2, gb, u2); st_pair(o.V3, gb, u3);
+                return;
+            }
+            // Nodes next to the grid's faces, with MODE 1 also their ghosts: on x1 within the pair (then still one
+            // store) or after it, on x2 and x3 the same once more at the face's offset, edges and corners
+            // included.  The lanes of a warp stay together here: only the extra stores are masked.
+            auto put = [&](float* A, int f, float2 v, int high, int lastK) {
+                if (MODE == 1) {
+                    if (has(XLO)) v.x = o.gf[f] * v.y;
+                    if (has(high)) v.y = o.gf[f] * v.x;
+                }
+                auto row = [&](unsigned at, float2 w) {
+                    st_pair(A, at, w, has(M_ + 2 * f), has(M_ + 2 * f + 1));
+                    if (MODE == 1 && has(X_ + f)) st_at(A, at + 8u, o.gf[f] * w.y);
+                };
+                row(gb, v);
+                if (MODE == 0) return;
+                const bool gy = has(GY_ + f);
+                const bool gz = K == 1 ? (o.gmask >> (12 + 2 * f) & 1) : K == lastK && (o.gmask >> (13 + 2 * f) & 1);
+                const unsigned oy = (unsigned)(J == 1 ? -4 * d.sy : 4 * d.sy), oz = (unsigned)(K == 1 ? -4 * d.sz : 4 * d.sz);
+                const float2 vy = mul2(v, dup(o.gf[3 + f]));
+                if (gy) row(gb + oy, vy);
+                if (gz) {
+                    row(gb + oz, mul2(v, dup(o.gf[6 + f])));
+                    if (gy) row(gb + oy + oz, mul2(vy, dup(o.gf[6 + f])));
+                }
+            };
+            if (K <= n3 - 2) {
+                put(o.V1, 0, u1, XH1, n3 - 2);
+                put(o.V2, 1, u2, XH2, n3 - 2);
+            }
+            put(o.V3, 2, u3, XH2, n3 - 1);
         }
     };
 
@@ -649,14 +674,14 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
     const float *A = S.in[0], *B = S.in[1];  // input planes K, K + 1
     auto step = [&](auto par, int K, const Carry& n, Carry& m) {
         constexpr int so = decltype(par)::value;
-        const bool own = K >= kA, inner = K >= 1 && K <= n3 - 3;
+        const bool own = K >= kA;
         if (halo) wait(&S.bar_s[so], so);
         __syncthreads();  // copies have landed; the velocities of plane K-1 are done with the shared stresses
-        stage1(par, K, own && !halo, inner, A, B, n, m);
+        if (busy) stage1(par, K, own && !halo, A, B, n, m);
         if (halo && own) wait(&S.bar_v[so], 2 + so);
         __syncthreads();
         if (!halo) {
-            velocity(par, K, own, inner, n, m);
+            if (busy) velocity(par, K, own, n, m);
         } else if (issuer && ok) {
             if (K + 2 < kB) issue_stage(K + 2);
             if (own && K + 1 < kB) issue_rhs(K + 1);

@@ -616,14 +616,14 @@ std::map<std::tuple<int, int, int, int>, int> g_tuned_chunk;
 // x3 chunk length of the fused sweep.  Each block marches over one chunk of
 // planes and pays for more planes than it owns (the halo plane below the chunk and
 // the pipeline fill), while the hardware scheduler balances the SMs only to within
-// one block at the end of the launch.  The time model (k + 1.4) * (n / 2 + 0.7), n =
-// blocks on the fullest SM (two are resident), picks the chunk among 1..24 planes; an
-// odd n counts an eighth more, as the last block alone on its SM does not run at twice
-// the speed.
+// one block at the end of the launch.  The time model (k + 2) * max(2.15, 1.1 n + 0.5), n =
+// blocks on the fullest SM (two are resident, and two together are hardly slower than one),
+// picks the chunk among 1..24 planes.
 // Measured on a GB300 (us per sweep, chunks of 1 / 2 / 3 / 4 / 8 / 16 planes): 47 x 31 x 39
-// 7.2 / 8.4 / 10.5 / 13.0 / 22.9 / 42.9, 63^3 17.2 / 17.8 / 16.2 / 16.2 / 28.0 / 52.7,
-// 131 x 117 x 101 80 / 65 / 59 / 58 / 59 / 61, 255^3 - / - / - / - / 345 / 348: the rule's
-// picks (1, 3, 4, 16) are within 2 % of the best.  sph_autotune measures instead.
+// 6.4 / 7.0 / 8.5 / 10.0 / 17 / 31, 63^3 15.8 / 13.5 / 12.7 / 12.3 / 18 / 32,
+// 131 x 117 x 101 77 / 60 / 53 / 50 / 45.2 / 44.3, 255^3 (8 / 16 / 24) 322 / 305 / 304,
+// 511 x 255 x 255 630 / 608 / 596: the rule's picks (1, 3, 8, 16, 16) are within 4 % of the
+// best (32 planes: 298 and 620).  sph_autotune measures instead.
 // tiles: (tiles in x1 and x2, planes) of each grid of the launch
 int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
     int best = 1, planes = 0;
@@ -633,7 +633,7 @@ int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
         long long blocks = 0;
         for (const auto& t : tiles) blocks += t.first * ((t.second + k - 1) / k);
         const int n = (int)((blocks + sms - 1) / sms);
-        const double t = (k + 1.4) * (0.5 * n + (n & 1 ? 0.125 : 0.0) + 0.7);
+        const double t = (k + 2.0) * std::max(2.15, 1.1 * n + 0.5);
         if (t < best_t) { best_t = t; best = k; }
         if (k >= planes) break;
     }
