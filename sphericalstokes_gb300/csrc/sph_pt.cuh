@@ -7,7 +7,7 @@
 //   k_rheo_tau compute_TII! + copy_BC!(τII) + power_law!   :243-265 (FP64: k_rheo, sph_march.cuh)
 //   k_edot_law strain-rate power law (not in the reference; FP64: k_edot, sph_march.cuh)
 //   k_nodes    compute_V!                        :267-329   (sph_march.cuh)
-//   k_bc       BC_R! / BC_θ! / BC_φ! and the cyl/cart BC kernels
+//   k_bc       BC_R! / BC_θ! / BC_φ! and the cyl/cart BC kernels, all stages
 // All three coordinate systems share the kernels; the metric terms come from
 // the template parameter G and the 1D tables in Geo.  The FP32 fused sweep in
 // sph_fused.cuh implements the same arithmetic with shared-memory tiling.
@@ -237,87 +237,217 @@ __global__ void __launch_bounds__(256) k_velocity_norm(KP<T> p) {
 // they are independent.  Each op writes both faces of its field:
 //   NEG     A[b] = -A[in]          COPY  A[b] = A[in]          ZERO  A[b] = 0
 //   LIN     A[b] = (x_cd - c1)*c0  LIN2M A[b] = 2*(x_cd - c1)*c0 - A[in]
-//   STRESS  normal-velocity ghost giving the boundary cell the total normal
-//           stress sig (x2 or x3 faces; not in the reference)
+//   STRESS  normal-velocity ghost that makes the boundary cell divergence-free
+//           (not in the reference)
 // x_cd is the cell-centre coordinate of the node along axis cd.  In the
 // homogeneous form (correction problem) constants vanish: LIN -> 0,
-// LIN2M -> -A[in], sig -> 0.
+// LIN2M -> -A[in].
 // BC_STRESS_SRC: BC_STRESS in a stage that also copies the two tangential fields
 // into their ghost layer; it reads those fields at the copies' source cells
 // instead of at the ghosts the copies are writing (the same values)
 enum BcKind { BC_NEG = 0, BC_COPY = 1, BC_ZERO = 2, BC_LIN = 3, BC_LIN2M = 4, BC_STRESS = 5, BC_STRESS_SRC = 6 };
 struct BcOp { int field; int kind; int cd; double c0, c1; int side; };  // side: -1 both faces, 0 low, 1 high
 struct BcStage { int dim; int nops; BcOp op[3]; };
+// The program as launched: stage D acts on axis D and has one op for every field f and side, op[D][f][side]; a
+// stress op, BC_STRESS_SRC, is on the normal field (bc_closed checks it).  A launch runs the stages
+// first .. last - 1, of which one at most has a stress op, or else it is a single stage.  Then the value of a
+// ghost follows from entries that the launch does not write: undo the stages from the last to the
+// first, each of which replaces a boundary index by an inner one.
+struct BcFaceOp { int kind, cd; double c0, c1; };
+struct BcProg { BcFaceOp op[3][3][2]; };
 
+// V[f] at offset o, as a select between the three pointers
+template <typename T>
+__device__ __forceinline__ T vload(const KP<T>& p, int f, int o) { return (f == 0 ? p.V1 : (f == 1 ? p.V2 : p.V3))[o]; }
 template <typename T>
 __device__ __forceinline__ T* vfield(const KP<T>& p, int f) { return f == 0 ? p.V1 : (f == 1 ? p.V2 : p.V3); }
 
-// one BC stage at face point (u, v) of the stage's faces (both sides); the body of k_bc and of
-// the batched BC launch over many grids
-template <typename T, int G>
-__device__ __forceinline__ void bc_body(const KP<T>& p, const BcStage& st, int homog, int u, int v) {
-    const Dims& d = p.d;
-    const int D = st.dim;
-    const int sy = d.sy, sz = d.sz;
-    for (int o = 0; o < st.nops; ++o) {
-        const BcOp op = st.op[o];
-        const int f = op.field;
-        // extents of field f: V1 (n1+1,n2,n3), V2 (n1,n2+1,n3), V3 (n1,n2,n3+1)
-        int ext[3] = {d.n1 + (f == 0), d.n2 + (f == 1), d.n3 + (f == 2)};
-        const int du = D == 0 ? 1 : 0, dv = D == 2 ? 1 : 2;
-        if (u >= ext[du] || v >= ext[dv]) continue;
-        T* A = vfield(p, f);
-        const int stride[3] = {1, sy, sz};
-        const int base = u * stride[du] + v * stride[dv];
-        for (int side = 0; side < 2; ++side) {
-            if (op.side >= 0 && op.side != side) continue;
-            const int b = side == 0 ? 0 : ext[D] - 1;
-            const int in = side == 0 ? 1 : ext[D] - 2;
-            const int cb = base + b * stride[D], ci = base + in * stride[D];
-            T val;
-            switch (op.kind) {
-                case BC_NEG: val = -A[ci]; break;
-                case BC_COPY: val = A[ci]; break;
-                case BC_ZERO: val = T(0); break;
-                case BC_LIN: {
-                    if (homog) { val = T(0); break; }
-                    const int idx = (op.cd == D) ? b : (op.cd == du ? u : v);
-                    const T* xc = op.cd == 0 ? p.geo.x1c : (op.cd == 1 ? p.geo.x2c : p.geo.x3c);
-                    val = (xc[idx] - T(op.c1)) * T(op.c0);
-                    break;
-                }
-                case BC_LIN2M: {
-                    if (homog) { val = -A[ci]; break; }
-                    const int idx = (op.cd == D) ? b : (op.cd == du ? u : v);
-                    const T* xc = op.cd == 0 ? p.geo.x1c : (op.cd == 1 ? p.geo.x2c : p.geo.x3c);
-                    val = T(2) * (xc[idx] - T(op.c1)) * T(op.c0) - A[ci];
-                    break;
-                }
-                default: {  // BC_STRESS: normal ghost of V1 (D == 0), V2 (D == 1) or V3 (D == 2) from div V = 0 in the boundary cell
-                    const int cellb = side == 0 ? 0 : ext[D] - 2;        // boundary cell index along D
-                    // tangential velocities of the boundary cell: at the ghost, or at the source of its copy
-                    const int ct = base + (op.kind == BC_STRESS_SRC ? cellb + (side == 0 ? 1 : -1) : cellb) * stride[D];
-                    const int i = (D == 0) ? cellb : u;
-                    const int j = (D == 1) ? cellb : (du == 1 ? u : v);
-                    const CellMetric<T> m = cell_metric<T, G>(p, i, j);
-                    if (D == 0)
-                        val = div_ghost<T, G, 0>(m, p.d1, side, A[ci], A[ci], p.V2[ct], p.V2[ct + sy], p.V3[ct], p.V3[ct + sz]);
-                    else if (D == 1)
-                        val = div_ghost<T, G, 1>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], A[ci], A[ci], p.V3[ct], p.V3[ct + sz]);
-                    else
-                        val = div_ghost<T, G, 2>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], p.V2[ct], p.V2[ct + sy], A[ci], A[ci]);
-                    break;
-                }
-            }
-            A[cb] = val;
+// one op with its coordinate factor looked up: applied to the inner value
+template <typename T>
+struct BcAct { int kind; T x, c0; };
+template <typename T>
+__device__ __forceinline__ BcAct<T> bc_act(const KP<T>& p, const BcFaceOp& op, int homog, int idx) {
+    BcAct<T> a;
+    a.kind = op.kind; a.x = T(0); a.c0 = T(0);
+    if (op.kind == BC_LIN || op.kind == BC_LIN2M) {
+        if (homog) {
+            a.kind = op.kind == BC_LIN ? BC_ZERO : BC_NEG;
+        } else {
+            const T* xc = op.cd == 0 ? p.geo.x1c : (op.cd == 1 ? p.geo.x2c : p.geo.x3c);
+            a.x = xc[idx] - T(op.c1);
+            a.c0 = T(op.c0);
         }
+    }
+    return a;
+}
+template <typename T>
+__device__ __forceinline__ T bc_apply(const BcAct<T>& a, T in) {
+    switch (a.kind) {
+        case BC_NEG: return -in;
+        case BC_ZERO: return T(0);
+        case BC_LIN: return a.x * a.c0;
+        case BC_LIN2M: return T(2) * a.x * a.c0 - in;
+        default: return in;
     }
 }
 
+__device__ __forceinline__ int bc_n(const Dims& d, int D) { return D == 0 ? d.n1 : (D == 1 ? d.n2 : d.n3); }
+
+// undo the stages first .. S - 1 at index x of field f: x becomes the index of the value they start from, act[s]
+// what stage s does to it.  Returns the stage whose stress op the entry is (x as that stage sees it), or -1.
+template <typename T, int S>
+__device__ __forceinline__ int bc_resolve(const KP<T>& p, const BcProg& q, int homog, int first, int f, int (&x)[3], BcAct<T> (&act)[S]) {
+    int stop = -1;
+#pragma unroll
+    for (int D = S - 1; D >= 0; --D) {
+        act[D].kind = BC_COPY;
+        const int last = bc_n(p.d, D) - 1 + (f == D);
+        const int side = x[D] == 0 ? 0 : (x[D] == last ? 1 : -1);
+        if (stop >= 0 || side < 0 || D < first) continue;
+        const BcFaceOp& op = q.op[D][f][side];
+        if (op.kind == BC_STRESS_SRC) { stop = D; continue; }
+        act[D] = bc_act(p, op, homog, op.cd == 0 ? x[0] : (op.cd == 1 ? x[1] : x[2]));
+        x[D] = side == 0 ? 1 : last - 1;
+    }
+    return stop;
+}
+
+// the divergence-free ghost of stage D at index x, from values after the stages first .. D - 1 (none with a stress op)
+template <typename T, int G, int D>
+__device__ __forceinline__ T bc_stress(const KP<T>& p, const BcProg& q, int homog, int first, const int (&x)[3]) {
+    const Dims& d = p.d;
+    const int n = bc_n(d, D), side = x[D] == 0 ? 0 : 1;
+    const int cell = side == 0 ? 0 : n - 1, src = side == 0 ? 1 : n - 2, in = side == 0 ? 1 : n - 1;
+    constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;  // tangential axes
+    // inside normal face, low and high faces along A and B: all five resolved, then loaded together
+    const CellMetric<T> c = cell_metric<T, G>(p, D == 0 ? cell : x[0], D == 1 ? cell : x[1]);
+    T v[5];
+    BcAct<T> act[5][D + 1];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+        const int f = m == 0 ? D : (m <= 2 ? A : B);
+        int y[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) y[a] = a == D ? (m == 0 ? in : src) : x[a] + ((m == 2 && a == A) || (m == 4 && a == B) ? 1 : 0);
+        bc_resolve<T, D + 1>(p, q, homog, first, f, y, act[m]);  // (stage D leaves it: y[D] is inside)
+        v[m] = vload(p, f, y[0] + d.sy * y[1] + d.sz * y[2]);
+    }
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+#pragma unroll
+        for (int s = 0; s < D; ++s) v[m] = bc_apply(act[m][s], v[m]);
+    if (D == 0) return div_ghost<T, G, 0>(c, p.d1, side, v[0], v[0], v[1], v[2], v[3], v[4]);
+    if (D == 1) return div_ghost<T, G, 1>(c, p.d1, side, v[1], v[2], v[0], v[0], v[3], v[4]);
+    return div_ghost<T, G, 2>(c, p.d1, side, v[1], v[2], v[3], v[4], v[0], v[0]);
+}
+
+// face point (u, v) of stage D: both faces of every field, loads first.  Other stages of the launch do not touch
+// what it reads: (u, v) is inside along the other two axes, or the launch is this stage alone
+template <typename T, int G, int D>
+__device__ __forceinline__ void bc_face(const KP<T>& p, const BcProg& q, int homog, int u, int v) {
+    const Dims& d = p.d;
+    const int x0 = D == 0 ? 0 : u, x1 = D == 1 ? 0 : (D == 0 ? u : v), x2 = D == 2 ? 0 : v;
+    const int base = x0 + d.sy * x1 + d.sz * x2, step = D == 0 ? 1 : (D == 1 ? d.sy : d.sz);
+    const int nu = D == 0 ? d.n2 : d.n1, nv = D == 2 ? d.n2 : d.n3, du = D == 0 ? 1 : 0, dv = D == 2 ? 1 : 2, n = bc_n(d, D);
+    T val[3][2];
+    BcAct<T> act[3][2];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        const int last = n - 1 + (f == D);
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const BcFaceOp& op = q.op[D][f][side];
+            act[f][side].kind = -1;
+            if (u >= nu + (f == du) || v >= nv + (f == dv) || op.kind == BC_STRESS_SRC) continue;
+            val[f][side] = vload(p, f, base + (side == 0 ? 1 : last - 1) * step);
+            act[f][side] = bc_act(p, op, homog, op.cd == D ? (side == 0 ? 0 : last) : (op.cd == 0 ? x0 : (op.cd == 1 ? x1 : x2)));
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int side = 0; side < 2; ++side)
+            if (act[f][side].kind >= 0) vfield(p, f)[base + (side == 0 ? 0 : n - 1 + (f == D)) * step] = bc_apply(act[f][side], val[f][side]);
+    if (u >= nu || v >= nv) return;
+    for (int side = 0; side < 2; ++side) {
+        if (q.op[D][D][side].kind != BC_STRESS_SRC) continue;
+        const int cell = side == 0 ? 0 : n - 1, ci = base + (side == 0 ? 1 : n - 1) * step, ct = base + (side == 0 ? 1 : n - 2) * step;
+        const CellMetric<T> m = cell_metric<T, G>(p, D == 0 ? cell : x0, D == 1 ? cell : x1);
+        T g;
+        if (D == 0)
+            g = div_ghost<T, G, 0>(m, p.d1, side, p.V1[ci], p.V1[ci], p.V2[ct], p.V2[ct + d.sy], p.V3[ct], p.V3[ct + d.sz]);
+        else if (D == 1)
+            g = div_ghost<T, G, 1>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], p.V2[ci], p.V2[ci], p.V3[ct], p.V3[ct + d.sz]);
+        else
+            g = div_ghost<T, G, 2>(m, p.d1, side, p.V1[ct], p.V1[ct + 1], p.V2[ct], p.V2[ct + d.sy], p.V3[ci], p.V3[ci]);
+        vfield(p, D)[base + (side == 0 ? 0 : n) * step] = g;
+    }
+}
+
+// Stages first .. last - 1 in one launch.  A single stage: blocks of face points.  Otherwise blocks z < last - first
+// take the points of their stage's faces that are inside along the other axes, and the blocks of the last
+// z everything near an edge of the box: a warp per 32 points of a line (field, direction of the line, places of the
+// other two indices) or per field's corners, each ghost undone to entries that the launch does not write.
+// Ghosts of a later stage are left to it.
+// (One stress op at most: its inputs then resolve to values that need no other stress ghost.)
+// Bound by latency, of the launch and of loads and stores in a row.  us per iteration with a launch for each
+// stage and each op's load behind the store before, and so: FP64 70 x 5 x 5 27.4 and 19.4,
+// FP32 95 x 79 x 67 42.1 and 33.9, FP64 63^3 126 and 117.5.
 template <typename T, int G>
-__global__ void k_bc(KP<T> p, BcStage st, int homog) {
+__global__ void __launch_bounds__(128) k_bc(const __grid_constant__ KP<T> p, const __grid_constant__ BcProg q, int homog, int first, int last) {
     pdl_enter();
-    bc_body<T, G>(p, st, homog, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
+    const Dims& d = p.d;
+    const int z = first + blockIdx.z;
+    const bool single = last - first == 1;
+    if (z < last) {
+        const int u = blockIdx.x * 32 + threadIdx.x, v = blockIdx.y * blockDim.y + threadIdx.y;
+        if (!single && (u < 1 || v < 1 || u > bc_n(d, z == 0 ? 1 : 0) - 2 || v > bc_n(d, z == 2 ? 1 : 2) - 2)) return;
+        if (z == 0) bc_face<T, G, 0>(p, q, homog, u, v);
+        else if (z == 1) bc_face<T, G, 1>(p, q, homog, u, v);
+        else bc_face<T, G, 2>(p, q, homog, u, v);
+        return;
+    }
+    const int w0 = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.y + threadIdx.y, nw = gridDim.x * gridDim.y * blockDim.y;
+    const int per = (max(d.n1, max(d.n2, d.n3)) + 29) / 32;  // warps of a line's n - 2 inner points
+    for (int w = w0; w < 3 + 81 * per; w += nw) {
+        int f = w, ax = 0, t = 0, b, c;
+        if (w < 3) {  // corners
+            if (threadIdx.x >= 27) continue;
+            const int a = threadIdx.x % 3;
+            b = threadIdx.x / 3 % 3;
+            c = threadIdx.x / 9;
+            if (a == 2 && f != 0) continue;
+            t = a == 0 ? 0 : d.n1 - 2 + a;
+        } else {
+            const int line = (w - 3) / per;
+            f = line / 27; ax = line / 9 % 3; b = line / 3 % 3; c = line % 3;
+            t = 1 + ((w - 3) % per) * 32 + threadIdx.x;
+            if (t > bc_n(d, ax) - 2) continue;
+        }
+        const int B = ax == 0 ? 1 : 0, C = ax == 2 ? 1 : 2;
+        if ((b == 2 && f != B) || (c == 2 && f != C)) continue;
+        const int xb = b == 0 ? 0 : bc_n(d, B) - 2 + b, xc = c == 0 ? 0 : bc_n(d, C) - 2 + c;
+        int x[3] = {ax == 0 ? t : xb, ax == 1 ? t : (ax == 0 ? xb : xc), ax == 2 ? t : xc};
+        bool ghost = false, later = false;
+#pragma unroll
+        for (int D = 0; D < 3; ++D) {
+            const bool g = x[D] == 0 || x[D] == bc_n(d, D) - 1 + (f == D);
+            if (D >= last) later = later || g;
+            else if (D >= first) ghost = ghost || g;
+        }
+        if (!ghost || later) continue;
+        const int at = x[0] + d.sy * x[1] + d.sz * x[2];
+        BcAct<T> act[3];
+        const int stop = bc_resolve<T, 3>(p, q, homog, first, f, x, act);
+        T v;
+        if (stop < 0) v = vload(p, f, x[0] + d.sy * x[1] + d.sz * x[2]);
+        else if (stop == 0) v = bc_stress<T, G, 0>(p, q, homog, first, x);
+        else if (stop == 1) v = bc_stress<T, G, 1>(p, q, homog, first, x);
+        else v = bc_stress<T, G, 2>(p, q, homog, first, x);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) v = bc_apply(act[s], v);
+        vfield(p, f)[at] = v;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -91,7 +91,7 @@ struct Ctx {
     unsigned long long* red = nullptr;   // device reduction slots
     unsigned long long* hred = nullptr;  // pinned host copy
     std::vector<BcStage> bc;      // BC program: ghost-velocity stages in the reference order (the adjoint transposes these)
-    std::vector<BcStage> bc_run;  // the program launched by launch_bc: bc, or an equivalent one with fewer stages
+    BcProg bc_run{};          // the program launched by launch_bc: bc with one stage per axis
     // the homogeneous program in closed form for the correction sweep (SweepOut): set where every
     // ghost is a multiple of its interior neighbour or divergence-free; SPH_NO_XGHOST=1: not used,
     // the BC launches follow each sweep
@@ -288,21 +288,48 @@ void build_ghosts(Ctx& c) {
     for (int i = 0; i < 9; ++i) c.ghost_gf[i] = gf[i];
 }
 
+// c.bc_run: the ops of each axis by field and side.  A stress op then shares its stage with the copies of the
+// tangential fields and reads their sources.  Checks what k_bc relies on (BcProg).
+int bc_closed(Ctx& c) {
+    std::memset(&c.bc_run, 0, sizeof(c.bc_run));
+    int seen = 0, dim = 0;
+    bool ok = true;
+    for (const BcStage& st : c.bc) {
+        ok = ok && st.dim >= dim && st.dim < 3;
+        if (!ok) break;
+        dim = st.dim;
+        for (int i = 0; i < st.nops; ++i) {
+            const BcOp& op = st.op[i];
+            for (int side = 0; side < 2; ++side) {
+                if (op.side >= 0 && op.side != side) continue;
+                const int bit = 1 << (6 * dim + 2 * op.field + side);
+                ok = ok && !(seen & bit);
+                seen |= bit;
+                BcFaceOp& r = c.bc_run.op[dim][op.field][side];
+                r.kind = op.kind; r.cd = op.cd; r.c0 = op.c0; r.c1 = op.c1;
+                if (op.kind == BC_STRESS) {
+                    r.kind = BC_STRESS_SRC;
+                    ok = ok && op.field == dim;
+                    for (int f = 0; f < 3; ++f) ok = ok && (f == dim || ((seen >> (6 * dim + 2 * f + side) & 1) && c.bc_run.op[dim][f][side].kind == BC_COPY));
+                }
+            }
+        }
+    }
+    return ok && seen == (1 << 18) - 1 ? SPH_OK : fail(SPH_ERR_UNSUPPORTED, "boundary program does not set every ghost once, axis by axis");
+}
+
 int build_bc_program(Ctx& c);
 int build_bc(Ctx& c) {
     const int rc = build_bc_program(c);
     if (rc != SPH_OK) return rc;
-    if (c.bc_run.empty()) c.bc_run = c.bc;
     build_ghosts(c);
-    return SPH_OK;
+    return bc_closed(c);
 }
 
-// the ghost-velocity stages of the BC set (Julia reference order), in c.bc; a
-// shorter equivalent program for the launches goes to c.bc_run where one exists
+// the ghost-velocity stages of the BC set (Julia reference order), in c.bc
 int build_bc_program(Ctx& c) {
     const sph_params& q = c.prm;
     c.bc.clear();
-    c.bc_run.clear();
     const double rsh = q.r * q.sh;
     if (q.bc == SPH_BC_FREE_SLIP) {  // SphericalStokes_plateau.jl:64-92
         c.bc.push_back(stage(0, {op(0, BC_NEG), op(1, BC_COPY), op(2, BC_COPY)}));
@@ -317,12 +344,6 @@ int build_bc_program(Ctx& c) {
         c.bc.push_back(stage(1, {op(1, BC_STRESS)}));
         c.bc.push_back(stage(2, {op(0, BC_COPY), op(1, BC_COPY)}));
         c.bc.push_back(stage(2, {op(2, BC_STRESS)}));
-        // the launched program: each copy stage merged with the stress stage after it,
-        // whose op then reads the copies' sources (same values, three launches)
-        c.bc_run.clear();
-        c.bc_run.push_back(c.bc[0]);
-        c.bc_run.push_back(stage(1, {op(0, BC_COPY), op(2, BC_COPY), op(1, BC_STRESS_SRC)}));
-        c.bc_run.push_back(stage(2, {op(0, BC_COPY), op(1, BC_COPY), op(2, BC_STRESS_SRC)}));
         return SPH_OK;
     }
     if (q.bc == SPH_BC_FREE_SURFACE) {  // free slip but at the top x1 face; its ghost after the copies
@@ -357,12 +378,15 @@ int build_bc_program(Ctx& c) {
 
 template <typename T, int G>
 void launch_bc(Ctx& c, KP<T>& p, int homog) {
-    for (size_t i = 0; i < c.bc_run.size(); ++i) {
-        const BcStage& st = c.bc_run[i];
-        int eu = st.dim == 0 ? c.d.n2 + 1 : c.d.n1 + 1;
-        int ev = st.dim == 2 ? c.d.n2 + 1 : c.d.n3 + 1;
-        dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
-        launch_pdl(c.use_pdl, k_bc<T, G>, g, blk2d(), 0, c.stream, p, st, homog);
+    const int eu = c.d.n1 > c.d.n2 ? c.d.n1 : c.d.n2, ev = c.d.n2 > c.d.n3 ? c.d.n2 : c.d.n3;
+    const int rows = (eu + 31) / 32 * (long long)ev <= 4LL * c.sms ? 1 : 4;  // (a warp per SM while they last)
+    auto stress = [&](int s) { return (int)(c.bc_run.op[s][s][0].kind == BC_STRESS_SRC || c.bc_run.op[s][s][1].kind == BC_STRESS_SRC); };
+    for (int a = 0, b; a < 3; a = b) {
+        int n = stress(a);
+        for (b = a + 1; b < 3 && n + stress(b) <= 1; ++b) n += stress(b);
+        const int gx = (eu + 32) / 32, edges = b - a == 1 ? 0 : (3 + 81 * ((std::max(eu, ev) + 29) / 32) + gx * rows - 1) / (gx * rows);
+        launch_pdl(c.use_pdl, k_bc<T, G>, dim3(gx, std::max((ev + rows) / rows, edges), b - a == 1 ? 1 : b - a + 1), dim3(32, rows), 0, c.stream, p, c.bc_run,
+                   homog, a, b);
     }
 }
 
