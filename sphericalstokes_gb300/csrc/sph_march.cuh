@@ -24,11 +24,15 @@
 
 namespace sph {
 
-constexpr int MC_NT = 128;  // threads per block
+// Threads per block.  No block shares anything, and the FP64 units of the fullest SM end last: single warps spread
+// most evenly.  us per iteration with blocks of 128 and of 32: 63^3 116.9 and 114.1, sector 21 x 15 x 138 44.3 and
+// 40.3, sector 110 x 28 x 30 64.1 and 60.2, 207^3 Cartesian 3372 and 3347, 127^3 sector 819 and 821.
+constexpr int MC_NT = 32;
 
 // planes per thread: enough to pay for the column's coefficients (`setup`, in planes), few enough for an even
 // share of blocks per SM (the FP64 units are the only bound, so the fullest SM ends last) and for `need`
-// blocks per SM, below which the loads of a plane are not hidden behind its FP64 instructions
+// times four warps per SM, below which the loads of a plane are not hidden behind its FP64 instructions; one more for
+// the tail, where the last warps of an SM run alone
 inline int march_chunk(long long columns, int planes, int sms, double setup, double need) {
     const long long cols = (columns + MC_NT - 1) / MC_NT;
     int best = 1;
@@ -36,7 +40,7 @@ inline int march_chunk(long long columns, int planes, int sms, double setup, dou
     for (int k = 1; k <= 16 && k <= planes; ++k) {
         const long long blocks = cols * ((planes + k - 1) / k);
         const double n = (double)((blocks + sms - 1) / sms);
-        const double t = (n > need ? n : need) * (k + setup);
+        const double t = ((n > 4 * need ? n : 4 * need) + 1.0) * (k + setup);
         if (t < best_t) { best_t = t; best = k; }
     }
     return best;
