@@ -22,7 +22,7 @@ namespace sph {
 struct BatchSweep {
     KP<float> p[2];                // correction problem in both ping-pong arrangements (a: the sweep reads p[a])
     SweepOut<float> o[2];          // outputs of a sweep reading arrangement a (the other buffer set)
-    const CUtensorMap* maps[2];    // TMA maps of the arrangement a sweep reads
+    SweepMaps maps[2];             // TMA maps of the arrangement a sweep reads
     int* err;                      // the solve's bounded-wait error word
     int geom;
 };
@@ -47,10 +47,14 @@ __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __re
     copy(&p, &s.p[a], sizeof(p));
     copy(&o, &s.o[a], sizeof(o));
     __syncthreads();
+    // maps in global memory are copied there between launches: the copy unit may hold older ones of this address
+    if (threadIdx.x == SW_NT - 32)
+        for (int i = 0; i < SM_COUNT; ++i)
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(s.maps[a].m + i) : "memory");
     const int kc = kchunk[it.x];
-    if (s.geom == SPH) sweep_body<SPH, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
-    else if (s.geom == CYL) sweep_body<CYL, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
-    else sweep_body<CART, 1>(p, o, kc, s.maps[a], s.err, it.y, it.z, it.w);
+    if (s.geom == SPH) sweep_body<SPH, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
+    else if (s.geom == CYL) sweep_body<CYL, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
+    else sweep_body<CART, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
 }
 
 // inner stopping test of every active solve: max |dV + rV| of arrangement 0 into red[solve];

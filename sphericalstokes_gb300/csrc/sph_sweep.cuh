@@ -178,6 +178,7 @@ constexpr int SI_N = SI_X * SI_Y, SO_N = SO_X * SO_Y, SR_N = SR_X * SO_Y, SV_N =
 
 // tensor maps of one arrangement of the buffers
 enum SweepMap { SM_V = 0, SM_ETA, SM_ETASM, SM_P, SM_TAU, SM_RP, SM_RHO, SM_RV, SM_COUNT };
+struct SweepMaps { alignas(128) CUtensorMap m[SM_COUNT]; };
 
 constexpr int pad128(int floats) { return (floats + 31) / 32 * 32; }
 struct SweepSmem {
@@ -270,6 +271,7 @@ __device__ __forceinline__ void sweep_fill_ghosts(const KP<float>* pp, int smask
         else v[4] = g;
     }
 }
+// maps: tensor maps among the launch's parameters, or in global memory after a tensor-map fence
 template <int G, int MODE>
 __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<float>& o, int kchunk, const CUtensorMap* __restrict__ maps,
                                            int* __restrict__ err, int bx, int by, int bz) {
@@ -703,9 +705,9 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
 
 template <int G, int MODE>
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep(const __grid_constant__ KP<float> p, const __grid_constant__ SweepOut<float> o, int kchunk,
-                                                    const CUtensorMap* __restrict__ maps, int* __restrict__ err) {
+                                                    const __grid_constant__ SweepMaps maps, int* __restrict__ err) {
     pdl_wait();  // no early release of the next grid: its blocks would take SM slots in this grid's tail
-    sweep_body<G, MODE>(p, o, kchunk, maps, err, blockIdx.x, blockIdx.y, blockIdx.z);
+    sweep_body<G, MODE>(p, o, kchunk, maps.m, err, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 }  // namespace sph

@@ -118,7 +118,7 @@ struct Ctx {
     int warm_len = 0;
     bool use_graphs = true;
     // TMA tensor maps of the sweep, one set per arrangement of the ping-pong and η buffers
-    CUtensorMap* d_maps = nullptr;       // [4][SM_COUNT] in device memory
+    SweepMaps maps[4];
     float* map_key[4][2] = {};           // V1 and η buffers of the arrangement a set was built for
     int* d_err = nullptr;                // set by a kernel whose bounded wait ran out
     bool use_tma = true;
@@ -698,22 +698,20 @@ bool encode_map(const Ctx& c, CUtensorMap* m, const float* base, int nf, unsigne
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// maps of the current buffer arrangement; returns the device pointer of the set or nullptr
-const CUtensorMap* tma_maps(Ctx& c) {
+// Maps of the current buffer arrangement, or nullptr.  They go to the sweep among its launch parameters: a copy to
+// device memory would have to be ordered before the launch on its stream, and fenced in every block.
+const SweepMaps* tma_maps(Ctx& c) {
     if (!c.use_tma) return nullptr;
     State<float>& t = c.s32;
     int slot = 0;
     for (; slot < 4 && c.map_key[slot][0]; ++slot)
-        if (c.map_key[slot][0] == t.f[F_V1] && c.map_key[slot][1] == t.f[F_ETA]) return c.d_maps + slot * SM_COUNT;
+        if (c.map_key[slot][0] == t.f[F_V1] && c.map_key[slot][1] == t.f[F_ETA]) return &c.maps[slot];
     if (slot == 4) return nullptr;
-    if (!c.d_maps) {
-        if (cudaMalloc((void**)&c.d_maps, sizeof(CUtensorMap) * 4 * SM_COUNT) != cudaSuccess) { c.use_tma = false; return nullptr; }
-    }
     if (!c.d_err) {
         if (cudaMalloc((void**)&c.d_err, sizeof(int)) != cudaSuccess) { c.use_tma = false; return nullptr; }
         cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream);
     }
-    CUtensorMap h[SM_COUNT];
+    CUtensorMap* h = c.maps[slot].m;
     bool ok = encode_map(c, &h[SM_V], t.f[F_V1], 3, SI_X, SI_Y);
     ok &= encode_map(c, &h[SM_ETA], t.f[F_ETA], 1, SI_X, SI_Y);
     ok &= encode_map(c, &h[SM_ETASM], t.f[F_ETA_SM], 1, SI_X, SI_Y);
@@ -722,13 +720,13 @@ const CUtensorMap* tma_maps(Ctx& c) {
     ok &= encode_map(c, &h[SM_RP], t.f[F_RP], 1, SO_X, SO_Y);
     ok &= encode_map(c, &h[SM_RHO], t.f[F_RHO], 1, SO_X, SO_Y);
     ok &= encode_map(c, &h[SM_RV], t.f[F_RV1], 3, SWX, SWY);
-    if (!ok || cudaMemcpy(c.d_maps + slot * SM_COUNT, h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (!ok) {
         c.use_tma = false;
         return nullptr;
     }
     c.map_key[slot][0] = t.f[F_V1];
     c.map_key[slot][1] = t.f[F_ETA];
-    return c.d_maps + slot * SM_COUNT;
+    return &c.maps[slot];
 }
 
 // build the tensor-map sets of all four arrangements (never inside a graph capture)
@@ -781,8 +779,8 @@ SweepOut<float> sweep_out(const Ctx& c, const KP<float>& p, bool fill) {
 template <int G, int MODE>
 bool launch_fused(Ctx& c, const KP<float>& p, bool fill) {
     const int kc = fused_chunk(c);
-    if (const CUtensorMap* maps = tma_maps(c)) {
-        launch_pdl(c.use_pdl, k_sweep<G, MODE>, sweep_grid(c.d, kc), dim3(SW_NT, 1, 1), sweep_smem_bytes(), c.stream, p, sweep_out(c, p, fill), kc, maps, c.d_err);
+    if (const SweepMaps* maps = tma_maps(c)) {
+        launch_pdl(c.use_pdl, k_sweep<G, MODE>, sweep_grid(c.d, kc), dim3(SW_NT, 1, 1), sweep_smem_bytes(), c.stream, p, sweep_out(c, p, fill), kc, *maps, c.d_err);
         return fill;
     }
     dim3 grid((c.d.n1 + FTX - 1) / FTX, (c.d.n2 + FTY - 1) / FTY, (c.d.n3 + kc - 1) / kc);
@@ -1429,11 +1427,11 @@ int batch_entry(Ctx& c, BatchSweep& e) {
     ensure_tma_maps(c);
     State<float>& t = c.s32;
     for (int a = 0; a < 2; ++a) {
-        const CUtensorMap* maps = tma_maps(c);
+        const SweepMaps* maps = tma_maps(c);
         if (!maps || !c.d_err) return fail(SPH_ERR_UNSUPPORTED, "batched sweeps need the TMA sweep");
         e.p[a] = make_kp_corr(c);
         e.o[a] = sweep_out(c, e.p[a], true);
-        e.maps[a] = maps;
+        e.maps[a] = *maps;
         swap_state(t);
     }
     e.err = c.d_err;
@@ -1988,7 +1986,6 @@ int sph_destroy(void* h) {
     free_state(c->s64);
     free_state(c->s32);
     if (c->phase) cudaFree(c->phase);
-    if (c->d_maps) cudaFree(c->d_maps);
     if (c->d_err) cudaFree(c->d_err);
     if (c->red) cudaFree(c->red);
     if (c->hred) cudaFreeHost(c->hred);
