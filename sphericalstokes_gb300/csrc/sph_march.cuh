@@ -158,15 +158,14 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
 }
 
 template <typename T, int G, int MODE>
-__global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p, int chunk) {
-    pdl_enter_small();
+__device__ __forceinline__ void nodes_body(const KP<T>& p, int chunk, int by) {
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int w = d.n1 - 1;
     const int I = col % w + 1, J = col / w + 1;
     if (J > d.n2 - 1) return;
     const int sy = d.sy, sz = d.sz;
-    const int K0 = blockIdx.y * chunk + 1, K1 = min(K0 + chunk, d.n3);  // K0 .. K1 - 1
+    const int K0 = by * chunk + 1, K1 = min(K0 + chunk, d.n3);  // K0 .. K1 - 1
     // the update wants the residual times (DT + DT') / 2: its half is folded into the coefficients
     const T s = MODE == 2 ? T(1) : T(0.5), h = T(0.5);
     const MomMetric<T> m = mom_metric<T, G>(p.geo, I, J, d.n1, d.n2);
@@ -228,18 +227,22 @@ __global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p
         q33 = s33; qdt = dt; p13a = t13a; p13b = t13b; p23 = t23;
     }
 }
+template <typename T, int G, int MODE>
+__global__ void __launch_bounds__(MC_NT) k_nodes(const __grid_constant__ KP<T> p, int chunk) {
+    pdl_enter_small();
+    nodes_body<T, G, MODE>(p, chunk, blockIdx.y);
+}
 
 // strain-rate power law (k_edot_law of sph_pt.cuh is the FP32 one): with x = (ε̇_II / ε̇_bg)^2 of the clamped
 // interior cell, η_t = 2 / (1/η_ini + 1/η_PL) = 2 η_ini / (1 + x^((n-1)/(2n))); RELAXED: η_out = η^(1-relax) η_t^relax
 template <bool RELAXED>
-__global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<double> p, int chunk) {
-    pdl_enter_small();
+__device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by) {
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
     if (j >= d.n2) return;
     const int sy = d.sy, sz = d.sz;
-    const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
+    const int k0 = by * chunk, k1 = min(k0 + chunk, d.n3);
     const double* tab = p.geo.pow_tab;
     const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
     int last = -1;
@@ -269,19 +272,23 @@ __global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<doubl
         p.eta_out[c] = et;
     }
 }
+template <bool RELAXED>
+__global__ void __launch_bounds__(MC_NT) k_edot(const __grid_constant__ KP<double> p, int chunk) {
+    pdl_enter_small();
+    edot_body<RELAXED>(p, chunk, blockIdx.y);
+}
 
 // compute_TII! + copy_BC!(τII) + power_law! (k_rheo_tau of sph_pt.cuh is the FP32 one): with x = (τII / τ_C)^2,
 // η_PL = η_ini x^((1-n)/2), η = 2 / (1/η_ini + 1/η_PL); RELAX: η_PL relaxed in log space
 // (CylindricalStokes_diapir.jl:185-192).  phase == 1 cells are linear.
 template <bool RELAX>
-__global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, int chunk) {
-    pdl_enter_small();
+__device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, int chunk, int by) {
     const Dims& d = p.d;
     const int col = blockIdx.x * MC_NT + threadIdx.x;
     const int i = col % d.n1, j = col / d.n1;
     if (j >= d.n2) return;
     const int sy = d.sy, sz = d.sz;
-    const int k0 = blockIdx.y * chunk, k1 = min(k0 + chunk, d.n3);
+    const int k0 = by * chunk, k1 = min(k0 + chunk, d.n3);
     const double* tab = p.geo.pow_tab;
     const int s0 = clampi(i, 1, d.n1 - 2) + sy * clampi(j, 1, d.n2 - 2);
     const int rim = (i == 0 || i == d.n1 - 1) + (j == 0 || j == d.n2 - 1);
@@ -341,6 +348,26 @@ __global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<doubl
             p.eta[c] = done && normal_pos(num) ? fast_div(num, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
         }
     }
+}
+
+template <bool RELAX>
+__global__ void __launch_bounds__(MC_NT) k_rheo(const __grid_constant__ KP<double> p, int faces_only, int chunk) {
+    pdl_enter_small();
+    rheo_body<RELAX>(p, faces_only, chunk, blockIdx.y);
+}
+
+// compute_V! and the viscosity law of one iteration in one launch: both follow the stresses and neither reads what
+// the other writes.  Blocks y < ny update the velocities, the others the viscosity.  LAW 0, 1: stress power law, plain
+// and relaxed; 2: strain-rate power law, relaxed.  With ηSM of the next iteration in the boundary launch (k_bc), three
+// launches an iteration in place of five; us per iteration: 70 x 5 x 5 18.6 and 12.9, spherical 63^3 114.0 and 107.7,
+// 127^3 sector 818 and 797, sector 21 x 15 x 138 39.6 and 35.7, FP32 95 x 79 x 67 (four launches, three) 33.9 and 30.9.
+template <int G, int LAW>
+__global__ void __launch_bounds__(MC_NT) k_nodes_law(const __grid_constant__ KP<double> p, int faces_only, int kn, int ny, int kl) {
+    pdl_enter_small();
+    const int by = blockIdx.y;
+    if (by < ny) nodes_body<double, G, 0>(p, kn, by);
+    else if (LAW == 2) edot_body<true>(p, kl, by - ny);
+    else rheo_body<LAW == 1>(p, faces_only, kl, by - ny);
 }
 
 }  // namespace sph

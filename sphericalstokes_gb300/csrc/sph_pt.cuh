@@ -38,9 +38,7 @@ __device__ __forceinline__ int order_bits(float x) {
 }
 __device__ __forceinline__ float from_order(int b, float) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); }
 template <typename T>
-__global__ void k_maxloc(KP<T> p, int faces_only) {
-    pdl_enter_small();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
+__device__ __forceinline__ void maxloc_body(const KP<T>& p, int faces_only, int i, int j, int k) {
     const Dims& d = p.d;
     if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;
     const int c = i + d.sy * j + d.sz * k;
@@ -53,6 +51,11 @@ __global__ void k_maxloc(KP<T> p, int faces_only) {
     const int off[6] = {-1, 1, -d.sy, d.sy, -d.sz, d.sz};
     for (int q = 0; q < 6; ++q) m = max(m, order_bits(E[s + off[q]]));
     p.etaSM[c] = from_order(m, T(0));
+}
+template <typename T>
+__global__ void k_maxloc(const __grid_constant__ KP<T> p, int faces_only) {
+    pdl_enter_small();
+    maxloc_body(p, faces_only, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -384,21 +387,35 @@ __device__ __forceinline__ void bc_face(const KP<T>& p, const BcProg& q, int hom
     }
 }
 
+constexpr int BC_SM_PLANES = 4;  // planes of ηSM per thread
+
 // Stages first .. last - 1 in one launch.  A single stage: blocks of face points.  Otherwise blocks z < last - first
 // take the points of their stage's faces that are inside along the other axes, and the blocks of the last
 // z everything near an edge of the box: a warp per 32 points of a line (field, direction of the line, places of the
 // other two indices) or per field's corners, each ghost undone to entries that the launch does not write.
 // Ghosts of a later stage are left to it.
 // (One stress op at most: its inputs then resolve to values that need no other stress ghost.)
+// Blocks past those, where a launch has them: ηSM of the next iteration (its η is final, and no boundary value enters).
 // Bound by latency, of the launch and of loads and stores in a row.  us per iteration with a launch for each
 // stage and each op's load behind the store before, and so: FP64 70 x 5 x 5 27.4 and 19.4,
 // FP32 95 x 79 x 67 42.1 and 33.9, FP64 63^3 126 and 117.5.
 template <typename T, int G>
-__global__ void __launch_bounds__(128) k_bc(const __grid_constant__ KP<T> p, const __grid_constant__ BcProg q, int homog, int first, int last) {
-    pdl_enter();
+__global__ void __launch_bounds__(128) k_bc(const __grid_constant__ KP<T> p, const __grid_constant__ BcProg q, int homog, int first, int last, int early) {
+    pdl_wait();
+    if (early) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const Dims& d = p.d;
     const int z = first + blockIdx.z;
     const bool single = last - first == 1;
+    const int nz = single ? 1 : last - first + 1;
+    if (blockIdx.z >= nz) {
+        const int nt = 32 * blockDim.y, cols = (d.n1 * d.n2 + nt - 1) / nt;
+        const int lin = ((blockIdx.z - nz) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+        const int col = lin % cols * nt + threadIdx.y * 32 + threadIdx.x, k0 = lin / cols * BC_SM_PLANES;
+        const int i = col % d.n1, j = col / d.n1;
+#pragma unroll
+        for (int k = 0; k < BC_SM_PLANES; ++k) maxloc_body(p, (int)(G == CART), i, j, k0 + k);
+        return;
+    }
     if (z < last) {
         const int u = blockIdx.x * 32 + threadIdx.x, v = blockIdx.y * blockDim.y + threadIdx.y;
         if (!single && (u < 1 || v < 1 || u > bc_n(d, z == 0 ? 1 : 0) - 2 || v > bc_n(d, z == 2 ? 1 : 2) - 2)) return;

@@ -377,7 +377,7 @@ int build_bc_program(Ctx& c) {
 }
 
 template <typename T, int G>
-void launch_bc(Ctx& c, KP<T>& p, int homog) {
+void launch_bc(Ctx& c, KP<T>& p, int homog, bool next_sm = false) {
     const int eu = c.d.n1 > c.d.n2 ? c.d.n1 : c.d.n2, ev = c.d.n2 > c.d.n3 ? c.d.n2 : c.d.n3;
     const int rows = (eu + 31) / 32 * (long long)ev <= 4LL * c.sms ? 1 : 4;  // (a warp per SM while they last)
     auto stress = [&](int s) { return (int)(c.bc_run.op[s][s][0].kind == BC_STRESS_SRC || c.bc_run.op[s][s][1].kind == BC_STRESS_SRC); };
@@ -385,8 +385,12 @@ void launch_bc(Ctx& c, KP<T>& p, int homog) {
         int n = stress(a);
         for (b = a + 1; b < 3 && n + stress(b) <= 1; ++b) n += stress(b);
         const int gx = (eu + 32) / 32, edges = b - a == 1 ? 0 : (3 + 81 * ((std::max(eu, ev) + 29) / 32) + gx * rows - 1) / (gx * rows);
-        launch_pdl(c.use_pdl, k_bc<T, G>, dim3(gx, std::max((ev + rows) / rows, edges), b - a == 1 ? 1 : b - a + 1), dim3(32, rows), 0, c.stream, p, c.bc_run,
-                   homog, a, b);
+        const int nz = b - a == 1 ? 1 : b - a + 1, gy = std::max((ev + rows) / rows, edges);
+        const bool sm = next_sm && b == 3;
+        const int smb = sm ? (c.d.n1 * c.d.n2 + 32 * rows - 1) / (32 * rows) * ((c.d.n3 + BC_SM_PLANES - 1) / BC_SM_PLANES) : 0;
+        // (the next grid is released early only without ηSM blocks: beside them it is placed unevenly, 31 us an iteration
+        // becoming 43 at FP32 95 x 79 x 67)
+        launch_pdl(c.use_pdl, k_bc<T, G>, dim3(gx, gy, nz + (smb + gx * gy - 1) / (gx * gy)), dim3(32, rows), 0, c.stream, p, c.bc_run, homog, a, b, (int)!sm);
     }
 }
 
@@ -612,16 +616,46 @@ void launch_rheology(Ctx& c, State<T>& s, KP<T>& p, bool strains = false) {
     }
 }
 
+// the velocity update and the viscosity law of an iteration, in one launch (FP64)
+template <int G, int LAW>
+void launch_nodes_law(Ctx& c, const KP<double>& p) {
+    const long long nodes = (long long)(c.d.n1 - 1) * (c.d.n2 - 1), cols = (long long)c.d.n1 * c.d.n2;
+    const int kn = march_chunk(nodes, c.d.n3 - 1, c.sms, 0.8, 3.0), kl = march_chunk(cols, c.d.n3, c.sms, 0.1, 3.0);
+    const int ny = (c.d.n3 - 1 + kn - 1) / kn;
+    launch_pdl(c.use_pdl, k_nodes_law<G, LAW>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), ny + (c.d.n3 + kl - 1) / kl), dim3(MC_NT), 0, c.stream, p,
+               (int)(G == CART), kn, ny, kl);
+}
+
+// One PT iteration.  A run of iterations computes the ηSM of each but the first with the boundary values of the
+// one before (k_bc); the last leaves ηSM as the reference does, that of the η its stresses used.
+struct IterPos { bool first = true, last = true; };
+inline bool chains_sm(const Ctx& c) { return c.prm.etasm_passes <= 1; }
+
 template <typename T, int G>
-void iterate_one(Ctx& c, State<T>& s) {
+void iterate_one(Ctx& c, State<T>& s, IterPos at) {
     KP<T> p = make_kp<T>(c, s);
-    launch_maxloc<T, G>(c, p);
-    const bool law = c.prm.rheology == SPH_RHEO_EDOT_POWER_RELAX;
+    if (at.first || !chains_sm(c)) launch_maxloc<T, G>(c, p);
+    const int rh = c.prm.rheology;
+    const bool law = rh == SPH_RHEO_EDOT_POWER_RELAX;
     if (law) launch_cells<T, G, WHAT_STRESS_LAW>(c, p);
     else launch_cells<T, G, WHAT_STRESS>(c, p);
-    launch_rheology<T, G>(c, s, p, law);
-    launch_nodes<T, G, 0>(c, p);
-    launch_bc<T, G>(c, p, 0);
+    if constexpr (sizeof(T) == 8) {
+        if (law) {
+            launch_nodes_law<G, 2>(c, p);
+            std::swap(s.f[F_ETA], s.f[F_ETA_OUT]);
+            p.eta = s.f[F_ETA]; p.eta_out = s.f[F_ETA_OUT];
+        } else if (rh == SPH_RHEO_TAU_POWER) {
+            launch_nodes_law<G, 0>(c, p);
+        } else if (rh == SPH_RHEO_TAU_POWER_RELAX && c.cur_n > 1.0) {
+            launch_nodes_law<G, 1>(c, p);
+        } else {
+            launch_nodes<T, G, 0>(c, p);
+        }
+    } else {
+        launch_rheology<T, G>(c, s, p, law);
+        launch_nodes<T, G, 0>(c, p);
+    }
+    launch_bc<T, G>(c, p, 0, !at.last && chains_sm(c));
 }
 
 // the fused FP32 sweep: new state into the second buffer set, then swap sets
@@ -790,9 +824,9 @@ bool launch_fused(Ctx& c, const KP<float>& p, bool fill) {
 
 // one reference iteration with the fused sweep (FP32)
 template <int G>
-void iterate_fused(Ctx& c, State<float>& s) {
+void iterate_fused(Ctx& c, State<float>& s, IterPos at) {
     KP<float> p = make_kp<float>(c, s);
-    launch_maxloc<float, G>(c, p);
+    if (at.first || !chains_sm(c)) launch_maxloc<float, G>(c, p);
     launch_fused<G, 0>(c, p, false);
     swap_state(s);
     KP<float> q = make_kp<float>(c, s);
@@ -805,31 +839,31 @@ void iterate_fused(Ctx& c, State<float>& s) {
     } else {
         launch_rheology<float, G>(c, s, q);
     }
-    launch_bc<float, G>(c, q, 0);
+    launch_bc<float, G>(c, q, 0, !at.last && chains_sm(c));
 }
 
 template <typename T>
-void iterate_dispatch(Ctx& c, State<T>& s) {
+void iterate_dispatch(Ctx& c, State<T>& s, IterPos at) {
     switch (c.prm.geometry) {
-        case SPH_GEOM_SPHERICAL: iterate_one<T, SPH>(c, s); break;
-        case SPH_GEOM_CYLINDRICAL: iterate_one<T, CYL>(c, s); break;
-        default: iterate_one<T, CART>(c, s); break;
+        case SPH_GEOM_SPHERICAL: iterate_one<T, SPH>(c, s, at); break;
+        case SPH_GEOM_CYLINDRICAL: iterate_one<T, CYL>(c, s, at); break;
+        default: iterate_one<T, CART>(c, s, at); break;
     }
 }
 template <>
-void iterate_dispatch<float>(Ctx& c, State<float>& s) {
+void iterate_dispatch<float>(Ctx& c, State<float>& s, IterPos at) {
     if (c.fused) {
         switch (c.prm.geometry) {
-            case SPH_GEOM_SPHERICAL: iterate_fused<SPH>(c, s); break;
-            case SPH_GEOM_CYLINDRICAL: iterate_fused<CYL>(c, s); break;
-            default: iterate_fused<CART>(c, s); break;
+            case SPH_GEOM_SPHERICAL: iterate_fused<SPH>(c, s, at); break;
+            case SPH_GEOM_CYLINDRICAL: iterate_fused<CYL>(c, s, at); break;
+            default: iterate_fused<CART>(c, s, at); break;
         }
         return;
     }
     switch (c.prm.geometry) {
-        case SPH_GEOM_SPHERICAL: iterate_one<float, SPH>(c, s); break;
-        case SPH_GEOM_CYLINDRICAL: iterate_one<float, CYL>(c, s); break;
-        default: iterate_one<float, CART>(c, s); break;
+        case SPH_GEOM_SPHERICAL: iterate_one<float, SPH>(c, s, at); break;
+        case SPH_GEOM_CYLINDRICAL: iterate_one<float, CYL>(c, s, at); break;
+        default: iterate_one<float, CART>(c, s, at); break;
     }
 }
 
@@ -1005,11 +1039,12 @@ int solve_plain(Ctx& c, State<T>& s, bool is32, const sph_solve_opts& o, sph_sol
     while (it < o.maxiter) {
         ++it;
         const bool check = (it % nout) == 0;
+        const IterPos at{it == 1 || nout == 1 || it % nout == 1, check || it == o.maxiter};
         if (check && ref) {
             int rc = snapshot<T>(c, s);
             if (rc) return rc;
         }
-        iterate_dispatch<T>(c, s);
+        iterate_dispatch<T>(c, s, at);
         if (!check) continue;
         CK(cudaGetLastError());
         if (ref) {
@@ -1257,7 +1292,7 @@ int run_warm_iterations(Ctx& c, int n) {
         CK(cudaStreamSynchronize(c.stream));
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < n; ++i) iterate_dispatch<float>(c, c.s32);  // recorded, not run
+        for (int i = 0; i < n; ++i) iterate_dispatch<float>(c, c.s32, {i == 0, i == n - 1});  // recorded, not run
         cudaError_t e = cudaStreamEndCapture(c.stream, &g);
         if (e != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
         e = cudaGraphInstantiate(&c.warm_graph[slot], g, 0);
@@ -1305,7 +1340,7 @@ int solve_mixed_g(Ctx& c, const sph_solve_opts& o, sph_solve_info* info, int64_t
             ++iters;
             const bool check = (iters % nout) == 0;
             if (check) { rc = snapshot<float>(c, t); if (rc) return rc; }
-            iterate_dispatch<float>(c, t);
+            iterate_dispatch<float>(c, t, {});
             if (!check) continue;
             rc = ref_err<float>(c, t, &werr, false);
             if (rc) return rc;
@@ -2279,8 +2314,8 @@ int sph_step(void* h, int64_t k) {
     if (rc) return rc;
     CK(cudaEventRecord(c->ev0, c->stream));
     for (int64_t i = 0; i < k; ++i) {
-        if (use32) iterate_dispatch<float>(*c, c->s32);
-        else iterate_dispatch<double>(*c, c->s64);
+        if (use32) iterate_dispatch<float>(*c, c->s32, {i == 0, i == k - 1});
+        else iterate_dispatch<double>(*c, c->s64, {i == 0, i == k - 1});
     }
     CK(cudaEventRecord(c->ev1, c->stream));
     CK(cudaGetLastError());
