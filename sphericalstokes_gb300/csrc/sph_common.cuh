@@ -120,8 +120,9 @@ __device__ __forceinline__ T fs_pressure(T t11, T q, T kappa, T v_in, T v_out) {
 // these bits (shuffles, atomicMax) therefore propagates NaN, as Julia's maximum
 // does, instead of dropping it (fmax) or folding it into +inf.
 __device__ __forceinline__ unsigned long long ord_bits(double x) {
-    x = fabs(x);
-    return x != x ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(x);
+    // (on the bits: a comparison of doubles would take an FP64 instruction)
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+    return b > 0x7ff0000000000000ULL ? 0x7ff8000000000000ULL : b;
 }
 __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 

@@ -869,9 +869,14 @@ void iterate_dispatch<float>(Ctx& c, State<float>& s, IterPos at) {
 
 // ---------------------------------------------------------------------------
 // reductions
+// the reduction slots cleared, then the maxima of the listed fields (k_maxabs)
 template <typename T>
-void launch_maxabs(Ctx& c, const T* a, const T* b, int slot) {
-    k_maxabs<T><<<ew_blocks(c.d.vol), 256, 0, c.stream>>>(a, b, c.d.vol, c.red + slot);
+int launch_maxabs(Ctx& c, std::initializer_list<MaxItem<T>> items) {
+    CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
+    MaxList<T> l{};
+    std::copy(items.begin(), items.end(), l.f);
+    launch_pdl(c.use_pdl, k_maxabs<T>, dim3(ew_blocks(c.d.vol), (unsigned)items.size()), dim3(256), 0, c.stream, l, c.d.vol, c.red);
+    return SPH_OK;
 }
 inline double slot_val(Ctx& c, int i) {
     double v;
@@ -887,15 +892,10 @@ int fetch_red(Ctx& c) {
 // relative velocity change of the last iteration (the reference's err)
 template <typename T>
 int ref_err(Ctx& c, State<T>& s, double* err, bool skip_nan_v3) {
-    CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
-    launch_maxabs<T>(c, s.f[F_V1], s.f[F_V1E], 0);
-    launch_maxabs<T>(c, s.f[F_V2], s.f[F_V2E], 1);
-    launch_maxabs<T>(c, s.f[F_V3], s.f[F_V3E], 2);
-    launch_maxabs<T>(c, s.f[F_V1], nullptr, 3);
-    launch_maxabs<T>(c, s.f[F_V2], nullptr, 4);
-    launch_maxabs<T>(c, s.f[F_V3], nullptr, 5);
+    int rc = launch_maxabs<T>(c, {{s.f[F_V1], s.f[F_V1E], 3, 0}, {s.f[F_V2], s.f[F_V2E], 4, 1}, {s.f[F_V3], s.f[F_V3E], 5, 2}});
+    if (rc) return rc;
     CK(cudaGetLastError());
-    int rc = fetch_red(c);
+    rc = fetch_red(c);
     if (rc) return rc;
     double e = 0.0;
     for (int f = 0; f < 3; ++f) {
@@ -911,10 +911,9 @@ int ref_err(Ctx& c, State<T>& s, double* err, bool skip_nan_v3) {
 
 template <typename T>
 int snapshot(Ctx& c, State<T>& s) {
-    const size_t b = sizeof(T) * c.d.vol;
-    CK(cudaMemcpyAsync(s.f[F_V1E], s.f[F_V1], b, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(s.f[F_V2E], s.f[F_V2], b, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(s.f[F_V3E], s.f[F_V3], b, cudaMemcpyDeviceToDevice, c.stream));
+    launch_pdl(c.use_pdl, k_copy3<T>, dim3(ew_blocks(c.d.vol), 3), dim3(256), 0, c.stream, s.f[F_V1E], s.f[F_V2E], s.f[F_V3E], s.f[F_V1], s.f[F_V2],
+               s.f[F_V3], c.d.vol);
+    CK(cudaGetLastError());
     return SPH_OK;
 }
 
@@ -939,16 +938,11 @@ int residual64_g(Ctx& c, double out[7], bool eta_from_law) {
         r.P = s.f[F_PRES];
     }
     launch_nodes<double, G, 2>(c, r);
-    CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
-    launch_maxabs<double>(c, s.f[F_RV1], nullptr, 0);
-    launch_maxabs<double>(c, s.f[F_RV2], nullptr, 1);
-    launch_maxabs<double>(c, s.f[F_RV3], nullptr, 2);
-    launch_maxabs<double>(c, s.f[F_RP], nullptr, 3);
-    launch_maxabs<double>(c, s.f[F_V1], nullptr, 4);
-    launch_maxabs<double>(c, s.f[F_V2], nullptr, 5);
-    launch_maxabs<double>(c, s.f[F_V3], nullptr, 6);
+    int rc = launch_maxabs<double>(c, {{s.f[F_RV1], nullptr, 0}, {s.f[F_RV2], nullptr, 1}, {s.f[F_RV3], nullptr, 2}, {s.f[F_RP], nullptr, 3},
+                                       {s.f[F_V1], nullptr, 4}, {s.f[F_V2], nullptr, 5}, {s.f[F_V3], nullptr, 6}});
+    if (rc) return rc;
     CK(cudaGetLastError());
-    int rc = fetch_red(c);
+    rc = fetch_red(c);
     if (rc) return rc;
     for (int i = 0; i < 4; ++i) out[i] = slot_val(c, i);
     out[4] = std::max(slot_val(c, 4), std::max(slot_val(c, 5), slot_val(c, 6)));
@@ -970,17 +964,14 @@ int residual64(Ctx& c, double out[7]) {
 }
 
 int compute_f_scale(Ctx& c) {
-    CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
-    launch_maxabs<double>(c, c.s64.f[F_RHO], nullptr, 0);
-    int rc = fetch_red(c);
+    int rc = launch_maxabs<double>(c, {{c.s64.f[F_RHO], nullptr, 0}});
+    if (rc || (rc = fetch_red(c))) return rc;
     if (rc) return rc;
     const sph_params& q = c.prm;
     double f = slot_val(c, 0) * std::fabs(q.g);
     if (q.bc == SPH_BC_STRESS) f = std::max(f, std::max(std::fabs(q.sig_bc[1]), std::fabs(q.sig_bc[2])) / q.l1);
     if (q.bc == SPH_BC_FREE_SURFACE) {  // the surface load's force scale, max|q| / l1
-        CK(cudaMemsetAsync(c.red, 0, sizeof(unsigned long long) * kRedSlots, c.stream));
-        launch_maxabs<double>(c, c.s64.f[F_LOAD], nullptr, 0);
-        if ((rc = fetch_red(c))) return rc;
+        if ((rc = launch_maxabs<double>(c, {{c.s64.f[F_LOAD], nullptr, 0}})) || (rc = fetch_red(c))) return rc;
         f = std::max(f, slot_val(c, 0) / q.l1);
     }
     c.f_scale = f > 0.0 ? f : 1.0;
@@ -2242,9 +2233,12 @@ static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf)
     const Adj a = adj_ptrs(c, true);
     const int nout = o.nout > 0 ? o.nout : 100;
     // max|b|
-    CK(cudaMemsetAsync(c->red, 0, sizeof(unsigned long long) * kRedSlots, c->stream));
-    for (int s = 0; s < 4; ++s) launch_maxabs<double>(*c, adj_slot(c, AJ_B1 + s), nullptr, s);
-    int rc = fetch_red(*c);
+    auto max4 = [&](int f) {
+        const int rc = launch_maxabs<double>(*c, {{adj_slot(c, f), nullptr, 0}, {adj_slot(c, f + 1), nullptr, 1}, {adj_slot(c, f + 2), nullptr, 2},
+                                                  {adj_slot(c, f + 3), nullptr, 3}});
+        return rc ? rc : fetch_red(*c);
+    };
+    int rc = max4(AJ_B1);
     if (rc) return rc;
     double bmax = 0.0;
     for (int s = 0; s < 4; ++s) bmax = std::max(bmax, slot_val(*c, s));
@@ -2265,9 +2259,7 @@ static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf)
         if ((rc = adj_apply<G>(c, p, true))) return rc;
         k_adj_residual<<<gu, blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3), adj_slot(c, AJ_BP),
                                                       adj_slot(c, AJ_R1), adj_slot(c, AJ_R2), adj_slot(c, AJ_R3), adj_slot(c, AJ_RP));
-        CK(cudaMemsetAsync(c->red, 0, sizeof(unsigned long long) * kRedSlots, c->stream));
-        for (int s = 0; s < 4; ++s) launch_maxabs<double>(*c, adj_slot(c, AJ_R1 + s), nullptr, s);
-        if ((rc = fetch_red(*c))) return rc;
+        if ((rc = max4(AJ_R1))) return rc;
         double r = 0.0;
         for (int s = 0; s < 4; ++s) r = std::max(r, slot_val(*c, s));
         err = r / bmax;
@@ -2901,8 +2893,9 @@ int sph_check_err_noalloc(int32_t m, const double* const* v, const double* const
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CK(cudaMemsetAsync(slots, 0, sizeof(unsigned long long) * 2 * m, st));  // max-reductions start at 0
     for (int i = 0; i < m; ++i) {
-        k_maxabs<double><<<ew_blocks(count[i]), 256, 0, st>>>(v[i], v_old[i], count[i], slots + i);
-        k_maxabs<double><<<ew_blocks(count[i]), 256, 0, st>>>(v[i], nullptr, count[i], slots + m + i);
+        MaxList<double> l{};
+        l.f[0] = {v[i], v_old[i], m + i, i};
+        k_maxabs<double><<<ew_blocks(count[i]), 256, 0, st>>>(l, count[i], slots);
     }
     CK(cudaGetLastError());
     unsigned long long h[2 * SPH_NOALLOC_MAX_ARRAYS];
