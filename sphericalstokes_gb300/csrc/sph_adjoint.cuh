@@ -21,7 +21,7 @@
 //   k_adj_eta      per cell λᵀ ∂R/∂η (and, for the law, that times dη_t/dε̇)
 //   k_adj_collect, k_adj_law   the law's dependence on V added to the adjoints of the strain rates
 //   k_adj_strain   adjoints of strain rates and div V -> V (all entries)
-// Measured on a GB300, 63^3 sector under the strain-rate law: 125 us per transposed iteration (820 with
+// Measured on a GB300, 63^3 sector under the strain-rate law: 114 us per transposed iteration (820 with
 // scatters by FP64 atomics and coefficients evaluated as stencils of unit vectors), the FP64 units 63 - 78 %
 // busy in the cell and node kernels; the rest is the five BC stages and launches.
 #pragma once
@@ -370,6 +370,8 @@ __global__ void __launch_bounds__(MC_NT) k_adj_law_params(const __grid_constant_
 
 // transpose of one homogeneous BC stage (faces normal to axis D) on the velocity adjoints: each boundary
 // entry's adjoint goes back to the entries its value was computed from, then is cleared
+// Bound by latency: one warp per block and loads before stores, us a stage (63^3, cold caches): x1 faces 16.4 and 4.2 (blocks of
+// 256, each op's load behind the store before), copies 4.4 - 7.9 and 3.6 - 4.0.  An iteration 131 and 114, at 39 x 23 x 31 38 and 29.
 template <int G, int D>
 __global__ void k_bc_adjoint(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, const __grid_constant__ BcStage st) {
     pdl_enter_small();
@@ -378,47 +380,59 @@ __global__ void k_bc_adjoint(const __grid_constant__ KP<double> p, const __grid_
     const int sy = d.sy, sz = d.sz;
     const int step = D == 0 ? 1 : (D == 1 ? sy : sz);
     const int base = D == 0 ? u * sy + v * sz : (D == 1 ? u + v * sz : u + v * sy);
-    for (int o = st.nops - 1; o >= 0; --o) {
-        const int f = st.op[o].field, kind = st.op[o].kind;
-        const int e0 = d.n1 + (f == 0), e1 = d.n2 + (f == 1), e2 = d.n3 + (f == 2);
-        if (u >= (D == 0 ? e1 : e0) || v >= (D == 2 ? e1 : e2)) continue;
-        const int ext = D == 0 ? e0 : (D == 1 ? e1 : e2);
-        double* A = f == 0 ? a.aV1 : (f == 1 ? a.aV2 : a.aV3);
-        for (int side = 1; side >= 0; --side) {
-            const int b = side == 0 ? 0 : ext - 1, in = side == 0 ? 1 : ext - 2;
-            const int cb = base + b * step, ci = base + in * step;
-            const double g = A[cb];
-            A[cb] = 0.0;
-            if (g == 0.0) continue;
-            switch (kind) {
-                // (one face point per source: no other thread of the stage adds to it)
-                case BC_NEG: A[ci] -= g; break;
-                case BC_COPY: A[ci] += g; break;
-                case BC_LIN2M: A[ci] -= g; break;  // homogeneous form: -A[in]
-                case BC_ZERO:
-                case BC_LIN: break;                              // constants: no dependence
-                default: {  // BC_STRESS on the x2 / x3 faces (div_ghost, D = 1, 2): linear in V1 at the cell's two x1
-                            // faces, the other tangential component and the normal one inside
-                    if (D == 0) break;
-                    const int cell = side == 0 ? 0 : ext - 2, cc = base + cell * step;
-                    const int i = u, j = D == 1 ? cell : v;
-                    const CellMetric<double> m = cell_metric<double, G>(p, i, j);
-                    const double sgn = side == 0 ? -1.0 : 1.0, hc1 = 0.5 * m.c1, hc2 = 0.5 * m.c2;
-                    const double s = -g / (D == 1 ? fma(sgn, m.a2, hc2) : sgn * m.a3);
-                    atomicAdd(a.aV1 + cc, s * (hc1 - p.d1));
-                    atomicAdd(a.aV1 + cc + 1, s * (hc1 + p.d1));
-                    if (D == 1) {
-                        atomicAdd(a.aV3 + cc, -s * m.a3);
-                        atomicAdd(a.aV3 + cc + sz, s * m.a3);
-                        atomicAdd(A + ci, s * (hc2 - sgn * m.a2));
-                    } else {
-                        atomicAdd(a.aV2 + cc, s * (hc2 - m.a2));
-                        atomicAdd(a.aV2 + cc + sy, s * (hc2 + m.a2));
-                        atomicAdd(A + ci, -s * sgn * m.a3);
-                    }
-                    break;
-                }
+    auto field = [&](int f) { return f == 0 ? a.aV1 : (f == 1 ? a.aV2 : a.aV3); };
+    auto ext = [&](int f, int ax) { return (ax == 0 ? d.n1 : (ax == 1 ? d.n2 : d.n3)) + (f == ax); };
+    auto on = [&](int f) { return u < ext(f, D == 0 ? 1 : 0) && v < ext(f, D == 2 ? 1 : 2); };
+    if (st.op[0].kind != BC_STRESS) {
+        // each face point has a source of its own, and the ops are on different fields: all loads, then all stores
+        double g[3][2], t[3][2];
+#pragma unroll
+        for (int o = 0; o < 3; ++o)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int f = st.op[o].field, e = ext(f, D);
+                if (o >= st.nops || !on(f) || (st.op[o].side >= 0 && st.op[o].side != side)) continue;
+                g[o][side] = field(f)[base + (side == 0 ? 0 : e - 1) * step];
+                t[o][side] = field(f)[base + (side == 0 ? 1 : e - 2) * step];
             }
+#pragma unroll
+        for (int o = 0; o < 3; ++o)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int f = st.op[o].field, e = ext(f, D), kind = st.op[o].kind;
+                if (o >= st.nops || !on(f) || (st.op[o].side >= 0 && st.op[o].side != side)) continue;
+                field(f)[base + (side == 0 ? 0 : e - 1) * step] = 0.0;
+                const double x = t[o][side], y = g[o][side];
+                if (kind == BC_COPY) field(f)[base + (side == 0 ? 1 : e - 2) * step] = x + y;
+                else if (kind == BC_NEG || kind == BC_LIN2M) field(f)[base + (side == 0 ? 1 : e - 2) * step] = x - y;  // (homogeneous form)
+            }
+        return;
+    }
+    // BC_STRESS on the x2 / x3 faces (div_ghost, D = 1, 2): linear in V1 at the cell's two x1 faces, the other
+    // tangential component and the normal one inside.  Alone in its stage.
+    if (D == 0 || !on(D)) return;
+    double* A = field(D);
+#pragma unroll
+    for (int side = 1; side >= 0; --side) {
+        const int e = ext(D, D), cb = base + (side == 0 ? 0 : e - 1) * step, ci = base + (side == 0 ? 1 : e - 2) * step;
+        const double g = A[cb];
+        A[cb] = 0.0;
+        if (g == 0.0) continue;
+        const int cell = side == 0 ? 0 : e - 2, cc = base + cell * step;
+        const int i = u, j = D == 1 ? cell : v;
+        const CellMetric<double> m = cell_metric<double, G>(p, i, j);
+        const double sgn = side == 0 ? -1.0 : 1.0, hc1 = 0.5 * m.c1, hc2 = 0.5 * m.c2;
+        const double s = -g / (D == 1 ? fma(sgn, m.a2, hc2) : sgn * m.a3);
+        atomicAdd(a.aV1 + cc, s * (hc1 - p.d1));
+        atomicAdd(a.aV1 + cc + 1, s * (hc1 + p.d1));
+        if (D == 1) {
+            atomicAdd(a.aV3 + cc, -s * m.a3);
+            atomicAdd(a.aV3 + cc + sz, s * m.a3);
+            atomicAdd(A + ci, s * (hc2 - sgn * m.a2));
+        } else {
+            atomicAdd(a.aV2 + cc, s * (hc2 - m.a2));
+            atomicAdd(a.aV2 + cc + sy, s * (hc2 + m.a2));
+            atomicAdd(A + ci, -s * sgn * m.a3);
         }
     }
 }

@@ -2174,9 +2174,9 @@ static void adj_bc(Ctx* c, const KP<double>& p, const Adj& a) {
     for (auto st = c->bc.rbegin(); st != c->bc.rend(); ++st) {
         int eu = st->dim == 0 ? c->d.n2 + 1 : c->d.n1 + 1;
         int ev = st->dim == 2 ? c->d.n2 + 1 : c->d.n3 + 1;
-        dim3 g((eu + 31) / 32, (ev + 7) / 8, 1);
+        const int rows = (eu + 31) / 32 * (long long)ev <= 4LL * c->sms ? 1 : 8;  // (few blocks else)
         auto k = st->dim == 0 ? k_bc_adjoint<G, 0> : (st->dim == 1 ? k_bc_adjoint<G, 1> : k_bc_adjoint<G, 2>);
-        launch_pdl(c->use_pdl, k, g, blk2d(), 0, c->stream, hp, a, *st);
+        launch_pdl(c->use_pdl, k, dim3((eu + 31) / 32, (ev + rows - 1) / rows), dim3(32, rows), 0, c->stream, hp, a, *st);
     }
 }
 
