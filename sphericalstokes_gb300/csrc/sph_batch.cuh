@@ -34,9 +34,12 @@ struct BatchSweep {
 // time, 29 ms now).
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __restrict__ b, const int4* __restrict__ items,
                                                           const int* __restrict__ active, const int* __restrict__ kchunk, int a) {
-    pdl_wait();  // as k_sweep: no early release of the next grid
+    // (items, flags and entries change between launches of the whole round only)
     const int4 it = items[blockIdx.x];
-    if (!active[it.x]) return;  // whole block: no barrier is reached
+    if (!active[it.x]) {  // whole block: no barrier is reached
+        pdl_wait();
+        return;
+    }
     // the solve's scalars and pointers in shared memory: the march reads them plane by plane
     __shared__ KP<float> p;
     __shared__ SweepOut<float> o;

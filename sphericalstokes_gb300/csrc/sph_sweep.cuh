@@ -332,6 +332,7 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
         ph ^= 1u << bit;
     };
 
+    pdl_wait();  // (nothing before this reads what the preceding sweep writes)
     if (issuer) {
         mbar_expect_tx(&S.bar_0, 4 * 5 * SI_N);
         issue_in(k0, &S.bar_0);
@@ -695,6 +696,11 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
         step(std::integral_constant<int, 0>{}, K, ca, cb);
         if (K + 1 >= kB) break;
         step(std::integral_constant<int, 1>{}, K + 1, cb, ca);
+        // The next grid's blocks may come once every block is within two planes of its end: their set-up then fills the
+        // tail of this grid.  us per sweep, released at the end (implicitly) and so: 63^3 12.9 and 11.8, 131 x 117 x 101
+        // 45.2 and 44.6, 255^3 305.2 and 304.6, sector 28 x 29 x 158 10.6 and 9.3; at the start of the block 28 x 75 x 72 became
+        // 11.6 (10.6; so 10.1), as early blocks leave the SMs unevenly filled.
+        if (K + 4 >= kB) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     }
     // Without a time-out every issued copy has been waited for, so none is in flight when the
     // block exits.  After a time-out copies issued before it may still be landing in this
@@ -706,7 +712,6 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
 template <int G, int MODE>
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep(const __grid_constant__ KP<float> p, const __grid_constant__ SweepOut<float> o, int kchunk,
                                                     const __grid_constant__ SweepMaps maps, int* __restrict__ err) {
-    pdl_wait();  // no early release of the next grid: its blocks would take SM slots in this grid's tail
     sweep_body<G, MODE>(p, o, kchunk, maps.m, err, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
