@@ -65,6 +65,9 @@ struct KP {
     T g;
     T tau_C, n_exp, relax, edot_bg;
     T law_i2, law_ex;                  // FP64 laws: 1/ε̇_bg², (n-1)/(2n) or 1/τ_C², (n-1)/2
+    T law_i1, law_rho;                 // 1/τ_C; (q+1)/(q-1)
+    float law_e, law_el;               // law_ex as head and tail
+    int law_p, law_q;                  // law_ex = law_p / law_q where that is a fast form (power_form), law_q = 0: is not
     T sig2, sig3;                      // prescribed total normal stress on x2 / x3 faces
     int traction;                      // 1: boundary cells on x2/x3 faces take P = τ_nn - σ_bc
     int fs;                            // 1: top cells (i = n1-1) take the free-surface pressure (fs_pressure)

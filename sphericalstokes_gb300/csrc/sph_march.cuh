@@ -263,7 +263,10 @@ __device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by
         }
         const double ei = p.eta_ini[c];
         double et = ei;
-        if (!(p.phase && p.phase[c])) et = fast_div(ei + ei, 1.0 + fast_pow(tab, x * p.law_i2, p.law_ex));
+        if (!(p.phase && p.phase[c])) {
+            const double w = x * p.law_i2;
+            et = fast_div(ei + ei, 1.0 + (p.law_q && root_range(w) ? root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el) : fast_pow(tab, w, p.law_ex)));
+        }
         if (RELAXED) {
             const double eo = p.eta[c];
             // exact for the half-way mean; else η (η_t/η)^relax
@@ -317,15 +320,34 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
             t2 = t2c;
             p.tII[c] = tii = tiic;
         }
-        const double cx = (p.phase && p.phase[c]) ? 0.0 : p.law_ex;
+        const bool lin = p.phase && p.phase[c];
+        const double cx = lin ? 0.0 : p.law_ex;
         const double ei = p.eta_ini[c], x = t2 * p.law_i2;
+        // integer n: (τII / τ_C)^(n-1) by multiplication
+        const double w = p.law_q ? small_pow(tii * p.law_i1, x, lin ? 0 : p.law_p) : 0.0;
         if (!RELAX) {
-            p.eta[c] = fast_div(ei + ei, 1.0 + fast_pow(tab, x, cx));
+            p.eta[c] = fast_div(ei + ei, 1.0 + (p.law_q ? w : fast_pow(tab, x, cx)));
         } else {
             const double po = p.eta_pl[c];
             double pl;
             bool done = false;
-            if (normal_pos(x) && normal_pos(ei) && normal_pos(po)) {
+            if (p.law_q) {  // η_PL' = po (ei / (po w))^relax
+                const double den = po * w;
+                // (η_PL itself, ei / w, has to be a normal number too: where it is not, it is 0 or infinite, as in power_law!)
+                const int ex = (__double2hiint(ei) >> 20) - (__double2hiint(w) >> 20);
+                if (normal_pos(w) && normal_pos(ei) && normal_pos(po) && normal_pos(den) && ex > -1000 && ex < 1000) {
+                    const double r = fast_div(ei, den);
+                    if (normal_pos(r)) {
+                        double h, t;
+                        log2_parts(tab, r, h, t);
+                        const double y = p.relax * h;
+                        if ((__double2hiint(y) & 0x7fffffff) < 0x408f4000) {  // |y| < 1000
+                            pl = po * exp2_parts(tab, y, fma(p.relax, t, fma(p.relax, h, -y)));
+                            done = true;
+                        }
+                    }
+                }
+            } else if (normal_pos(x) && normal_pos(ei) && normal_pos(po)) {
                 // η_PL' = po 2^(relax (log2 ei - log2 po - cx log2 x)), the exponent as a head and a tail
                 double hx, tx, hi, ti, ho, to;
                 log2_parts(tab, x, hx, tx);
@@ -334,7 +356,8 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
                 const double L = hi - ho, q = cx * hx, s = L - q;
                 const double low = ((ti - to) - fma(cx, tx, fma(cx, hx, -q))) + ((L - s) - q);
                 const double y = p.relax * s;
-                if ((__double2hiint(y) & 0x7fffffff) < 0x408f4000) {  // |y| < 1000
+                // |y| < 1000, and η_PL before the relaxation a normal number
+                if ((__double2hiint(y) & 0x7fffffff) < 0x408f4000 && (__double2hiint(hi - q) & 0x7fffffff) < 0x408f4000) {
                     pl = po * exp2_parts(tab, y, fma(p.relax, low, fma(p.relax, s, -y)));
                     done = true;
                 }
