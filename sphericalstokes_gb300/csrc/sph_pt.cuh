@@ -103,8 +103,10 @@ __device__ __forceinline__ T tau_II(const KP<T>& p, int s) {
 
 // compute_TII! + copy_BC!(τII) + power_law! (RELAX: log-space relaxation of
 // η_PL, CylindricalStokes_diapir.jl:185-192).  phase==1 cells are linear.
+// Its launch overlaps the end of the sweep before it: FP32 iteration at 95 x 79 x 67 30.9 us without, 29.2 with.
 template <typename T, bool RELAX>
 __global__ void k_rheo_tau(KP<T> p, int faces_only, T n_exp) {
+    pdl_enter_small();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     const Dims& d = p.d;
     if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;
@@ -135,6 +137,7 @@ __global__ void k_rheo_tau(KP<T> p, int faces_only, T n_exp) {
 // η_PL = η_ini (edot_II/edot_bg)^((1-n)/n); RELAXED: η_out = η^(1-relax) η_t^relax.
 template <typename T, bool RELAXED>
 __global__ void k_edot_law(KP<T> p) {
+    pdl_enter_small();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     const Dims& d = p.d;
     if (i >= d.n1 || j >= d.n2 || k >= d.n3) return;

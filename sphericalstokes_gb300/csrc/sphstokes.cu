@@ -585,7 +585,7 @@ void launch_edot(Ctx& c, const KP<T>& p) {
         const int k = march_chunk(cols, c.d.n3, c.sms, 0.1, 3.0);
         launch_pdl(c.use_pdl, k_edot<RELAXED>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, k);
     } else {
-        k_edot_law<T, RELAXED><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p);
+        launch_pdl(c.use_pdl, k_edot_law<T, RELAXED>, grid_cells(c.d), blk2d(), 0, c.stream, p);
     }
 }
 template <typename T, bool RELAX>
@@ -595,7 +595,7 @@ void launch_tau_law(Ctx& c, const KP<T>& p, int faces_only) {
         const int k = march_chunk(cols, c.d.n3, c.sms, 0.1, 3.0);
         launch_pdl(c.use_pdl, k_rheo<RELAX>, dim3((unsigned)((cols + MC_NT - 1) / MC_NT), (c.d.n3 + k - 1) / k), dim3(MC_NT), 0, c.stream, p, faces_only, k);
     } else {
-        k_rheo_tau<T, RELAX><<<grid_cells(c.d), blk2d(), 0, c.stream>>>(p, faces_only, T(c.cur_n));
+        launch_pdl(c.use_pdl, k_rheo_tau<T, RELAX>, grid_cells(c.d), blk2d(), 0, c.stream, p, faces_only, T(c.cur_n));
     }
 }
 
