@@ -228,8 +228,8 @@ int sph_update_params(void* ctx, const sph_params* params);
  * outcome of each solve is infos[i].status.
  *  - Lockstep batch, when every solve is SPH_PREC_MIXED on SPH_CRIT_RESIDUAL without a warm
  *    start (warm_tol 0), with the TMA sweep and one even nout for all: the solves advance
- *    together, and one correction sweep of all of them is one launch per geometry over a
- *    work list of (solve, tile, x3 chunk) blocks plus one launch per BC stage, a round of
+ *    together, and one correction sweep of all of them is one launch over a work list
+ *    of (solve, tile, x3 chunk) blocks, its chunk length picked for the whole batch, a round of
  *    nout sweeps replayed from one CUDA graph; each solve's FP64 outer steps, inner tests
  *    and budget are its own, and its results equal those of sph_solve alone.  infos[i].seconds
  *    and device_ms are those of the whole batch; `threads` is not used.
@@ -240,7 +240,7 @@ int sph_batch_solve(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sp
 /* Autotuner of the fused FP32 sweep (no counterpart in the reference): times `sweeps`
  * correction sweeps for each candidate x3 chunk length (planes per block) and keeps
  * the fastest for this context and for every later context of the same geometry and
- * grid size.  MIXED with SPH_KERNELS_AUTO only; the FP64 state is not changed. */
+ * grid size (solved alone; a lockstep batch picks one for all its grids).  MIXED with SPH_KERNELS_AUTO only; the FP64 state is not changed. */
 int sph_autotune(void* ctx, int32_t sweeps, int32_t* best_chunk, double* best_ms_per_sweep);
 
 /* exactly k reference PT iterations (equal3! ... BC_φ!, SphericalStokes_diapir.jl:413-425) */

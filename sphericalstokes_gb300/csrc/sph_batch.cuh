@@ -30,8 +30,8 @@ struct BatchSweep {
 // one correction sweep of every active solve (items: x = solve, y, z, w = tile x, y, chunk; kchunk: planes per
 // block of each solve).  All geometries in one launch: a block runs the body of its own, and the
 // blocks of a small batch fill the SMs together (12 grids of 31 .. 47 cells a side, 600 sweeps with the
-// FP64 steps and copies: 50.8 ms with a launch per geometry and each solve's own chunk, 39.2 ms so with the sweep of that
-// time, 29 ms now).
+// FP64 steps and copies: 50.8 ms with a launch per geometry and each solve's own chunk, 39.2 ms so, 26.6 ms with
+// the sweep of now and blocks of one geometry on an SM).
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __restrict__ b, const int4* __restrict__ items,
                                                           const int* __restrict__ active, const int* __restrict__ kchunk, int a) {
     // (items, flags and entries change between launches of the whole round only)

@@ -125,6 +125,7 @@ struct Ctx {
     bool use_pdl = true;  // sweep and BC kernels launched with a programmatic dependency (pdl_enter)
     bool fused = true;   // FP32 sweeps use the fused kernel
     int fused_chunk = 0; // planes per block of the fused sweep (0: chosen by fused_chunk())
+    bool chunk_fixed = false;  // by SPH_FUSED_CHUNK: in batches too
     int sms = 152;
     int fused_slots = 0; // resident blocks of the fused TMA sweep on the device (SMs x blocks per SM)
     double* adj = nullptr;  // adjoint arrays (AJ_COUNT slots of the box), allocated on first use
@@ -1608,7 +1609,8 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
     for (BatchSolve& b : bs) { int rc = sync64(*b.c); if (rc) return rc; }
 
     // work lists: blocks of the member solves' fused sweeps and inner tests.  The chunk of planes per
-    // block comes from all members' blocks together, unless a solve has its own (sph_autotune).
+    // block comes from all members' blocks together (that of sph_autotune is for a grid alone: 1978 us per sweep
+    // of 256 solves with it, 519 so).
     std::vector<BatchSweep> host((size_t)n);
     std::vector<int4> items;
     std::vector<int> kchunk((size_t)n, 1);
@@ -1624,14 +1626,30 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             tiles.push_back({sweep_tiles(bs[i].c->d), bs[i].c->d.n3});
         }
         members = mem.size();
+        // By geometry: the three bodies together do not fit the instruction caches, and an SM whose two blocks run
+        // different ones waits for instructions (8.9 of 17 cycles per instruction).  us per sweep in the caller's order and
+        // so: 256 solves of 31 .. 47 cells a side 877 and 518, twelve 31.4 and 28.9, twelve of 47 .. 63 105 and 85.
+        std::stable_sort(mem.begin(), mem.end(), [&](int x, int y) { return bs[x].c->prm.geometry < bs[y].c->prm.geometry; });
         const int common = chunk_rule(tiles, bs[0].c->sms);
         for (int i : mem) {
             Ctx& c = *bs[i].c;
-            kchunk[i] = c.fused_chunk > 0 ? c.fused_chunk : common;
+            const int parts = (c.d.n3 + common - 1) / common;  // equal ones: the common length leaves a short last chunk
+            kchunk[i] = c.chunk_fixed ? c.fused_chunk : (c.d.n3 + parts - 1) / parts;
             const dim3 gr = sweep_grid(c.d, kchunk[i]);
             for (unsigned z = 0; z < gr.z; ++z) for (unsigned y = 0; y < gr.y; ++y) for (unsigned x = 0; x < gr.x; ++x) items.push_back(make_int4(i, (int)x, (int)y, (int)z));
         }
         fz_n = nm_off = items.size();
+        // The first blocks go to one SM each, the next to the same SMs again: neighbours in the list share an SM.
+        const size_t sms = bs[0].c->sms;
+        if (fz_n > sms) {
+            const size_t two = std::min(fz_n - sms, sms);  // SMs with a second block
+            std::vector<int4> head(sms + two);
+            for (size_t b = 0; b < sms; ++b) {
+                head[b] = items[b < two ? 2 * b : b + two];
+                if (b < two) head[sms + b] = items[2 * b + 1];
+            }
+            std::copy(head.begin(), head.end(), items.begin());
+        }
         for (int i : mem) {
             const dim3 gv = grid_vel(bs[i].c->d);
             for (unsigned z = 0; z < gv.z; ++z) for (unsigned y = 0; y < gv.y; ++y) for (unsigned x = 0; x < gv.x; ++x)
@@ -1870,7 +1888,7 @@ int sph_create(const sph_params* prm, void** out) {
         auto it = g_tuned_chunk.find(std::make_tuple(q.geometry, q.n1, q.n2, q.n3));
         if (it != g_tuned_chunk.end()) c->fused_chunk = it->second;
     }
-    if (const char* e = std::getenv("SPH_FUSED_CHUNK")) c->fused_chunk = std::atoi(e);
+    if (const char* e = std::getenv("SPH_FUSED_CHUNK")) { c->fused_chunk = std::atoi(e); c->chunk_fixed = c->fused_chunk > 0; }
     Dims& d = c->d;
     d.n1 = q.n1; d.n2 = q.n2; d.n3 = q.n3;
     d.px = ((q.n1 + 1 + 31) / 32) * 32; d.py = q.n2 + 1; d.pz = q.n3 + 1;
