@@ -437,7 +437,7 @@ __global__ void k_bc_adjoint(const __grid_constant__ KP<double> p, const __grid_
     }
 }
 
-// pseudo-steps of the current viscosity (k_stress's DT_R) for the adjoint iteration
+// pseudo-steps of the current viscosity (k_cells' DT_R) for the adjoint iteration
 __global__ void __launch_bounds__(256) k_pt_dtr(KP<double> p) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     const Dims& d = p.d;

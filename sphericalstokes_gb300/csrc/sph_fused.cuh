@@ -17,7 +17,7 @@
 // Every state field is read once and written once per sweep (halo re-reads
 // hit L2); the old and new states are different buffers (ping-pong) and the
 // boundary-condition stages run afterwards on the new state.  The arithmetic is the
-// shared core of sph_core.cuh: results equal those of k_stress + k_velocity.
+// shared core of sph_core.cuh: results equal those of k_cells + k_nodes up to rounding.
 //
 // MODE 0: reference iteration (ρg body force).  MODE 1: correction problem of
 // the mixed-precision solve (right-hand sides rP, rV; η and ηSM frozen).
