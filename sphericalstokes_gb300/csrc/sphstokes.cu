@@ -701,7 +701,7 @@ std::map<std::tuple<int, int, int, int>, int> g_tuned_chunk;
 // 6.4 / 7.0 / 8.5 / 10.0 / 17 / 31, 63^3 15.8 / 13.5 / 12.7 / 12.3 / 18 / 32,
 // 131 x 117 x 101 77 / 60 / 53 / 50 / 45.2 / 44.3, 255^3 (8 / 16 / 24) 322 / 305 / 304,
 // 511 x 255 x 255 630 / 608 / 596: the rule's picks (1, 3, 8, 16, 16) are within 4 % of the
-// best (32 planes: 298 and 620).  sph_autotune measures instead.
+// best (32 planes: 298 and 620).  (Before a sweep released the next grid early, which takes 0.1 to 1.1 us off each.)  sph_autotune measures instead.
 // tiles: (tiles in x1 and x2, planes) of each grid of the launch
 int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
     int best = 1, planes = 0;
