@@ -691,17 +691,9 @@ dim3 sweep_grid(const Dims& d, int chunk) { return dim3((d.n1 + SWX - 1) / SWX, 
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, int> g_tuned_chunk;
 
-// x3 chunk length of the fused sweep.  Each block marches over one chunk of
-// planes and pays for more planes than it owns (the halo plane below the chunk and
-// the pipeline fill), while the hardware scheduler balances the SMs only to within
-// one block at the end of the launch.  The time model (k + 2) * max(2.15, 1.1 n + 0.5), n =
-// blocks on the fullest SM (two are resident, and two together are hardly slower than one),
-// picks the chunk among 1..24 planes.
-// Measured on a GB300 (us per sweep, chunks of 1 / 2 / 3 / 4 / 8 / 16 planes): 47 x 31 x 39
-// 6.4 / 7.0 / 8.5 / 10.0 / 17 / 31, 63^3 15.8 / 13.5 / 12.7 / 12.3 / 18 / 32,
-// 131 x 117 x 101 77 / 60 / 53 / 50 / 45.2 / 44.3, 255^3 (8 / 16 / 24) 322 / 305 / 304,
-// 511 x 255 x 255 630 / 608 / 596: the rule's picks (1, 3, 8, 16, 16) are within 4 % of the
-// best (32 planes: 298 and 620).  (Before a sweep released the next grid early, which takes 0.1 to 1.1 us off each.)  sph_autotune measures instead.
+// x3 chunk length of a batch's sweeps: the time model (k + 2) * max(2.15, 1.1 n + 0.5), n = blocks on the fullest SM
+// (two are resident, and two together are hardly slower than one), over 1..24 planes.  us per sweep of 256 grids of
+// 31 .. 47 cells a side, chunks of 8 / 16 (its pick) / 24 planes: 580 / 515 / 530; of 64: 221 / 201 / 207.
 // tiles: (tiles in x1 and x2, planes) of each grid of the launch
 int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
     int best = 1, planes = 0;
@@ -717,13 +709,45 @@ int chunk_rule(const std::vector<std::pair<long long, int>>& tiles, int sms) {
     }
     return best;
 }
+
+// x3 chunk length of the sweep of one grid: the end of its last block, in planes.  A block takes its planes and one more
+// (the halo plane below), two blocks are resident on an SM, and the blocks start in order of x3, so that the short
+// last chunks of a column (the rest of n3 / k) come last, on the slots that the others leave free.  A last wave on
+// half the SMs' slots or fewer runs an eighth faster.  Chunks above 24 planes are not considered: 32 are better at
+// 255^3 (298 us) but worse at 511 x 255 x 255 (620).
+// Measured on a GB300, us per sweep with the rule above and with this one: 38 x 172 x 248 77.7 and 62.0, 200 x 16 x 200
+// 34.4 and 28.8, 127 x 32 x 244 35.2 and 28.9, 96 x 85 x 180 39.6 and 32.2, 127^3 58.0 and 50.1, 221 x 116 x 80 53.7 and 45.6,
+// 131 x 117 x 101 44.5 and 44.1; the same length, or the same time, at 47 x 31 x 39, 63^3, 255^3 and 511 x 255 x 255.
+// Of 15 lengths tried at ten sizes its pick is the best or within 1 %.
+// sph_autotune measures instead.
+int grid_chunk(long long tiles, int planes, int sms) {
+    const long long slots = 2LL * sms;
+    int best = 1;
+    double best_t = 1e300;
+    for (int k = 1; k <= 24 && k <= planes; k += k < 16 ? 1 : 4) {
+        const long long full = tiles * (planes / k), q = full / slots, r = full % slots;
+        const int rem = planes % k, u = k + 1;
+        double t = (double)(q + (r > 0)) * u;
+        if (rem) {
+            const long long fit = (slots - r) * (u / (rem + 1));  // short blocks that end before the last full ones
+            if (r == 0 || tiles > fit) {
+                const long long late = r == 0 ? tiles : tiles - fit;
+                t += (double)((late + slots - 1) / slots) * (rem + 1);
+            }
+        } else if (r > 0 && r <= sms) {
+            t -= 0.125 * u;
+        }
+        if (t < best_t) { best_t = t; best = k; }
+    }
+    return best;
+}
 long long sweep_tiles(const Dims& d) {
     const dim3 t = sweep_grid(d, d.n3);
     return (long long)t.x * t.y;
 }
 int fused_chunk(const Ctx& c) {
     if (c.fused_chunk > 0) return c.fused_chunk;
-    return chunk_rule({{sweep_tiles(c.d), c.d.n3}}, c.sms);
+    return grid_chunk(sweep_tiles(c.d), c.d.n3, c.sms);
 }
 
 // ---------------------------------------------------------------------------
