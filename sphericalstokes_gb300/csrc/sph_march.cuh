@@ -265,7 +265,11 @@ __device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by
         double et = ei;
         if (!(p.phase && p.phase[c])) {
             const double w = x * p.law_i2;
-            et = fast_div(ei + ei, 1.0 + (p.law_q && root_range(w) ? root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el) : fast_pow(tab, w, p.law_ex)));
+            double f;
+            if (p.law_q && root_range(w)) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
+            else if (normal_pos(w)) f = fast_pow(tab, w, p.law_ex);
+            else f = pow(sqrt(x) / p.edot_bg, 2.0 * p.law_ex);  // (the square of the ratio leaves the range first)
+            et = fast_div(ei + ei, 1.0 + f);
         }
         if (RELAXED) {
             const double eo = p.eta[c];
@@ -326,7 +330,9 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
         // integer n: (τII / τ_C)^(n-1) by multiplication
         const double w = p.law_q ? small_pow(tii * p.law_i1, x, lin ? 0 : p.law_p) : 0.0;
         if (!RELAX) {
-            p.eta[c] = fast_div(ei + ei, 1.0 + (p.law_q ? w : fast_pow(tab, x, cx)));
+            double f = w;
+            if (!p.law_q) f = normal_pos(x) ? fast_pow(tab, x, cx) : pow(tii / p.tau_C, 2.0 * cx);  // (as in edot_body)
+            p.eta[c] = fast_div(ei + ei, 1.0 + f);
         } else {
             const double po = p.eta_pl[c];
             double pl;
