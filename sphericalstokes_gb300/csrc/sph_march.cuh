@@ -272,9 +272,13 @@ __device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by
             et = fast_div(ei + ei, 1.0 + f);
         }
         if (RELAXED) {
+            // the half-way mean as a root, else η (η_t/η)^relax; by logarithms where the product or the quotient is no
+            // normal number (a cell without viscosity keeps none)
             const double eo = p.eta[c];
-            // exact for the half-way mean; else η (η_t/η)^relax
-            et = p.relax == 0.5 ? fast_sqrt(eo * et) : eo * fast_pow(tab, fast_div(et, eo), p.relax);
+            const bool half = p.relax == 0.5;
+            const double r = half ? eo * et : fast_div(et, eo);
+            if (normal_pos(r)) et = half ? fast_sqrt(r) : eo * fast_pow(tab, r, p.relax);
+            else et = exp((1.0 - p.relax) * log(eo) + p.relax * log(et));
         }
         p.eta_out[c] = et;
     }

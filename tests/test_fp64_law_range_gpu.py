@@ -1,11 +1,13 @@
 """The FP64 viscosity laws at the ends of the double range: a state at rest, strain rates and stresses whose
-squared ratio to the law's scale leaves the range.
+squared ratio to the law's scale leaves the range, cells without viscosity, an old and a target
+viscosity whose product or quotient leaves it.
 
 The strain-rate invariant is computed here from the velocities (Cartesian grid), in extended precision, and so
 are the laws; every scale is compared, none is skipped.
 
 Tolerance: 1e-12.  The invariant is a sum of squares of some ten roundings each (differences of
-neighbouring values are exact to half a unit), 1e-14 in all.
+neighbouring values are exact to half a unit), 1e-14 in all.  The mean by logarithms, exp of values y up to
+745, loses |y| 2^-53 in each of two logarithms and in their sum: 3 * 745 * 1.1e-16 = 2.5e-13.
 """
 import numpy as np
 import pytest
@@ -17,6 +19,8 @@ pytestmark = pytest.mark.gpu
 X = np.longdouble
 N = (7, 6, 9)
 VSCALES = (0.0, 1e-140, 1e-60, 1e-9, 1.0, 1e9, 1e60, 1e140)
+# scales of the old viscosity and of the prefactor
+PAIRS = ((1.0, 1.0), (1e-160, 1e160), (1e160, 1e-160), (1e300, 1e-300), (1e-300, 1e300), (1e290, 1e290), (1e-290, 1e-290), (1e-150, 1.0))
 
 
 def clamped(a):
@@ -83,6 +87,21 @@ def test_strain_rates_over_the_range(n_exp, relax, edot_bg):
         ratio = invariant(p, V) / X(edot_bg)
         t = X(2) * ini.astype(X) / (X(1) + ratio ** ((X(n_exp) - 1) / X(n_exp)))
         check(got, eta.astype(X) ** (X(1) - X(relax)) * t ** X(relax))
+
+
+@pytest.mark.parametrize("relax", [0.3, 0.5, 0.9])
+@pytest.mark.parametrize("n_exp", [1.7, 3.0])
+@pytest.mark.parametrize("pair", PAIRS)
+def test_old_and_target_viscosity_far_apart(n_exp, relax, pair):
+    rng = np.random.default_rng(2)
+    p = edot_params(n_exp, relax, 0.25)
+    V = velocities(rng, 1.0)
+    eta, ini = (s * np.exp(rng.standard_normal(N)) for s in pair)
+    eta[2:4, 1, :] = 0.0  # cells without viscosity keep none
+    got = run_edot(p, V, eta, ini)
+    t = X(2) * ini.astype(X) / (X(1) + (invariant(p, V) / X(0.25)) ** ((X(n_exp) - 1) / X(n_exp)))
+    check(got, eta.astype(X) ** (X(1) - X(relax)) * t ** X(relax))
+    assert np.all(got[2:4, 1, :] == 0.0)
 
 
 @pytest.mark.parametrize("n_exp", [1.5, 2.0, 2.5, 3.0])
