@@ -9,22 +9,22 @@
 
 namespace sph {
 
-// a / b in five FP64 operations: PTX's approximate reciprocal r (relative error below 2^-20), the
-// quotient a r, and two corrections by its residual, q += r (a - b q), each of which multiplies the error
-// by that of r: to 2^-40, then below 2^-60 (Newton's iteration for the quotient, Markstein's last step).  At
-// most one unit in the last place from the IEEE quotient.  near_div: b and the quotient well inside the range
-// of normal numbers (sums of viscosities; a zero or infinite b gives NaN).  fast_div: any operands, those out
-// of the middle of the range (integer tests, no FP64 issue) by the IEEE division.
-__device__ __forceinline__ double near_div(double a, double b) {
+// a / b in five FP64 operations: PTX's approximate reciprocal r (relative error e near 2^-20), one Newton step (e^2),
+// the quotient a r and one step by its residual, q += r (a - b q) (Markstein, IBM J. Res. Dev. 34, 1990), which leaves e^4
+// before the last rounding: the IEEE quotient but for about one pair of operands in 2^24.  (Two residual steps with the
+// reciprocal as it comes take as many operations and leave e^3: 297 of 2^20 quotients were one unit off.)  For b and the
+// quotient inside the range of normal numbers.
+__device__ __forceinline__ double mid_div(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(fma(-b, r, 1.0), r, r);
     const double q = a * r;
-    const double q1 = fma(fma(-b, q, a), r, q);
-    return fma(fma(-b, q1, a), r, q1);
+    return fma(fma(-b, q, a), r, q);
 }
+__device__ __forceinline__ double near_div(double a, double b) { return mid_div(a, b); }
 __device__ __forceinline__ double fast_div(double a, double b) {
     if ((__double2hiint(a) & 0x7fffffff) >= 0x7ff00000 || (unsigned)(__double2hiint(b) & 0x7fffffff) - 0x00300000u >= 0x7fa00000u) return a / b;
-    return near_div(a, b);
+    return mid_div(a, b);
 }
 __device__ __forceinline__ float near_div(float a, float b) { return pdiv(a, b); }
 
