@@ -47,10 +47,14 @@ inline int march_chunk(long long columns, int planes, int sms, double setup, dou
 }
 
 enum CellsWhat { WHAT_STRESS = 0, WHAT_STRESS_LAW, WHAT_STRAIN, WHAT_VISC };
+// Resident blocks per SM that the registers of k_cells leave room for.  us a launch without a bound (123 registers) and with 20 (96):
+// spherical 63^3, WHAT_STRESS, whose blocks are all resident at 20 only, 56.1 and 55.2; 127^3 sector, WHAT_STRESS_LAW,
+// 384 and 385.
+constexpr int cells_blocks(int what) { return what == WHAT_STRESS || what == WHAT_STRESS_LAW ? 20 : 24; }
 
 // RHS: continuity right-hand side rP (P -= KBDT (div V + rP))
 template <typename T, int G, int WHAT, bool RHS>
-__global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p, int chunk) {
+__global__ void __launch_bounds__(MC_NT, cells_blocks(WHAT)) k_cells(const __grid_constant__ KP<T> p, int chunk) {
     constexpr bool PT = WHAT == WHAT_STRESS || WHAT == WHAT_STRESS_LAW;
     constexpr bool ETA = WHAT != WHAT_STRAIN;
     pdl_enter_small();
@@ -72,20 +76,53 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
     const T e23_3 = G == SPH ? e.iRc1 * e.iSh * p.d3 : p.d3;
     const bool v12 = i < d.n1 - 1 && j < d.n2 - 1, v13 = i < d.n1 - 1 && j < d.n2 - 2, v23 = i < d.n1 - 2 && j < d.n2 - 1;
     int c = i + sy * j + sz * k0;
-    // sums over two cells of a plane: X along x1 in row j + 1, Y along x2 in column i + 1
+    // Sums over two cells of a plane: X along x1 in row j + 1, Y along x2 in column i + 1.  Cells past the grid are
+    // replaced by the last ones inside (their edges are not stored), so that `mid` tells of cells of the grid only.
+    const int ox = i < d.n1 - 1 ? 1 : 0, oy = j < d.n2 - 1 ? sy : 0;
     T eX = T(0), eY = T(0), sX = T(0), sY = T(0);
-    if (ETA) {
-        const T a = p.eta[c + 1], b = p.eta[c + sy], q = p.eta[c + sy + 1];
-        eX = b + q; eY = a + q;
-    }
+    // whether the quotients of this column may be formed by mid_div: its steps, and η and ηSM of the plane below
+    bool steps = true, below = true;
     if (PT) {
-        const T a = p.etaSM[c + 1], b = p.etaSM[c + sy], q = p.etaSM[c + sy + 1];
-        sX = b + q; sY = a + q;
+        MidRange<T, 60> m;
+        m.add(p.gsc); m.add(p.kbc); m.add(p.vpdt2);
+        steps = m.ok();
+    }
+    {
+        MidRange<T, 400> m;
+        if (ETA) {
+            const T a = p.eta[c + ox], b = p.eta[c + oy], q = p.eta[c + ox + oy];
+            eX = b + q; eY = a + q;
+            if (PT) { m.add(p.eta[c]); m.add(a); m.add(b); m.add(q); }
+        }
+        if (PT) {
+            const T a = p.etaSM[c + ox], b = p.etaSM[c + oy], q = p.etaSM[c + ox + oy];
+            sX = b + q; sY = a + q;
+            m.add(p.etaSM[c]); m.add(a); m.add(b); m.add(q);
+            below = steps && m.ok();
+        }
     }
     const T gsc4 = T(0.25) * p.gsc;
-    // (entries past the grid are padding of the box: finite, and their results are not stored)
+    // (velocities past the grid are padding of the box: finite, and their results are not stored)
     for (int k = k0; k < k1; ++k, c += sz) {
         const int u = c + sz;
+        // sums of the plane above; edges of it: sums e, s of η and ηSM over four cells
+        T e12 = T(0), e13 = T(0), e23 = T(0), s12 = T(0), s13 = T(0), s23 = T(0);
+        const int w = k < d.n3 - 1 ? u : c;
+        MidRange<T, 400> mid;
+        if (ETA) {
+            const T o = p.eta[w], a = p.eta[w + ox], b = p.eta[w + oy], q = p.eta[w + ox + oy];
+            const T x = b + q, y = a + q;
+            e12 = (o + a) + x; e13 = eX + x; e23 = eY + y;
+            eX = x; eY = y;
+            if (PT) { mid.add(o); mid.add(a); mid.add(b); mid.add(q); }
+        }
+        if (PT) {
+            const T o = p.etaSM[w], a = p.etaSM[w + ox], b = p.etaSM[w + oy], q = p.etaSM[w + ox + oy];
+            const T x = b + q, y = a + q;
+            s12 = gsc4 * ((o + a) + x); s13 = gsc4 * (sX + x); s23 = gsc4 * (sY + y);  // aG = GSDT s / 4
+            sX = x; sY = y;
+            mid.add(o); mid.add(a); mid.add(b); mid.add(q);
+        }
         const T v1p = p.V1[c + 1], v2p = p.V2[c + sy], v3p = p.V3[u];
         const T D1 = v1p - p.V1[c], D2 = v2p - p.V2[c], D3 = v3p - p.V3[c];
         T D11 = p.d1 * D1, D22, D33, div;
@@ -99,61 +136,55 @@ __global__ void __launch_bounds__(MC_NT) k_cells(const __grid_constant__ KP<T> p
             D22 = a2 * D2; D33 = a3 * D3;
             div = D11 + D22 + D33;
         }
-        if (WHAT == WHAT_STRAIN || WHAT == WHAT_STRESS_LAW) p.sDD[c] = h * fma(D11, D11, fma(D22, D22, D33 * D33));
+        const T v1a = p.V1[u + 1], v1b = p.V1[u + 1 + sy], v2a = p.V2[u + sy], v2b = p.V2[u + sy + 1];
+        const T v3q = p.V3[u + sy], v3t = p.V3[u + sy + 1], v3s = p.V3[u + 1];
+        T D12 = fma(e12_2, v1b - v1a, e1_d * (v2b - v2a));
+        if (G != CART) D12 = fma(e1_v, v2a, D12);
+        T D13 = fma(e13_3, v1b - p.V1[c + 1 + sy], e13_d * (v3t - v3q));
+        if (G == SPH) D13 = fma(e1_v, v3q, D13);
+        T D23 = fma(e23_3, v2b - p.V2[c + 1 + sy], e23_2 * (v3t - v3s));
+        if (G == SPH) D23 = fma(e23_v, v3s, D23);
+        const bool w12 = v12 && k < d.n3 - 2, w13 = v13 && k < d.n3 - 1, w23 = v23 && k < d.n3 - 1;
+        if (WHAT == WHAT_STRAIN || WHAT == WHAT_STRESS_LAW) {
+            p.sDD[c] = h * fma(D11, D11, fma(D22, D22, D33 * D33));
+            if (w12) p.s12[c] = D12;
+            if (w13) p.s13[c] = D13;
+            if (w23) p.s23[c] = D23;
+        }
         if (PT) {
-            const T sm = p.etaSM[c], et = p.eta[c];
+            const T et = p.eta[c], sm = p.etaSM[c];
             const T gs = p.gsc * sm, kb = p.kbc * sm, gs2 = gs + gs;
-            const T f = near_div(et, et + gs);  // 1/(1 + GSDT/η)
+            const T m11 = fma(gs2, D11, p.t11[c]), m22 = fma(gs2, D22, p.t22[c]), m33 = fma(gs2, D33, p.t33[c]);
+            const T m12 = fma(s12, D12, p.t12[c]), m13 = fma(s13, D13, p.t13[c]), m23 = fma(s23, D23, p.t23[c]);
             T Pn = fma(-kb, RHS ? div + p.rP[c] : div, p.P[c]);
-            const T n11 = fma(gs2, D11, p.t11[c]) * f, n22 = fma(gs2, D22, p.t22[c]) * f, n33 = fma(gs2, D33, p.t33[c]) * f;
+            // 1/(1 + GSDT/η), the step, and at the edges aE / (aE + aG), aE = e / 4.  One rare branch for all five,
+            // behind the loads of the plane: a branch for each cost 10 % of an iteration, one before the loads 4 %.
+            const T b0 = et + gs, b12 = fma(T(4), s12, e12), b13 = fma(T(4), s13, e13), b23 = fma(T(4), s23, e23);
+            T f = mid_div(et, b0), dt = mid_div(p.vpdt2, fma(gs, f, kb)), q12 = mid_div(e12, b12), q13 = mid_div(e13, b13), q23 = mid_div(e23, b23);
+            const bool above = steps && mid.ok();
+            if (__builtin_expect(!(below && above), 0)) {
+                f = et / b0;
+                dt = p.vpdt2 / fma(gs, f, kb);
+                q12 = e12 / b12; q13 = e13 / b13; q23 = e23 / b23;
+            }
+            below = above;
+            const T n11 = m11 * f, n22 = m22 * f, n33 = m33 * f;
             if (p.traction) traction_pressure(j, k, d.n2, d.n3, n22, n33, p.sig2, p.sig3, Pn);
             if (p.fs && i == d.n1 - 1) Pn = fs_pressure(n11, p.top_load ? p.top_load[c] : T(0), p.fs_kappa, p.V1[c], v1p);
             p.P[c] = Pn;
             p.t11[c] = n11; p.t22[c] = n22; p.t33[c] = n33;
-            p.DT_R[c] = near_div(p.vpdt2, fma(gs, f, kb));
+            p.DT_R[c] = dt;
+            if (w12) p.t12[c] = m12 * q12;
+            if (w13) p.t13[c] = m13 * q13;
+            if (w23) p.t23[c] = m23 * q23;
         } else if (WHAT == WHAT_VISC) {
             const T x = T(2) * p.eta[c];
             p.t11[c] = x * D11; p.t22[c] = x * D22; p.t33[c] = x * D33;
             p.rP[c] = div;
+            if (w12) p.t12[c] = T(0.25) * e12 * D12;
+            if (w13) p.t13[c] = T(0.25) * e13 * D13;
+            if (w23) p.t23[c] = T(0.25) * e23 * D23;
         }
-        // edges: sums of the plane above
-        T eX0 = T(0), eXn = T(0), eYn = T(0), sX0 = T(0), sXn = T(0), sYn = T(0);
-        if (ETA) {
-            const T a = p.eta[u + 1], b = p.eta[u + sy], q = p.eta[u + sy + 1];
-            eX0 = p.eta[u] + a; eXn = b + q; eYn = a + q;
-        }
-        if (PT) {
-            const T a = p.etaSM[u + 1], b = p.etaSM[u + sy], q = p.etaSM[u + sy + 1];
-            sX0 = p.etaSM[u] + a; sXn = b + q; sYn = a + q;
-        }
-        auto edge = [&](T* t, T* s, T D, T e4, T s4, bool ok) {
-            if (PT) {  // (τ + aG D) aE / (aE + aG), aE = e4 / 4, aG = GSDT s4 / 4
-                const T g = gsc4 * s4;
-                const T v = fma(g, D, t[c]) * near_div(e4, fma(T(4), g, e4));
-                if (ok) t[c] = v;
-            } else if (WHAT == WHAT_VISC) {
-                if (ok) t[c] = T(0.25) * e4 * D;
-            }
-            if ((WHAT == WHAT_STRAIN || WHAT == WHAT_STRESS_LAW) && ok) s[c] = D;
-        };
-        const T v1a = p.V1[u + 1], v1b = p.V1[u + 1 + sy], v2a = p.V2[u + sy], v2b = p.V2[u + sy + 1];
-        const T v3q = p.V3[u + sy], v3t = p.V3[u + sy + 1], v3s = p.V3[u + 1];
-        {
-            T D = fma(e12_2, v1b - v1a, e1_d * (v2b - v2a));
-            if (G != CART) D = fma(e1_v, v2a, D);
-            edge(p.t12, p.s12, D, eX0 + eXn, sX0 + sXn, v12 && k < d.n3 - 2);
-        }
-        {
-            T D = fma(e13_3, v1b - p.V1[c + 1 + sy], e13_d * (v3t - v3q));
-            if (G == SPH) D = fma(e1_v, v3q, D);
-            edge(p.t13, p.s13, D, eX + eXn, sX + sXn, v13 && k < d.n3 - 1);
-        }
-        {
-            T D = fma(e23_3, v2b - p.V2[c + 1 + sy], e23_2 * (v3t - v3s));
-            if (G == SPH) D = fma(e23_v, v3s, D);
-            edge(p.t23, p.s23, D, eY + eYn, sY + sYn, v23 && k < d.n3 - 1);
-        }
-        eX = eXn; eY = eYn; sX = sXn; sY = sYn;
     }
 }
 
@@ -261,24 +292,29 @@ __device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by
             x = fma(1.0 / 64.0, fma(a, a, fma(b, b, q * q)), p.sDD[s]);
             last = kc;
         }
-        const double ei = p.eta_ini[c];
+        const double ei = p.eta_ini[c], eo = RELAXED ? p.eta[c] : ei, w = x * p.law_i2;
+        const bool lin = p.phase && p.phase[c], half = p.relax == 0.5;
         double et = ei;
-        if (!(p.phase && p.phase[c])) {
-            const double w = x * p.law_i2;
-            double f;
-            if (p.law_q && root_range(w)) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
-            else if (normal_pos(w)) f = fast_pow(tab, w, p.law_ex);
-            else f = pow(sqrt(x) / p.edot_bg, 2.0 * p.law_ex);  // (the square of the ratio leaves the range first)
-            et = fast_div(ei + ei, 1.0 + f);
-        }
-        if (RELAXED) {
-            // the half-way mean as a root, else η (η_t/η)^relax; by logarithms where the product or the quotient is no
-            // normal number (a cell without viscosity keeps none)
-            const double eo = p.eta[c];
-            const bool half = p.relax == 0.5;
-            const double r = half ? eo * et : fast_div(et, eo);
-            if (normal_pos(r)) et = half ? fast_sqrt(r) : eo * fast_pow(tab, r, p.relax);
-            else et = exp((1.0 - p.relax) * log(eo) + p.relax * log(et));
+        MidRange<double, 400> mid;
+        mid.add(ei); mid.add(eo);
+        if (p.law_q && (half || !RELAXED) && mid.ok() && root_range(w)) {  // (every intermediate value is a normal number)
+            if (!lin) et = mid_div(ei + ei, 1.0 + root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el));
+            if (RELAXED) et = mid_sqrt(eo * et);
+        } else {
+            if (!lin) {
+                double f;
+                if (p.law_q && root_range(w)) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
+                else if (normal_pos(w)) f = fast_pow(tab, w, p.law_ex);
+                else f = pow(sqrt(x) / p.edot_bg, 2.0 * p.law_ex);  // (the square of the ratio leaves the range first)
+                et = near_div(ei + ei, 1.0 + f);
+            }
+            if (RELAXED) {
+                // the half-way mean as a root, else η (η_t/η)^relax; by logarithms where the product or the quotient is no
+                // normal number (a cell without viscosity keeps none)
+                const double r = half ? eo * et : near_div(et, eo);
+                if (normal_pos(r)) et = half ? fast_sqrt(r) : eo * fast_pow(tab, r, p.relax);
+                else et = exp((1.0 - p.relax) * log(eo) + p.relax * log(et));
+            }
         }
         p.eta_out[c] = et;
     }
@@ -336,7 +372,7 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
         if (!RELAX) {
             double f = w;
             if (!p.law_q) f = normal_pos(x) ? fast_pow(tab, x, cx) : pow(tii / p.tau_C, 2.0 * cx);  // (as in edot_body)
-            p.eta[c] = fast_div(ei + ei, 1.0 + f);
+            p.eta[c] = near_div(ei + ei, 1.0 + f);
         } else {
             const double po = p.eta_pl[c];
             double pl;
@@ -346,7 +382,7 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
                 // (η_PL itself, ei / w, has to be a normal number too: where it is not, it is 0 or infinite, as in power_law!)
                 const int ex = (__double2hiint(ei) >> 20) - (__double2hiint(w) >> 20);
                 if (normal_pos(w) && normal_pos(ei) && normal_pos(po) && normal_pos(den) && ex > -1000 && ex < 1000) {
-                    const double r = fast_div(ei, den);
+                    const double r = near_div(ei, den);
                     if (normal_pos(r)) {
                         double h, t;
                         log2_parts(tab, r, h, t);
@@ -378,7 +414,7 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
             }
             p.eta_pl[c] = pl;
             const double num = (ei + ei) * pl;
-            p.eta[c] = done && normal_pos(num) ? fast_div(num, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
+            p.eta[c] = done && normal_pos(num) ? near_div(num, ei + pl) : 2.0 / (1.0 / ei + 1.0 / pl);
         }
     }
 }

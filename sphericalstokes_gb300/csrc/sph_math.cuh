@@ -9,11 +9,11 @@
 
 namespace sph {
 
-// a / b in five FP64 operations: PTX's approximate reciprocal r (relative error e near 2^-20), one Newton step (e^2),
-// the quotient a r and one step by its residual, q += r (a - b q) (Markstein, IBM J. Res. Dev. 34, 1990), which leaves e^4
-// before the last rounding: the IEEE quotient but for about one pair of operands in 2^24.  (Two residual steps with the
-// reciprocal as it comes take as many operations and leave e^3: 297 of 2^20 quotients were one unit off.)  For b and the
-// quotient inside the range of normal numbers.
+// a / b in five FP64 operations, for operands of 2^-500 .. 2^500 in magnitude (quotient and residuals are then inside the
+// range of normal numbers): PTX's approximate reciprocal r (relative error e near 2^-20), one Newton step (e^2), the
+// quotient a r and one step by its residual, q += r (a - b q) (Markstein, IBM J. Res. Dev. 34, 1990), which leaves e^4
+// before the last rounding: the IEEE quotient but for about one pair of operands in 2^24.  (Two residual steps with
+// the reciprocal as it comes take as many operations and leave e^3: 297 of 2^20 quotients were one unit off.)
 __device__ __forceinline__ double mid_div(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
@@ -21,17 +21,33 @@ __device__ __forceinline__ double mid_div(double a, double b) {
     const double q = a * r;
     return fma(fma(-b, q, a), r, q);
 }
-__device__ __forceinline__ double near_div(double a, double b) { return mid_div(a, b); }
-__device__ __forceinline__ double fast_div(double a, double b) {
-    if ((__double2hiint(a) & 0x7fffffff) >= 0x7ff00000 || (unsigned)(__double2hiint(b) & 0x7fffffff) - 0x00300000u >= 0x7fa00000u) return a / b;
-    return mid_div(a, b);
+__device__ __forceinline__ float mid_div(float a, float b) { return pdiv(a, b); }
+
+// whether every number added is positive and of 2^-E .. 2^E (integer operations, no FP64 issue)
+template <typename T, int E>
+struct MidRange {
+    unsigned lo = ~0u, hi = 0u;
+    __device__ __forceinline__ void add(T x) {
+        if constexpr (sizeof(T) == 8) {
+            const unsigned v = (unsigned)__double2hiint(x);
+            lo = min(lo, v);
+            hi = max(hi, v);
+        }
+    }
+    __device__ __forceinline__ bool ok() const { return sizeof(T) != 8 || (lo >= (1023u - E) << 20 && hi < (1023u + E) << 20); }
+};
+
+// a / b of any operands: those that are not positive or outside the range, infinities and NaN among them, by the IEEE division
+__device__ __forceinline__ double near_div(double a, double b) {
+    MidRange<double, 500> m;
+    m.add(a);
+    m.add(b);
+    return m.ok() ? mid_div(a, b) : a / b;
 }
-__device__ __forceinline__ float near_div(float a, float b) { return pdiv(a, b); }
 
 // square root of a positive normal x in seven FP64 operations: the approximate reciprocal root, one
 // coupled (Goldschmidt) step for the root and half its reciprocal, and the residual correction; others by sqrt()
-__device__ __forceinline__ double fast_sqrt(double x) {
-    if (!((unsigned)__double2hiint(x) - 0x00200000u < 0x7fc00000u)) return sqrt(x);
+__device__ __forceinline__ double mid_sqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double g = x * y, h = 0.5 * y;
@@ -39,6 +55,7 @@ __device__ __forceinline__ double fast_sqrt(double x) {
     const double g1 = fma(g, e, g);
     return fma(fma(-g1, g1, x), fma(h, e, h), g1);
 }
+__device__ __forceinline__ double fast_sqrt(double x) { return (unsigned)__double2hiint(x) - 0x00200000u < 0x7fc00000u ? mid_sqrt(x) : sqrt(x); }
 
 // ---------------------------------------------------------------------------
 // x^c of positive normal numbers, after the table-driven scheme of P. T. P. Tang (ACM TOMS 15-18, 1989-1992):

@@ -62,6 +62,25 @@ def test_near_div_is_the_ieee_quotient(probe, lo, hi):
     nearly_ieee(probe(0, a, a + b), a / (a + b), 4)
 
 
+@pytest.mark.parametrize("ea", [-1022, -501, -499, 0, 498, 500, 1022])
+@pytest.mark.parametrize("eb", [-1022, -501, -499, 0, 498, 500, 1022])
+def test_near_div_over_the_range(probe, ea, eb):
+    """the edges of the range whose quotients are formed without the IEEE division, overflow and underflow"""
+    rng = np.random.default_rng(5)
+    a, b = numbers(rng, ea, ea + 2, 1 << 12), numbers(rng, eb, eb + 2, 1 << 12)
+    with np.errstate(over="ignore", under="ignore"):
+        nearly_ieee(probe(0, a, b), a / b, 0)
+
+
+def test_near_div_of_any_operand(probe):
+    v = [0.0, 5e-324, 1e-310, 2.3e-308, 1e-200, 1e-155, 1.0, 1e155, 1e200, 1e300, 1.79e308, np.inf, np.nan]
+    v = np.array(v + [-x for x in v])
+    a, b = (x.ravel() for x in np.meshgrid(v, v))
+    with np.errstate(all="ignore"):
+        np.testing.assert_array_equal(probe(0, a, b), a / b)
+        np.testing.assert_array_equal(np.signbit(probe(0, a, b))[~np.isnan(a / b)], np.signbit(a / b)[~np.isnan(a / b)])
+
+
 @pytest.mark.parametrize("lo,hi", [(-1, 1), (-30, 30), (-1000, 1000)])
 def test_fast_sqrt_is_the_ieee_root(probe, lo, hi):
     a = numbers(np.random.default_rng(2), lo, hi)
