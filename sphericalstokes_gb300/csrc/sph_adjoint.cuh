@@ -37,16 +37,16 @@ struct Adj {
     double *d11, *d22, *d33;             // adjoint of the strain rates: 2η aτ, or the memory μ (MEM)
     double *e12, *e13, *e23;             // edges: avg4(η) aτ, or μ
     double *x12, *x13, *x23;             // law: edge adjoints with the law's part
-    double *q12, *q13, *q23;             // edge adjoint times D / (4 avg4 η)
+    double *q12, *q13, *q23;             // edges' share of λᵀ ∂R/∂η of each of their four cells
     double *E1, *M1, *E2, *M2, *E3;      // cells: what V reads of them (cell_out)
     double *aV1, *aV2, *aV3, *aP;        // output: adjoint of V (all entries), P
     double *gEta, *gRho, *gW;            // λᵀ ∂R/∂η, λᵀ ∂R/∂ρ per cell; gEta times the law's derivative
     // fixed factors (k_adj_setup)
-    double *fc, *wc;                     // cells: f, (1 - f) 2η
-    double *f12, *f13, *f23, *w12, *w13, *w23;  // edges: f, (1 - f) avg4 η
-    double *c11, *c22, *c33;             // D_ii / η
-    double *g12, *g13, *g23;             // D_edge / (4 avg4 η)
-    double *lw, *lr, *la, *lb, *lc;      // law: dη_t/dε̇, η/(2ε̇), and (mean shear rates) / (16 ε̇) of interior cells
+    double *wc, *ie;                     // cells: 1 - f, 1 / η
+    double *y12, *y13, *y23, *w12, *w13, *w23;  // edges: avg4 η, 1 - f
+    double *c11, *c22, *c33;             // D_ii
+    double *g12, *g13, *g23;             // law: D_edge / (4 avg4 η)
+    double *lw, *lr, *la, *lb, *lc;      // law: dη_t/dε̇, 1/(2ε̇), and (mean shear rates) / (16 ε̇) of interior cells
 };
 
 // cell adjoints aD_ii and λ_P as the six face velocities read them: +-E1 + M1 (V1), +-E2 + M2, +-E3
@@ -69,28 +69,28 @@ __global__ void __launch_bounds__(MC_NT) k_adj_setup(const __grid_constant__ KP<
     if (j >= d.n2) return;
     const int sy = d.sy, sz = d.sz, c = i + sy * j + sz * k;
     const double et = p.eta[c], gs = p.gsc * p.etaSM[c];
-    a.fc[c] = et / (et + gs);
-    a.wc[c] = 2.0 * et * (gs / (et + gs));
+    a.wc[c] = gs / (et + gs);
+    a.ie[c] = 1.0 / et;
     const CellD<double> D = cell_strain<double, G>(p.geo, p.d1, p.d2, p.d3, i, j, p.V1[c], p.V1[c + 1], p.V2[c], p.V2[c + sy], p.V3[c], p.V3[c + sz]);
-    a.c11[c] = D.D11 / et; a.c22[c] = D.D22 / et; a.c33[c] = D.D33 / et;
-    auto edge = [&](double* f, double* w, double* g, int q, int o1, int o2, int o3, double De) {
+    a.c11[c] = D.D11; a.c22[c] = D.D22; a.c33[c] = D.D33;
+    auto edge = [&](double* y, double* w, double* g, int q, int o1, int o2, int o3, double De) {
         const double aE = 0.25 * (p.eta[q] + p.eta[q + o1] + p.eta[q + o2] + p.eta[q + o3]);
         const double aG = 0.25 * p.gsc * (p.etaSM[q] + p.etaSM[q + o1] + p.etaSM[q + o2] + p.etaSM[q + o3]);
-        f[c] = aE / (aE + aG);
-        w[c] = aE * (aG / (aE + aG));
-        g[c] = 0.25 * De / aE;
+        y[c] = aE;
+        w[c] = aG / (aE + aG);
+        if (LAW) g[c] = 0.25 * De / aE;
     };
     if (i < d.n1 - 1 && j < d.n2 - 1 && k < d.n3 - 2) {
         const int q = c + sz;
-        edge(a.f12, a.w12, a.g12, q, sy, 1, 1 + sy, edge12<double, G>(p.geo, p.d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]));
+        edge(a.y12, a.w12, a.g12, q, sy, 1, 1 + sy, edge12<double, G>(p.geo, p.d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]));
     }
     if (i < d.n1 - 1 && j < d.n2 - 2 && k < d.n3 - 1) {
         const int q = c + sy;
-        edge(a.f13, a.w13, a.g13, q, sz, 1, 1 + sz, edge13<double, G>(p.geo, p.d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]));
+        edge(a.y13, a.w13, a.g13, q, sz, 1, 1 + sz, edge13<double, G>(p.geo, p.d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]));
     }
     if (i < d.n1 - 2 && j < d.n2 - 1 && k < d.n3 - 1) {
         const int q = c + 1;
-        edge(a.f23, a.w23, a.g23, q, sz, sy, sy + sz, edge23<double, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]));
+        edge(a.y23, a.w23, a.g23, q, sz, sy, sy + sz, edge23<double, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]));
     }
     if (!LAW) return;
     // The law (k_edot, unrelaxed target η_t = 2/(1/η_ini + 1/η_PL), η_PL = η_ini (ε̇_II/ε̇_bg)^m, m = (1-n)/n, ε̇_II of the
@@ -110,15 +110,16 @@ __global__ void __launch_bounds__(MC_NT) k_adj_setup(const __grid_constant__ KP<
     }
     a.lw[c] = w;
     const bool own = s == c && ed > 0.0;  // interior cell
-    a.lr[c] = own ? et / (2.0 * ed) : 0.0;
+    a.lr[c] = own ? 1.0 / (2.0 * ed) : 0.0;
     a.la[c] = own ? av / (16.0 * ed) : 0.0;
     a.lb[c] = own ? bv / (16.0 * ed) : 0.0;
     a.lc[c] = own ? cv / (16.0 * ed) : 0.0;
 }
 
 // λ_V -> adjoint of σ (cells; the traction-slaved pressure of far-field-stress boundary cells goes to τ22 / τ33)
-// and of the edge stresses.  MEM: the memory μ relaxes toward it and λ_P -= KBDT (M_Pᵀ λ_V - b_P); else
-// the adjoints of the strain rates themselves, of P and ρ.  LAW: k_adj_law finishes the cells.
+// and of the edge stresses.  MEM: the memory μ relaxes toward it, μ += (1 - f) (2η σ - μ), whose fixed point is 2η σ
+// whatever the rounding of f, and λ_P -= KBDT (M_Pᵀ λ_V - b_P); else the adjoints of the strain rates
+// themselves, of P, ρ and η (σ D: no quotient by η, which may be zero).  LAW: k_adj_law finishes the cells.
 template <int G, bool MEM, bool LAW>
 __global__ void __launch_bounds__(MC_NT) k_adj_stress(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, int chunk) {
     pdl_enter_small();
@@ -178,38 +179,50 @@ __global__ void __launch_bounds__(MC_NT) k_adj_stress(const __grid_constant__ KP
         const double aP = b2 || b3 ? 0.0 : pe;
         double D11, D22, D33, lP = a.lP[c];
         if (MEM) {
-            const double f = a.fc[c], w = a.wc[c];
-            D11 = fma(w, s11, f * a.d11[c]); D22 = fma(w, s22, f * a.d22[c]); D33 = fma(w, s33, f * a.d33[c]);
+            const double w = a.wc[c], e2 = 2.0 * p.eta[c];
+            D11 = a.d11[c]; D22 = a.d22[c]; D33 = a.d33[c];
+            D11 = fma(w, fma(e2, s11, -D11), D11); D22 = fma(w, fma(e2, s22, -D22), D22); D33 = fma(w, fma(e2, s33, -D33), D33);
             lP = fma(-p.kbc * p.etaSM[c], aP - a.bP[c], lP);
             a.lP[c] = lP;
         } else {
             const double e2 = 2.0 * p.eta[c];
             D11 = e2 * s11; D22 = e2 * s22; D33 = e2 * s33;
             a.aP[c] = aP;
+            a.gEta[c] = 2.0 * fma(s11, a.c11[c], fma(s22, a.c22[c], s33 * a.c33[c]));
             if (G != CART) a.gRho[c] = -0.5 * p.g * (A0 + A1);
             else a.gRho[c] = -0.5 * p.g * (Z0 + Z1);
         }
         a.d11[c] = D11; a.d22[c] = D22; a.d33[c] = D33;
         if (!LAW) cell_out<G>(m, d1, a, c, D11, D22, D33, lP);
-        auto edge = [&](double* E, double* Q, const double* f, const double* w, const double* g, double t, int q, int o1, int o2, int o3) {
-            double x;
-            if (MEM) x = fma(w[c], t, f[c] * E[c]);
-            else x = 0.25 * (p.eta[q] + p.eta[q + o1] + p.eta[q + o2] + p.eta[q + o3]) * t;
+        auto edge = [&](double* E, double* Q, const double* y, const double* w, const double* g, double t, double De) {
+            double x = E[c];
+            if (MEM) x = fma(w[c], fma(y[c], t, -x), x);
+            else x = y[c] * t;
             E[c] = x;
-            if (!MEM || LAW) Q[c] = g[c] * x;
+            if (!MEM) Q[c] = 0.25 * t * De;
+            else if (LAW) Q[c] = g[c] * x;
         };
         const double A11 = L1(1, 1, 1), B11 = L2(1, 1, 1), Z11 = L3(1, 1, 1);
-        if (e12 && k < n3 - 2)
-            edge(a.e12, a.q12, a.f12, a.w12, a.g12, fma(t12a, L1(1, 0, 1), fma(t12b, A11, fma(t12c, L2(0, 1, 1), t12d * B11))), c + sz, sy, 1, 1 + sy);
-        if (e13 && k < n3 - 1)
-            edge(a.e13, a.q13, a.f13, a.w13, a.g13, fma(t13a, L1(1, 1, 0) - A11, fma(t13c, L3(0, 1, 1), t13d * Z11)), c + sy, sz, 1, 1 + sz);
-        if (e23 && k < n3 - 1)
-            edge(a.e23, a.q23, a.f23, a.w23, a.g23, fma(t23a, L2(1, 1, 0) - B11, fma(t23c, L3(1, 0, 1), t23d * Z11)), c + 1, sz, sy, sy + sz);
+        if (e12 && k < n3 - 2) {
+            const int q = c + sz;
+            const double De = MEM ? 0.0 : edge12<double, G>(p.geo, d1, p.d2, i, p.V2[q + sy], p.V2[q + sy + 1], p.V1[q + 1], p.V1[q + 1 + sy]);
+            edge(a.e12, a.q12, a.y12, a.w12, a.g12, fma(t12a, L1(1, 0, 1), fma(t12b, A11, fma(t12c, L2(0, 1, 1), t12d * B11))), De);
+        }
+        if (e13 && k < n3 - 1) {
+            const int q = c + sy;
+            const double De = MEM ? 0.0 : edge13<double, G>(p.geo, d1, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + 1], p.V1[q + 1], p.V1[q + 1 + sz]);
+            edge(a.e13, a.q13, a.y13, a.w13, a.g13, fma(t13a, L1(1, 1, 0) - A11, fma(t13c, L3(0, 1, 1), t13d * Z11)), De);
+        }
+        if (e23 && k < n3 - 1) {
+            const int q = c + 1;
+            const double De = MEM ? 0.0 : edge23<double, G>(p.geo, p.d2, p.d3, i, j, p.V3[q + sz], p.V3[q + sz + sy], p.V2[q + sy], p.V2[q + sy + sz]);
+            edge(a.e23, a.q23, a.y23, a.w23, a.g23, fma(t23a, L2(1, 1, 0) - B11, fma(t23c, L3(1, 0, 1), t23d * Z11)), De);
+        }
     }
 }
 
-// λᵀ ∂R/∂η per cell: the cell's own part and its twelve edges'; times the law's derivative for k_adj_law
-template <bool LAW>
+// λᵀ ∂R/∂η per cell: the cell's own part (of the memory: μ D / η) and its twelve edges'; times the law's derivative for k_adj_law
+template <bool MEM, bool LAW>
 __global__ void __launch_bounds__(MC_NT) k_adj_eta(const __grid_constant__ KP<double> p, const __grid_constant__ Adj a, int chunk) {
     pdl_enter_small();
     const Dims& d = p.d;
@@ -223,7 +236,9 @@ __global__ void __launch_bounds__(MC_NT) k_adj_eta(const __grid_constant__ KP<do
         const int c = i + sy * j + sz * k;
         const bool km = k > 0;
         // (edge entries outside the edges' extents are zero)
-        double g = fma(a.d11[c], a.c11[c], fma(a.d22[c], a.c22[c], a.d33[c] * a.c33[c]));
+        double g;
+        if (MEM) g = fma(a.d11[c], a.c11[c], fma(a.d22[c], a.c22[c], a.d33[c] * a.c33[c])) * a.ie[c];
+        else g = a.gEta[c];
         if (km) g += (a.q12[c - sz] + (im ? a.q12[c - 1 - sz] : 0.0)) + (jm ? a.q12[c - sy - sz] + (im ? a.q12[c - 1 - sy - sz] : 0.0) : 0.0);
         if (jm) g += (a.q13[c - sy] + (im ? a.q13[c - 1 - sy] : 0.0)) + (km ? a.q13[c - sy - sz] + (im ? a.q13[c - 1 - sy - sz] : 0.0) : 0.0);
         if (im) g += (a.q23[c - 1] + (jm ? a.q23[c - 1 - sy] : 0.0)) + (km ? a.q23[c - 1 - sz] + (jm ? a.q23[c - 1 - sy - sz] : 0.0) : 0.0);

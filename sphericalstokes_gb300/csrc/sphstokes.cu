@@ -2152,7 +2152,7 @@ enum AdjSlot {
     AJ_GEI, AJ_GN, AJ_M11, AJ_M22, AJ_M33, AJ_M12, AJ_M13, AJ_M23,  // memory of the transposed PT
     AJ_D11, AJ_D22, AJ_D33, AJ_E12, AJ_E13, AJ_E23,                 // adjoints of the strain rates (no memory)
     AJ_X12, AJ_X13, AJ_X23, AJ_Q12, AJ_Q13, AJ_Q23, AJ_O1, AJ_O2, AJ_O3, AJ_O4, AJ_O5, AJ_GW,
-    AJ_FC, AJ_WC, AJ_F12, AJ_F13, AJ_F23, AJ_W12, AJ_W13, AJ_W23, AJ_C11, AJ_C22, AJ_C33, AJ_G12, AJ_G13, AJ_G23,
+    AJ_WC, AJ_IE, AJ_Y12, AJ_Y13, AJ_Y23, AJ_W12, AJ_W13, AJ_W23, AJ_C11, AJ_C22, AJ_C33, AJ_G12, AJ_G13, AJ_G23,
     AJ_LW, AJ_LR, AJ_LA, AJ_LB, AJ_LC, AJ_COUNT
 };
 
@@ -2216,8 +2216,8 @@ static Adj adj_ptrs(Ctx* c, bool mem) {
     a.E1 = s(AJ_O1); a.M1 = s(AJ_O2); a.E2 = s(AJ_O3); a.M2 = s(AJ_O4); a.E3 = s(AJ_O5);
     a.aV1 = s(AJ_V1); a.aV2 = s(AJ_V2); a.aV3 = s(AJ_V3); a.aP = s(AJ_P);
     a.gEta = s(AJ_GETA); a.gRho = s(AJ_GRHO); a.gW = s(AJ_GW);
-    a.fc = s(AJ_FC); a.wc = s(AJ_WC);
-    a.f12 = s(AJ_F12); a.f13 = s(AJ_F13); a.f23 = s(AJ_F23); a.w12 = s(AJ_W12); a.w13 = s(AJ_W13); a.w23 = s(AJ_W23);
+    a.wc = s(AJ_WC); a.ie = s(AJ_IE);
+    a.y12 = s(AJ_Y12); a.y13 = s(AJ_Y13); a.y23 = s(AJ_Y23); a.w12 = s(AJ_W12); a.w13 = s(AJ_W13); a.w23 = s(AJ_W23);
     a.c11 = s(AJ_C11); a.c22 = s(AJ_C22); a.c33 = s(AJ_C33); a.g12 = s(AJ_G12); a.g13 = s(AJ_G13); a.g23 = s(AJ_G23);
     a.lw = s(AJ_LW); a.lr = s(AJ_LR); a.la = s(AJ_LA); a.lb = s(AJ_LB); a.lc = s(AJ_LC);
     return a;
@@ -2259,11 +2259,11 @@ static void adj_rows(Ctx* c, const KP<double>& p, const Adj& a) {
     if (law) launch_pdl(c->use_pdl, k_adj_stress<G, MEM, true>, adj_cells(c, ks), nt, 0, c->stream, p, a, ks);
     else launch_pdl(c->use_pdl, k_adj_stress<G, MEM, false>, adj_cells(c, ks), nt, 0, c->stream, p, a, ks);
     if (law) {
-        launch_pdl(c->use_pdl, k_adj_eta<true>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
+        launch_pdl(c->use_pdl, k_adj_eta<MEM, true>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
         launch_pdl(c->use_pdl, k_adj_collect, grid_cells(c->d), blk2d(), 0, c->stream, p, a);
         launch_pdl(c->use_pdl, k_adj_law<G>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
     } else if (!MEM) {
-        launch_pdl(c->use_pdl, k_adj_eta<false>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
+        launch_pdl(c->use_pdl, k_adj_eta<false, false>, adj_cells(c, kl), nt, 0, c->stream, p, a, kl);
     }
     const long long nodes = (long long)(c->d.n1 + 1) * (c->d.n2 + 1);
     const int kn = march_chunk(nodes, c->d.n3 + 1, c->sms, 0.6, 8.0);
