@@ -189,8 +189,7 @@ __global__ void __launch_bounds__(MC_NT) k_adj_stress(const __grid_constant__ KP
             D11 = e2 * s11; D22 = e2 * s22; D33 = e2 * s33;
             a.aP[c] = aP;
             a.gEta[c] = 2.0 * fma(s11, a.c11[c], fma(s22, a.c22[c], s33 * a.c33[c]));
-            if (G != CART) a.gRho[c] = -0.5 * p.g * (A0 + A1);
-            else a.gRho[c] = -0.5 * p.g * (Z0 + Z1);
+            if (a.gRho) a.gRho[c] = -0.5 * p.g * (G != CART ? A0 + A1 : Z0 + Z1);
         }
         a.d11[c] = D11; a.d22[c] = D22; a.d33[c] = D33;
         if (!LAW) cell_out<G>(m, d1, a, c, D11, D22, D33, lP);
@@ -478,19 +477,18 @@ __global__ void __launch_bounds__(256) k_adj_velocity_update(const __grid_consta
     if (i <= d.n1 - 2 && j <= d.n2 - 2) lV3[c] += (a.aV3[c] - bV3[c]) * ((p.DT_R[c - sz] + p.DT_R[c]) * h);
 }
 
-// residual of the transposed system, r = Aᵀλ - b (convergence check)
-__global__ void __launch_bounds__(256) k_adj_residual(KP<double> p, Adj a, const double* bV1, const double* bV2, const double* bV3,
-                                                      const double* bP, double* rV1, double* rV2, double* rV3, double* rP) {
+// residual of the transposed system, r = Aᵀλ - b, in place of Aᵀλ (convergence check)
+__global__ void __launch_bounds__(256) k_adj_residual(KP<double> p, Adj a, const double* bV1, const double* bV2, const double* bV3, const double* bP) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     const Dims& d = p.d;
     if (i > d.n1 || j > d.n2 || k > d.n3) return;
     const int sy = d.sy, sz = d.sz;
     const int c = i + sy * j + sz * k;
     const bool in1 = i >= 1 && i <= d.n1 - 1, in2 = j >= 1 && j <= d.n2 - 1, in3 = k >= 1 && k <= d.n3 - 1;
-    rV1[c] = (in1 && in2 && in3 && j <= d.n2 - 2 && k <= d.n3 - 2) ? a.aV1[c] - bV1[c] : 0.0;
-    rV2[c] = (in1 && in2 && in3 && i <= d.n1 - 2 && k <= d.n3 - 2) ? a.aV2[c] - bV2[c] : 0.0;
-    rV3[c] = (in1 && in2 && in3 && i <= d.n1 - 2 && j <= d.n2 - 2) ? a.aV3[c] - bV3[c] : 0.0;
-    rP[c] = (i < d.n1 && j < d.n2 && k < d.n3) ? a.aP[c] - bP[c] : 0.0;
+    a.aV1[c] = (in1 && in2 && in3 && j <= d.n2 - 2 && k <= d.n3 - 2) ? a.aV1[c] - bV1[c] : 0.0;
+    a.aV2[c] = (in1 && in2 && in3 && i <= d.n1 - 2 && k <= d.n3 - 2) ? a.aV2[c] - bV2[c] : 0.0;
+    a.aV3[c] = (in1 && in2 && in3 && i <= d.n1 - 2 && j <= d.n2 - 2) ? a.aV3[c] - bV3[c] : 0.0;
+    a.aP[c] = (i < d.n1 && j < d.n2 && k < d.n3) ? a.aP[c] - bP[c] : 0.0;
 }
 
 }  // namespace sph

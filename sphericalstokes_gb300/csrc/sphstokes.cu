@@ -128,7 +128,7 @@ struct Ctx {
     bool chunk_fixed = false;  // by SPH_FUSED_CHUNK: in batches too
     int sms = 152;
     int fused_slots = 0; // resident blocks of the fused TMA sweep on the device (SMs x blocks per SM)
-    double* adj = nullptr;  // adjoint arrays (AJ_COUNT slots of the box), allocated on first use
+    double* adj = nullptr;  // adjoint arrays (AJ_STATE slots of the box), allocated on first use
     // per-launch timing of the fused sweep kernel (sph_sweep_profile): event pairs
     // recorded around each launch while prof_next < prof_ev.size()/2
     std::vector<cudaEvent_t> prof_ev;
@@ -2147,25 +2147,41 @@ static int write_file(const std::string& path, const void* data, size_t bytes) {
 
 // ---------------------------------------------------------------------------
 // adjoint of the FP64 residual (sph_adjoint.cuh)
+//
+// Arrays of an adjoint call.  Those before AJ_STATE are its own, allocated by the first call; the others, which no
+// call leaves for the next, lie in boxes of the FP64 state that hold nothing between calls (adj_state_slot).
 enum AdjSlot {
-    AJ_LV1, AJ_LV2, AJ_LV3, AJ_LP, AJ_V1, AJ_V2, AJ_V3, AJ_P, AJ_GETA, AJ_GRHO, AJ_B1, AJ_B2, AJ_B3, AJ_BP, AJ_R1, AJ_R2, AJ_R3, AJ_RP, AJ_ETA,
-    AJ_GEI, AJ_GN, AJ_M11, AJ_M22, AJ_M33, AJ_M12, AJ_M13, AJ_M23,  // memory of the transposed PT
-    AJ_D11, AJ_D22, AJ_D33, AJ_E12, AJ_E13, AJ_E23,                 // adjoints of the strain rates (no memory)
-    AJ_X12, AJ_X13, AJ_X23, AJ_Q12, AJ_Q13, AJ_Q23, AJ_O1, AJ_O2, AJ_O3, AJ_O4, AJ_O5, AJ_GW,
-    AJ_WC, AJ_IE, AJ_Y12, AJ_Y13, AJ_Y23, AJ_W12, AJ_W13, AJ_W23, AJ_C11, AJ_C22, AJ_C33, AJ_G12, AJ_G13, AJ_G23,
-    AJ_LW, AJ_LR, AJ_LA, AJ_LB, AJ_LC, AJ_COUNT
+    AJ_LV1, AJ_LV2, AJ_LV3, AJ_LP, AJ_V1, AJ_V2, AJ_V3, AJ_P, AJ_GETA, AJ_B1, AJ_B2, AJ_B3, AJ_BP, AJ_ETA, AJ_GEI, AJ_GN,
+    AJ_M11, AJ_M22, AJ_M33, AJ_M12, AJ_M13, AJ_M23,  // memory of the transposed PT
+    AJ_D22, AJ_D33, AJ_E12, AJ_E13, AJ_E23,          // adjoints of the strain rates (no memory)
+    AJ_Q12, AJ_Q13, AJ_Q23, AJ_G12, AJ_G13, AJ_G23,
+    AJ_STATE,
+    AJ_D11 = AJ_STATE, AJ_O1, AJ_O2, AJ_O3, AJ_O4, AJ_O5, AJ_Y12, AJ_Y13, AJ_Y23, AJ_LC,
+    AJ_C11, AJ_C22, AJ_C33, AJ_W12, AJ_W13, AJ_W23, AJ_WC, AJ_IE, AJ_LW, AJ_LR, AJ_LA, AJ_LB,
+    AJ_COUNT,
+    AJ_X12 = AJ_Q12, AJ_X13 = AJ_Q13, AJ_X23 = AJ_Q23,  // k_adj_law writes them after k_adj_eta, the last reader of the others
+    AJ_GW = AJ_GEI,                                     // (k_adj_law_params comes last)
+    AJ_GRHO = AJ_M11                                    // sph_residual_vjp only, which has no memory
 };
+// Box of the FP64 state that holds slot s: the second copy of the PT state (the ping-pong of the FP32 sweeps) and scratch
+// of the residual, the exit check and the viscosity law.  Arrays of edges lie where a field of those edges does, so that the
+// entries past a field's extent stay zero.
+static int adj_state_slot(int s) {
+    static const int box[AJ_COUNT - AJ_STATE] = {F_A_P, F_A_V1, F_A_V2, F_A_V3, F_A_T11, F_A_T22, F_A_T12, F_A_T13, F_A_T23, F_A_T33,
+                                                 F_Q11, F_Q22, F_Q33, F_Q12, F_Q13, F_Q23, F_PRES, F_RP, F_ETA_OUT, F_V1E, F_V2E, F_V3E};
+    return box[s - AJ_STATE];
+}
 
 static int adj_alloc(Ctx* c) {
     if (c->prm.bc == SPH_BC_FREE_SURFACE)  // no transposed free-surface BC or top-cell pressure
         return fail(SPH_ERR_UNSUPPORTED, "the adjoint is not built for SPH_BC_FREE_SURFACE");
     if (c->adj) return SPH_OK;
-    const size_t b = sizeof(double) * (size_t)c->d.vol * AJ_COUNT;
+    const size_t b = sizeof(double) * (size_t)c->d.vol * AJ_STATE;
     if (cudaMalloc((void**)&c->adj, b) != cudaSuccess) return fail(SPH_ERR_NOMEM, "adjoint arrays");
     CK(cudaMemsetAsync(c->adj, 0, b, c->stream));
     return SPH_OK;
 }
-static double* adj_slot(Ctx* c, int s) { return c->adj + (size_t)s * c->d.vol; }
+static double* adj_slot(Ctx* c, int s) { return s < AJ_STATE ? c->adj + (size_t)s * c->d.vol : c->s64.f[adj_state_slot(s)]; }
 
 // host array with a field's extent (reference layout) <-> an adjoint slot; NULL host: zero
 static int adj_upload(Ctx* c, int slot, int field, const double* host) {
@@ -2205,17 +2221,17 @@ static KP<double> adj_kp(Ctx* c) {
     return p;
 }
 
-// mem: the iteration of the transposed solve (adjoints of the strain rates are the memory)
-static Adj adj_ptrs(Ctx* c, bool mem) {
+// mem: the iteration of the transposed solve (adjoints of the strain rates are the memory); rho: ∂R/∂ρ too
+static Adj adj_ptrs(Ctx* c, bool mem, bool rho) {
     auto s = [&](int i) { return adj_slot(c, i); };
     Adj a;
     a.lV1 = s(AJ_LV1); a.lV2 = s(AJ_LV2); a.lV3 = s(AJ_LV3); a.lP = s(AJ_LP); a.bP = s(AJ_BP);
-    const int d = mem ? AJ_M11 : AJ_D11;
-    a.d11 = s(d); a.d22 = s(d + 1); a.d33 = s(d + 2); a.e12 = s(d + 3); a.e13 = s(d + 4); a.e23 = s(d + 5);
+    a.d11 = s(mem ? AJ_M11 : AJ_D11); a.d22 = s(mem ? AJ_M22 : AJ_D22); a.d33 = s(mem ? AJ_M33 : AJ_D33);
+    a.e12 = s(mem ? AJ_M12 : AJ_E12); a.e13 = s(mem ? AJ_M13 : AJ_E13); a.e23 = s(mem ? AJ_M23 : AJ_E23);
     a.x12 = s(AJ_X12); a.x13 = s(AJ_X13); a.x23 = s(AJ_X23); a.q12 = s(AJ_Q12); a.q13 = s(AJ_Q13); a.q23 = s(AJ_Q23);
     a.E1 = s(AJ_O1); a.M1 = s(AJ_O2); a.E2 = s(AJ_O3); a.M2 = s(AJ_O4); a.E3 = s(AJ_O5);
     a.aV1 = s(AJ_V1); a.aV2 = s(AJ_V2); a.aV3 = s(AJ_V3); a.aP = s(AJ_P);
-    a.gEta = s(AJ_GETA); a.gRho = s(AJ_GRHO); a.gW = s(AJ_GW);
+    a.gEta = s(AJ_GETA); a.gRho = rho ? s(AJ_GRHO) : nullptr; a.gW = s(AJ_GW);
     a.wc = s(AJ_WC); a.ie = s(AJ_IE);
     a.y12 = s(AJ_Y12); a.y13 = s(AJ_Y13); a.y23 = s(AJ_Y23); a.w12 = s(AJ_W12); a.w13 = s(AJ_W13); a.w23 = s(AJ_W23);
     a.c11 = s(AJ_C11); a.c22 = s(AJ_C22); a.c33 = s(AJ_C33); a.g12 = s(AJ_G12); a.g13 = s(AJ_G13); a.g23 = s(AJ_G23);
@@ -2244,7 +2260,7 @@ static void adj_bc(Ctx* c, const KP<double>& p, const Adj& a) {
 // the fixed factors of the state behind p (after adj_kp)
 template <int G>
 static void adj_setup(Ctx* c, const KP<double>& p) {
-    const Adj a = adj_ptrs(c, false);
+    const Adj a = adj_ptrs(c, false, false);
     if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX) k_adj_setup<G, true><<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a);
     else k_adj_setup<G, false><<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a);
 }
@@ -2272,11 +2288,11 @@ static void adj_rows(Ctx* c, const KP<double>& p, const Adj& a) {
     launch_pdl(c->use_pdl, k_adj_strain<G>, gn, nt, 0, c->stream, p, a, x12, x13, x23, kn);
 }
 
-// Aᵀ λ (λ in the AJ_L* slots) into AJ_V*, AJ_P, with ∂R/∂η, ∂R/∂ρ contractions; with_bc: the
+// Aᵀ λ (λ in the AJ_L* slots) into AJ_V*, AJ_P, with ∂R/∂η and (rho) ∂R/∂ρ contractions; with_bc: the
 // transposed homogeneous BC program (interior-unknown form)
 template <int G>
-static int adj_apply(Ctx* c, KP<double>& p, bool with_bc) {
-    const Adj a = adj_ptrs(c, false);
+static int adj_apply(Ctx* c, KP<double>& p, bool with_bc, bool rho) {
+    const Adj a = adj_ptrs(c, false, rho);
     adj_rows<G, false>(c, p, a);
     if (c->prm.rheology == SPH_RHEO_EDOT_POWER_RELAX)
         k_adj_law_params<<<adj_cells(c, 1), MC_NT, 0, c->stream>>>(p, a, adj_slot(c, AJ_GEI), adj_slot(c, AJ_GN));
@@ -2291,7 +2307,7 @@ template <int G>
 static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf) {
     KP<double> p = adj_kp<G>(c);
     adj_setup<G>(c, p);
-    const Adj a = adj_ptrs(c, true);
+    const Adj a = adj_ptrs(c, true, false);
     const int nout = o.nout > 0 ? o.nout : 100;
     // max|b|
     auto max4 = [&](int f) {
@@ -2317,10 +2333,9 @@ static int adjoint_solve_g(Ctx* c, const sph_solve_opts& o, sph_solve_info* inf)
                    adj_slot(c, AJ_LV3), adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3));
         if (it % nout) continue;
         // convergence: the transposed residual Aᵀλ - b of the current λ
-        if ((rc = adj_apply<G>(c, p, true))) return rc;
-        k_adj_residual<<<gu, blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3), adj_slot(c, AJ_BP),
-                                                      adj_slot(c, AJ_R1), adj_slot(c, AJ_R2), adj_slot(c, AJ_R3), adj_slot(c, AJ_RP));
-        if ((rc = max4(AJ_R1))) return rc;
+        if ((rc = adj_apply<G>(c, p, true, false))) return rc;
+        k_adj_residual<<<gu, blk2d(), 0, c->stream>>>(p, a, adj_slot(c, AJ_B1), adj_slot(c, AJ_B2), adj_slot(c, AJ_B3), adj_slot(c, AJ_BP));
+        if ((rc = max4(AJ_V1))) return rc;
         double r = 0.0;
         for (int s = 0; s < 4; ++s) r = std::max(r, slot_val(*c, s));
         err = r / bmax;
@@ -2498,9 +2513,9 @@ int sph_residual_vjp(void* h, const double* lV1, const double* lV2, const double
         return rc;
     const int G = c->prm.geometry;
     const bool bc = (flags & 1) != 0;
-    if (G == SPH) { KP<double> p = adj_kp<SPH>(c); adj_setup<SPH>(c, p); rc = adj_apply<SPH>(c, p, bc); }
-    else if (G == CYL) { KP<double> p = adj_kp<CYL>(c); adj_setup<CYL>(c, p); rc = adj_apply<CYL>(c, p, bc); }
-    else { KP<double> p = adj_kp<CART>(c); adj_setup<CART>(c, p); rc = adj_apply<CART>(c, p, bc); }
+    if (G == SPH) { KP<double> p = adj_kp<SPH>(c); adj_setup<SPH>(c, p); rc = adj_apply<SPH>(c, p, bc, true); }
+    else if (G == CYL) { KP<double> p = adj_kp<CYL>(c); adj_setup<CYL>(c, p); rc = adj_apply<CYL>(c, p, bc, true); }
+    else { KP<double> p = adj_kp<CART>(c); adj_setup<CART>(c, p); rc = adj_apply<CART>(c, p, bc, true); }
     if (rc) return rc;
     if ((rc = adj_download(c, AJ_V1, SPH_FIELD_V1, aV1)) || (rc = adj_download(c, AJ_V2, SPH_FIELD_V2, aV2)) ||
         (rc = adj_download(c, AJ_V3, SPH_FIELD_V3, aV3)) || (rc = adj_download(c, AJ_P, SPH_FIELD_P, aP)) ||
@@ -2522,7 +2537,7 @@ int sph_advect(void* h, double dt, double delta, int32_t nf, const double* const
     for (int f = 0; f < nf; ++f) {
         if ((rc = adj_upload(c, AJ_B1 + f, SPH_FIELD_P, phi[f]))) return rc;
         F.in[f] = adj_slot(c, AJ_B1 + f);
-        F.out[f] = adj_slot(c, AJ_R1 + f);
+        F.out[f] = adj_slot(c, AJ_LV1 + f);
     }
     KP<double> p = make_kp<double>(*c, c->s64);
     const int G = c->prm.geometry;
@@ -2531,7 +2546,7 @@ int sph_advect(void* h, double dt, double delta, int32_t nf, const double* const
     else k_advect<CART><<<grid_cells(c->d), blk2d(), 0, c->stream>>>(p, F, dt, delta);
     CK(cudaGetLastError());
     for (int f = 0; f < nf; ++f)
-        if ((rc = adj_download(c, AJ_R1 + f, SPH_FIELD_P, phi_new[f]))) return rc;
+        if ((rc = adj_download(c, AJ_LV1 + f, SPH_FIELD_P, phi_new[f]))) return rc;
     return SPH_OK;
 }
 
@@ -2546,11 +2561,11 @@ int sph_advect_vjp(void* h, double dt, double delta, int32_t nf, const double* c
     AdvFields F, M;
     F.nf = M.nf = nf;
     for (int f = 0; f < nf; ++f) {
-        if ((rc = adj_upload(c, AJ_B1 + f, SPH_FIELD_P, phi[f])) || (rc = adj_upload(c, AJ_R1 + f, SPH_FIELD_P, mu_new[f])) ||
+        if ((rc = adj_upload(c, AJ_B1 + f, SPH_FIELD_P, phi[f])) || (rc = adj_upload(c, AJ_LV1 + f, SPH_FIELD_P, mu_new[f])) ||
             (rc = adj_upload(c, AJ_M11 + f, SPH_FIELD_P, nullptr)))
             return rc;
         F.in[f] = adj_slot(c, AJ_B1 + f);
-        M.in[f] = adj_slot(c, AJ_R1 + f);
+        M.in[f] = adj_slot(c, AJ_LV1 + f);
         M.out[f] = adj_slot(c, AJ_M11 + f);
     }
     for (int s = AJ_V1; s <= AJ_V3; ++s) CK(cudaMemsetAsync(adj_slot(c, s), 0, sizeof(double) * c->d.vol, c->stream));
@@ -2580,7 +2595,7 @@ int sph_bc_vjp(void* h, double* aV1, double* aV2, double* aV3) {
         return rc;
     KP<double> p = make_kp<double>(*c, c->s64);
     p.sig2 = 0.0; p.sig3 = 0.0;
-    const Adj a = adj_ptrs(c, false);
+    const Adj a = adj_ptrs(c, false, false);
     const int G = c->prm.geometry;
     if (G == SPH) adj_bc<SPH>(c, p, a);
     else if (G == CYL) adj_bc<CYL>(c, p, a);
@@ -2623,7 +2638,6 @@ int sph_adjoint_solve(void* h, const double* bV1, const double* bV2, const doubl
         (rc = adj_upload(c, AJ_LV1, SPH_FIELD_V1, lV1)) || (rc = adj_upload(c, AJ_LV2, SPH_FIELD_V2, lV2)) ||
         (rc = adj_upload(c, AJ_LV3, SPH_FIELD_V3, lV3)) || (rc = adj_upload(c, AJ_LP, SPH_FIELD_P, lP)))
         return rc;
-    for (int s = AJ_R1; s <= AJ_RP; ++s) CK(cudaMemsetAsync(adj_slot(c, s), 0, sizeof(double) * c->d.vol, c->stream));
     sph_solve_info local;
     std::memset(&local, 0, sizeof(local));
     sph_solve_info* inf = info ? info : &local;
