@@ -289,6 +289,9 @@ int sph_corr_set(void* ctx, int32_t field, const double* host, int64_t count);
  * time-out: SPH_ERR_CUDA, with the context marked unusable (every later call that launches
  * work on it fails with SPH_ERR_CUDA; destroy it).  No copy or fault is involved. */
 int sph_selftest_wait_timeout(void* ctx);
+/* The same without reading the error word: SPH_OK, and the next call that runs sweeps on this
+ * context reports the time-out. */
+int sph_selftest_wait_flag(void* ctx);
 
 /* MIXED only (no counterpart in the reference: measurement): k sweeps as sph_sweep,
  * launched one at a time with a CUDA event pair on the library's stream around each

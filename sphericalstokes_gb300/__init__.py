@@ -138,6 +138,7 @@ _SIGS = {
     "sph_corr_get": ([C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_int64], C.c_int),
     "sph_corr_set": ([C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_int64], C.c_int),
     "sph_selftest_wait_timeout": ([C.c_void_p], C.c_int),
+    "sph_selftest_wait_flag": ([C.c_void_p], C.c_int),
     "sph_solve_history_ms": ([C.c_void_p, C.POINTER(C.c_double), C.c_int64, C.POINTER(C.c_int64)], C.c_int),
 }
 

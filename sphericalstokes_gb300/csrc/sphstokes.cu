@@ -1063,6 +1063,31 @@ int download_box(Ctx& c, const T* box, const int e[3], double* host) {
 }
 
 // ---------------------------------------------------------------------------
+// The error word of the TMA sweep kernels: set when a bounded wait on a copy barrier ran
+// out.  The kernel then stopped issuing copies and finished its march on whatever its
+// tiles held, so the FP32 state is suspect and copies may have been in flight when its
+// blocks exited: the context is marked unusable (every later call that would launch work
+// on it fails) and the caller destroys it.
+int check_kernel_flag(Ctx& c) {
+    if (!c.d_err) return SPH_OK;
+    int h = 0;
+    CK(cudaMemcpyAsync(&h, c.d_err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+    if (h) {
+        c.broken = true;
+        return fail(SPH_ERR_CUDA, "a bounded wait on a TMA barrier ran out in the fused sweep; the context is unusable");
+    }
+    return SPH_OK;
+}
+
+// SPH_OK, or the failure every entry point that launches work returns on a context
+// marked unusable by check_kernel_flag
+int usable(const Ctx& c) {
+    if (c.broken) return fail(SPH_ERR_CUDA, "context unusable: a bounded wait of a sweep kernel ran out earlier; destroy it");
+    return SPH_OK;
+}
+
+// ---------------------------------------------------------------------------
 // plain PT solve (FP64 or FP32 state)
 template <typename T>
 int solve_plain(Ctx& c, State<T>& s, bool is32, const sph_solve_opts& o, sph_solve_info* info, int64_t* hi, double* he, int64_t cap) {
@@ -1092,6 +1117,7 @@ int solve_plain(Ctx& c, State<T>& s, bool is32, const sph_solve_opts& o, sph_sol
             if (rc) return rc;
             err = out[6];
         }
+        if (is32) { int rc = check_kernel_flag(c); if (rc) return rc; }
         if (info && info->nhist < cap) {
             if (hi) hi[info->nhist] = it;
             if (he) he[info->nhist] = err;
@@ -1102,6 +1128,7 @@ int solve_plain(Ctx& c, State<T>& s, bool is32, const sph_solve_opts& o, sph_sol
         if (c.prm.switch_err > 0.0 && err < c.prm.switch_err) c.cur_n = c.prm.n_exp_late;
         if (err < o.tol && (!ref || it > 20)) { status = SPH_OK; break; }
     }
+    if (is32 && it % nout) { int rc = check_kernel_flag(c); if (rc) return rc; }
     if (info) { info->iters = it; info->err = err; info->status = status; }
     return SPH_OK;
 }
@@ -1153,30 +1180,6 @@ int prepare_correction(Ctx& c, const double out[7]) {
 }
 
 // ---------------------------------------------------------------------------
-// The error word of the TMA sweep kernels: set when a bounded wait on a copy barrier ran
-// out.  The kernel then stopped issuing copies and finished its march on whatever its
-// tiles held, so the FP32 state is suspect and copies may have been in flight when its
-// blocks exited: the context is marked unusable (every later call that would launch work
-// on it fails) and the caller destroys it.
-int check_kernel_flag(Ctx& c) {
-    if (!c.d_err) return SPH_OK;
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, c.d_err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
-    if (h) {
-        c.broken = true;
-        return fail(SPH_ERR_CUDA, "a bounded wait on a TMA barrier ran out in the fused sweep; the context is unusable");
-    }
-    return SPH_OK;
-}
-
-// SPH_OK, or the failure every entry point that launches work returns on a context
-// marked unusable by check_kernel_flag
-int usable(const Ctx& c) {
-    if (c.broken) return fail(SPH_ERR_CUDA, "context unusable: a bounded wait of a sweep kernel ran out earlier; destroy it");
-    return SPH_OK;
-}
-
 // KP of the correction problem: homogeneous boundary data
 KP<float> make_kp_corr(Ctx& c) {
     KP<float> q = make_kp<float>(c, c.s32);
@@ -1382,6 +1385,7 @@ int solve_mixed_g(Ctx& c, const sph_solve_opts& o, sph_solve_info* info, int64_t
             if (!(werr == werr) || std::isinf(werr)) { warm_ok = false; break; }
             if (werr < o.warm_tol && iters > 20) break;
         }
+        if ((rc = check_kernel_flag(c))) return rc;
         if (warm_ok) {  // widen V, P (η is recomputed from the law)
             k_convert<double, float><<<ew_blocks(vol), 256, 0, c.stream>>>(s.f[F_V1], t.f[F_V1], vol);
             k_convert<double, float><<<ew_blocks(vol), 256, 0, c.stream>>>(s.f[F_V2], t.f[F_V2], vol);
@@ -2392,7 +2396,7 @@ int sph_step(void* h, int64_t k) {
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     c->last_ms = ms;
     if (use32) c->stale64 = true;
-    return SPH_OK;
+    return use32 ? check_kernel_flag(*c) : SPH_OK;
 }
 
 int sph_solve(void* h, const sph_solve_opts* o, sph_solve_info* info, int64_t* hist_iter, double* hist_err, int64_t hist_cap) {
@@ -2838,7 +2842,7 @@ int sph_corr_set(void* h, int32_t field, const double* host, int64_t count) {
     return corr_access(h, field, nullptr, host, count);
 }
 
-int sph_selftest_wait_timeout(void* h) {
+int sph_selftest_wait_flag(void* h) {
     Ctx* c = static_cast<Ctx*>(h);
     if (!c) return fail(SPH_ERR_INVALID, "ctx is NULL");
     if (int rc_ = usable(*c)) return rc_;
@@ -2849,7 +2853,12 @@ int sph_selftest_wait_timeout(void* h) {
     // 1000 polls of at most 1 us each: the wait runs out within a few milliseconds
     k_wait_selftest<<<1, 32, 0, c->stream>>>(c->d_err, 1000, 1000u);
     CK(cudaGetLastError());
-    return check_kernel_flag(*c);
+    return SPH_OK;
+}
+
+int sph_selftest_wait_timeout(void* h) {
+    const int rc = sph_selftest_wait_flag(h);
+    return rc ? rc : check_kernel_flag(*static_cast<Ctx*>(h));
 }
 
 int sph_residual(void* h, double out[7]) {
