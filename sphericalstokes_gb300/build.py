@@ -46,7 +46,7 @@ def _stale(target: Path, sources: list[Path]) -> bool:
 
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:
-    sources = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + [ROOT / "include" / "sphstokes.h"]
+    sources = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "sphstokes.h"]
     if not force and not _stale(LIB, sources):
         return LIB
     cmd = [_nvcc(), *NVCC_FLAGS, f"-I{ROOT / 'include'}", "-o", str(LIB) + ".tmp", str(CSRC / "sphstokes.cu")]
