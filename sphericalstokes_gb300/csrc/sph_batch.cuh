@@ -32,6 +32,8 @@ struct BatchSweep {
 // blocks of a small batch fill the SMs together (12 grids of 31 .. 47 cells a side, 600 sweeps with the
 // FP64 steps and copies: 50.8 ms with a launch per geometry and each solve's own chunk, 39.2 ms so, 26.6 ms with
 // the sweep of now and blocks of one geometry on an SM).
+// LIFT: if any solve has small viscosities (the others' results do not change).
+template <bool LIFT>
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __restrict__ b, const int4* __restrict__ items,
                                                           const int* __restrict__ active, const int* __restrict__ kchunk, int a) {
     // (items, flags and entries change between launches of the whole round only)
@@ -55,9 +57,9 @@ __global__ void __launch_bounds__(SW_NT, 2) k_sweep_batch(const BatchSweep* __re
         for (int i = 0; i < SM_COUNT; ++i)
             asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(s.maps[a].m + i) : "memory");
     const int kc = kchunk[it.x];
-    if (s.geom == SPH) sweep_body<SPH, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
-    else if (s.geom == CYL) sweep_body<CYL, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
-    else sweep_body<CART, 1>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
+    if (s.geom == SPH) sweep_body<SPH, 1, LIFT>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
+    else if (s.geom == CYL) sweep_body<CYL, 1, LIFT>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
+    else sweep_body<CART, 1, LIFT>(p, o, kc, s.maps[a].m, s.err, it.y, it.z, it.w);
 }
 
 // inner stopping test of every active solve: max |dV + rV| of arrangement 0 into red[solve];

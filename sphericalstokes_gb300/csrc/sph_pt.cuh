@@ -502,14 +502,15 @@ __device__ __forceinline__ void block_max_to(unsigned long long v, unsigned long
     }
 }
 
-// The maxima of up to 7 fields in one launch, field blockIdx.y: max|a| into red[slot], and max|a - b| into
-// red[slot_d] where there is a b.  A launch per maximum and per snapshot copy cost a check as much as several iterations
+// The maxima of up to 8 fields in one launch, field blockIdx.y: max|a| into red[slot], and max|a - b| into
+// red[slot_d] where there is a b; slot_d = kLeast: the least positive a, as the greatest of its inverted bits.  A launch per maximum and per snapshot copy cost a check as much as several iterations
 // of a small grid: 200 FP64 iterations at 70 x 5 x 5 with a check every 10 took 4.24 ms with them, 3.42 with this
 // and k_copy3; the FP64 residual of a 47 x 31 x 39 grid 73 and 37 us.
 template <typename T>
 struct MaxItem { const T *a, *b; int slot, slot_d; };
 template <typename T>
-struct MaxList { MaxItem<T> f[7]; };
+struct MaxList { MaxItem<T> f[8]; };
+constexpr int kLeast = -1;
 template <typename T>
 __global__ void __launch_bounds__(256) k_maxabs(const __grid_constant__ MaxList<T> list, long long n, unsigned long long* red) {
     pdl_enter_small();
@@ -518,6 +519,11 @@ __global__ void __launch_bounds__(256) k_maxabs(const __grid_constant__ MaxList<
     unsigned long long m = 0ULL, e = 0ULL;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
         const T x = a[q];
+        if (f.slot_d == kLeast) {
+            const long long v = __double_as_longlong((double)x);
+            m = umax64(m, v > 0 ? ~(unsigned long long)v : 0ULL);
+            continue;
+        }
         m = umax64(m, ord_bits((double)x));
         if (b) e = umax64(e, ord_bits((double)x - (double)b[q]));
     }

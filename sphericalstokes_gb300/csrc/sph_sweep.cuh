@@ -75,6 +75,7 @@ struct SweepOut {
     // divergence-free; it is not stored but evaluated where the next sweep reads it.
     int gmask, smask;
     float gf[9];
+    float small;  // 2^-126 / min(1, GSDT/ηSM, KBDT/ηSM)
     // scalars of the sweep as pairs (operands of the paired instructions straight from constant memory)
     float2 d1, d1q, d2, gsc, kbc, nkbc, vp, third, half;  // d1, d1 / 4, d2, GSDT/ηSM, ±KBDT/ηSM, vpdt² / 2, -1/3, -1/2
 };
@@ -149,6 +150,14 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 __device__ __forceinline__ float2 div2(float2 a, float2 b) { return __fmul2_rn(a, make_float2(rcp_approx(b.x), rcp_approx(b.y))); }
+// The divisors of the sweep are GSDT, KBDT or more: subnormal only where ηSM is below `small` (SweepOut).  LIFT: there both
+// operands are multiplied by 2^24 first, which changes no other bit of a quotient.
+template <bool LIFT>
+__device__ __forceinline__ float2 div2(float2 a, float2 b, float2 etaSM, float small) {
+    if (!LIFT) return div2(a, b);
+    const float2 c = make_float2(etaSM.x < small ? 16777216.f : 1.f, etaSM.y < small ? 16777216.f : 1.f);
+    return div2(mul2(a, c), mul2(b, c));
+}
 __device__ __forceinline__ float2 keep2(float2 x, bool m0, bool m1) { return make_float2(m0 ? x.x : 0.f, m1 ? x.y : 0.f); }
 
 // stores at a 32-bit unsigned byte offset from a field's base: the address is the
@@ -272,7 +281,10 @@ __device__ __forceinline__ void sweep_fill_ghosts(const KP<float>* pp, int smask
     }
 }
 // maps: tensor maps among the launch's parameters, or in global memory after a tensor-map fence
-template <int G, int MODE>
+// LIFT: divisors may be subnormal (div2).  MODE 1 has fixed η and its least one is known to the host (Ctx::small32); the η of
+// MODE 0 changes, and it always lifts.  us per sweep without and with: 63^3 11.80 and 12.07, 255^3 304.4 and 309.0 (by a branch to __fdividef 12.20
+// and 317.1; both marches in one kernel, chosen by a word in memory, 12.19 and 307.7).
+template <int G, int MODE, bool LIFT>
 __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<float>& o, int kchunk, const CUtensorMap* __restrict__ maps,
                                            int* __restrict__ err, int bx, int by, int bz) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -480,7 +492,7 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
                 D22 = mul2(C.a2, e2); D33 = mul2(C.a3, e3);
             }
             const float2 gs = mul2(o.gsc, n.sP), kb = mul2(o.kbc, n.sP);
-            const float2 f = div2(n.eP, add2(n.eP, gs));
+            const float2 f = div2<LIFT>(n.eP, add2(n.eP, gs), n.sP, o.small);
             const float2 gs2 = add2(gs, gs);
             if (MODE == 1) div = add2(div, old(S.rp[so], 0));
             vP = fma2(mul2(o.nkbc, n.sP), div, old(S.P[so], 0));
@@ -500,12 +512,14 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
                     set(vP, l, P);
                 }
             }
-            vdt = div2(o.vp, fma2(gs, f, kb));
+            vdt = div2<LIFT>(o.vp, fma2(gs, f, kb), n.sP, o.small);
         }
+        float2 st = dup(0.f);  // LIFT: ηSM of the cell that all three edges have in common
         auto sums = [&](const float* A, float2& P, float2& X0, float2& X, float2& Y) {
             P = ldP(A, 0);
             const float2 s = ldS(A, 0, P), q = ldP(A, 1), t = ldS(A, 1, q);
             X0 = add2(P, s); X = add2(q, t); Y = add2(s, t);
+            if (LIFT) st = t;
         };
         float2 eX0, sX0;
         sums(B + 3 * SI_N, m.eP, eX0, m.eX, m.eY);
@@ -514,7 +528,7 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
         // (τ + aG D) aE / (aE + aG) with D4 = D / 4
         auto edge = [&](float2 told, float2 s4, float2 e4, float2 D4) {
             const float2 g4 = mul2(o.gsc, s4);
-            return mul2(fma2(g4, D4, told), div2(e4, add2(e4, g4)));
+            return mul2(fma2(g4, D4, told), div2<LIFT>(e4, add2(e4, g4), st, o.small));
         };
         const float2 b1T = ld2(B, 1), b2T = ld2(B2, 1), b3Q = ldP(B3, 1), b3T = ldS(B3, 1, b3Q);
         {
@@ -709,10 +723,10 @@ __device__ __forceinline__ void sweep_body(const KP<float>& p, const SweepOut<fl
     if (halo && !ok && err) atomicExch(err, 1);
 }
 
-template <int G, int MODE>
+template <int G, int MODE, bool LIFT>
 __global__ void __launch_bounds__(SW_NT, 2) k_sweep(const __grid_constant__ KP<float> p, const __grid_constant__ SweepOut<float> o, int kchunk,
                                                     const __grid_constant__ SweepMaps maps, int* __restrict__ err) {
-    sweep_body<G, MODE>(p, o, kchunk, maps.m, err, blockIdx.x, blockIdx.y, blockIdx.z);
+    sweep_body<G, MODE, LIFT>(p, o, kchunk, maps.m, err, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 }  // namespace sph

@@ -99,6 +99,8 @@ struct Ctx {
     bool ghost_fuse = true;
     int ghost_gmask = 0, ghost_smask = 0;
     float ghost_gf[9] = {};
+    // divisors of the sweeps may be subnormal: at the η of the last FP64 residual, of the prepared correction problem
+    bool small_eta = false, small32 = false;
     bool ghost_stored = false;  // the next sweep reads the stored ghosts (after sph_corr_set)
     double cur_n = 1.0;
     double f_scale = 1.0;
@@ -197,6 +199,14 @@ void power_form(bool strain_rate, double n, int* p, int* q) {
     static const int form[4][2] = {{1, 4}, {1, 3}, {3, 8}, {2, 5}};
     for (int k = 0; k < 4; ++k)
         if (n == k + 2.0) { *p = form[k][0]; *q = form[k][1]; }
+}
+
+// the sweeps' error word
+int alloc_err(Ctx& c) {
+    if (c.d_err) return SPH_OK;
+    if (cudaMalloc((void**)&c.d_err, sizeof(int)) != cudaSuccess) return fail(SPH_ERR_NOMEM, "error word");
+    CK(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
+    return SPH_OK;
 }
 
 template <typename T>
@@ -738,10 +748,6 @@ const SweepMaps* tma_maps(Ctx& c) {
     for (; slot < 4 && c.map_key[slot][0]; ++slot)
         if (c.map_key[slot][0] == t.f[F_V1] && c.map_key[slot][1] == t.f[F_ETA]) return &c.maps[slot];
     if (slot == 4) return nullptr;
-    if (!c.d_err) {
-        if (cudaMalloc((void**)&c.d_err, sizeof(int)) != cudaSuccess) { c.use_tma = false; return nullptr; }
-        cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream);
-    }
     CUtensorMap* h = c.maps[slot].m;
     bool ok = encode_map(c, &h[SM_V], t.f[F_V1], 3, SI_X, SI_Y);
     ok &= encode_map(c, &h[SM_ETA], t.f[F_ETA], 1, SI_X, SI_Y);
@@ -775,14 +781,16 @@ void set_sweep_attrs() {
     const int f = (int)fused_smem_bytes(), w = (int)sweep_smem_bytes();
     cudaFuncSetAttribute(k_fused<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
     cudaFuncSetAttribute(k_fused<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
-    cudaFuncSetAttribute(k_sweep<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
-    cudaFuncSetAttribute(k_sweep<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
+    cudaFuncSetAttribute(k_sweep<G, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
+    cudaFuncSetAttribute(k_sweep<G, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
+    cudaFuncSetAttribute(k_sweep<G, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, w);
 }
 int set_fused_attrs() {
     set_sweep_attrs<SPH>();
     set_sweep_attrs<CYL>();
     set_sweep_attrs<CART>();
-    cudaFuncSetAttribute(k_sweep_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem_bytes());
+    cudaFuncSetAttribute(k_sweep_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem_bytes());
+    cudaFuncSetAttribute(k_sweep_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem_bytes());
     CK(cudaGetLastError());
     return SPH_OK;
 }
@@ -796,6 +804,7 @@ SweepOut<float> sweep_out(const Ctx& c, const KP<float>& p, bool fill) {
     o.t11 = t.f[F_A_T11]; o.t22 = t.f[F_A_T22]; o.t33 = t.f[F_A_T33]; o.t12 = t.f[F_A_T12]; o.t13 = t.f[F_A_T13]; o.t23 = t.f[F_A_T23];
     auto pair = [](float x) { return make_float2(x, x); };
     o.d1 = pair(p.d1); o.d1q = pair(0.25f * p.d1); o.d2 = pair(p.d2); o.gsc = pair(p.gsc); o.kbc = pair(p.kbc); o.nkbc = pair(-p.kbc);
+    o.small = 0x1p-126f / std::min(1.f, std::min(p.gsc, p.kbc));
     o.vp = pair(0.5f * p.vpdt2); o.third = pair(-1.f / 3.f); o.half = pair(-0.5f);
     if (fill) {
         o.gmask = c.ghost_gmask;
@@ -812,7 +821,8 @@ bool launch_fused(Ctx& c, const KP<float>& p, bool fill) {
     const SweepMaps* maps = tma_maps(c);
     const int kc = fused_chunk(c, maps != nullptr);
     if (maps) {
-        launch_pdl(c.use_pdl, k_sweep<G, MODE>, sweep_grid(c.d, kc), dim3(SW_NT, 1, 1), sweep_smem_bytes(), c.stream, p, sweep_out(c, p, fill), kc, *maps, c.d_err);
+        auto k = MODE == 0 || c.small32 ? k_sweep<G, MODE, true> : k_sweep<G, MODE, MODE == 0>;
+        launch_pdl(c.use_pdl, k, sweep_grid(c.d, kc), dim3(SW_NT, 1, 1), sweep_smem_bytes(), c.stream, p, sweep_out(c, p, fill), kc, *maps, c.d_err);
         return fill;
     }
     dim3 grid((c.d.n1 + FTX - 1) / FTX, (c.d.n2 + FTY - 1) / FTY, (c.d.n3 + kc - 1) / kc);
@@ -937,11 +947,16 @@ int residual64_g(Ctx& c, double out[7], bool eta_from_law) {
     }
     launch_nodes<double, G, 2>(c, r);
     int rc = launch_maxabs<double>(c, {{s.f[F_RV1], nullptr, 0}, {s.f[F_RV2], nullptr, 1}, {s.f[F_RV3], nullptr, 2}, {s.f[F_RP], nullptr, 3},
-                                       {s.f[F_V1], nullptr, 4}, {s.f[F_V2], nullptr, 5}, {s.f[F_V3], nullptr, 6}});
+                                       {s.f[F_V1], nullptr, 4}, {s.f[F_V2], nullptr, 5}, {s.f[F_V3], nullptr, 6}, {eta_eff, nullptr, 7, kLeast}});
     if (rc) return rc;
     CK(cudaGetLastError());
     rc = fetch_red(c);
     if (rc) return rc;
+    // (ηSM is a maximum over η; twice the limit for the rounding to FP32)
+    const unsigned long long least = ~c.hred[7];
+    double eta_min;
+    std::memcpy(&eta_min, &least, sizeof(double));
+    c.small_eta = c.hred[7] && eta_min * std::min(1.0, std::min(p.gsc, p.kbc)) < 0x1p-125;
     for (int i = 0; i < 4; ++i) out[i] = slot_val(c, i);
     out[4] = std::max(slot_val(c, 4), std::max(slot_val(c, 5), slot_val(c, 6)));
     out[5] = c.f_scale;
@@ -1109,6 +1124,26 @@ int outer_residual(Ctx& c, double out[7]) {
     return residual64_g<G>(c, out, false);
 }
 
+// the captured launches of a context (correction sweeps, warm-start iterations): dropped
+// when the launch parameters they hold change
+void drop_graphs(Ctx& c) {
+    for (int i = 0; i < 2; ++i) {
+        if (c.corr_graph[i]) cudaGraphExecDestroy(c.corr_graph[i]);
+        c.corr_graph[i] = nullptr;
+        c.corr_graph_key[i] = nullptr;
+        if (c.warm_graph[i]) cudaGraphExecDestroy(c.warm_graph[i]);
+        c.warm_graph[i] = nullptr;
+        c.warm_key[i][0] = c.warm_key[i][1] = nullptr;
+    }
+    c.graph_len = 0;
+    c.warm_len = 0;
+}
+
+void set_small32(Ctx& c, bool small) {
+    if (small != c.small32) drop_graphs(c);  // they hold the other kernel
+    c.small32 = small;
+}
+
 // freeze η_eff, ηSM and the FP64 residual into the FP32 correction problem, zero δ
 template <int G>
 int prepare_correction(Ctx& c, const double out[7]) {
@@ -1128,6 +1163,7 @@ int prepare_correction(Ctx& c, const double out[7]) {
     CK(cudaGetLastError());
     c.corr_r0 = std::max(out[0], std::max(out[1], out[2]));
     c.corr_ready = true;
+    set_small32(c, c.small_eta);
     c.ghost_stored = false;
     c.stale32 = true;  // the FP32 state no longer mirrors the FP64 state
     return SPH_OK;
@@ -1243,21 +1279,6 @@ int ensure_correction(Ctx& c) {
     rc = G == SPH ? outer_residual<SPH>(c, out) : (G == CYL ? outer_residual<CYL>(c, out) : outer_residual<CART>(c, out));
     if (rc) return rc;
     return G == SPH ? prepare_correction<SPH>(c, out) : (G == CYL ? prepare_correction<CYL>(c, out) : prepare_correction<CART>(c, out));
-}
-
-// the captured launches of a context (correction sweeps, warm-start iterations): dropped
-// when the launch parameters they hold change
-void drop_graphs(Ctx& c) {
-    for (int i = 0; i < 2; ++i) {
-        if (c.corr_graph[i]) cudaGraphExecDestroy(c.corr_graph[i]);
-        c.corr_graph[i] = nullptr;
-        c.corr_graph_key[i] = nullptr;
-        if (c.warm_graph[i]) cudaGraphExecDestroy(c.warm_graph[i]);
-        c.warm_graph[i] = nullptr;
-        c.warm_key[i][0] = c.warm_key[i][1] = nullptr;
-    }
-    c.graph_len = 0;
-    c.warm_len = 0;
 }
 
 // n (even, >= 8) FP32 nonlinear iterations of the warm start as one graph launch; after an
@@ -1661,6 +1682,7 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
     CK(cudaMemsetAsync(dev.entries, 0, sizeof(BatchSweep) * n, dev.stream));
     if (int rc = build_lists()) return rc;
     std::vector<int> act((size_t)n, 0);
+    bool lift = false;
 
     // one round: nout sweeps of every active solve (arrangement a = s & 1 read by sweep s)
     auto capture = [&]() -> int {
@@ -1673,7 +1695,7 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             const BatchSweep* E = dev.entries;
             const int* act_d = dev.active;
             const int* kc_d = dev.kchunk;
-            launch_pdl(pdl, k_sweep_batch, dim3((unsigned)fz_n), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items, act_d, kc_d, a);
+            launch_pdl(pdl, lift ? k_sweep_batch<true> : k_sweep_batch<false>, dim3((unsigned)fz_n), dim3(SW_NT), sweep_smem_bytes(), dev.stream, E, dev.items, act_d, kc_d, a);
         }
         cudaError_t e = cudaStreamEndCapture(dev.stream, &g);
         if (e != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e));
@@ -1710,6 +1732,10 @@ int batch_lockstep(void* const* ctxs, int32_t n, const sph_solve_opts* opts, sph
             } else {
                 act[i] = 1;
                 any = true;
+                if (b.c->small32 && !lift) {  // the other kernel from here on
+                    lift = true;
+                    if (dev.graph) { CK(cudaStreamSynchronize(dev.stream)); cudaGraphExecDestroy(dev.graph); dev.graph = nullptr; }
+                }
             }
         }
         size_t open_solves = 0;
@@ -1892,12 +1918,13 @@ int sph_create(const sph_params* prm, void** out) {
     if (q.precision != SPH_PREC_FP64) {
         if ((rc = alloc_state<float>(*c, c->s32))) return cleanup(rc == SPH_ERR_CUDA ? SPH_ERR_NOMEM : rc);
         c->has32 = true;
+        if ((rc = alloc_err(*c))) return cleanup(rc);
     }
     if ((rc = set_fused_attrs())) return cleanup(rc);
     {
         int dev = 0, sms = 0, per_sm = 0;
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<SPH, 1>, SW_NT, sweep_smem_bytes()) == cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<SPH, 1, false>, SW_NT, sweep_smem_bytes()) == cudaSuccess)
             c->fused_slots = sms * per_sm;
         if (sms > 0) c->sms = sms;
         cudaGetLastError();
@@ -2783,6 +2810,7 @@ static int corr_access(void* h, int32_t field, double* host, const double* src, 
     if (rc) return rc;
     float* dev = c->s32.f[slot];
     if (src) c->ghost_stored = true;  // the caller's boundary velocities need not satisfy the BCs
+    if (src && (slot == F_ETA || slot == F_ETA_SM)) set_small32(*c, true);  // (of any size)
     return host ? download_box<float>(*c, dev, e, host) : upload_box<float>(*c, dev, e, src);
 }
 
@@ -2800,10 +2828,7 @@ int sph_selftest_wait_flag(void* h) {
     Ctx* c = static_cast<Ctx*>(h);
     if (!c) return fail(SPH_ERR_INVALID, "ctx is NULL");
     if (int rc_ = usable(*c)) return rc_;
-    if (!c->d_err) {
-        if (cudaMalloc((void**)&c->d_err, sizeof(int)) != cudaSuccess) return fail(SPH_ERR_NOMEM, "error word");
-        CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    }
+    if (int rc_ = alloc_err(*c)) return rc_;
     // 1000 polls of at most 1 us each: the wait runs out within a few milliseconds
     k_wait_selftest<<<1, 32, 0, c->stream>>>(c->d_err, 1000, 1000u);
     CK(cudaGetLastError());
