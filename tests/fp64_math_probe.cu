@@ -1,4 +1,4 @@
-// Element-wise access to the FP64 primitives of sph_math.cuh for test_fp64_math_gpu.py.
+// Element-wise access to the primitives of sph_math.cuh, and the FP32 quotient of the ghost stencils, for test_fp64_math_gpu.py.
 #include "sph_math.cuh"
 
 using namespace sph;
@@ -11,6 +11,7 @@ __global__ void k_probe(int op, long long n, const double* a, const double* b, d
         case 0: out[i] = near_div(x, y); break;
         case 2: out[i] = fast_sqrt(x); break;
         case 3: out[i] = fast_pow(tab, x, c); break;
+        case 5: out[i] = gdiv((float)x, (float)y); break;
         default: {
             const double e = (double)p / q;
             out[i] = root_pow(x, p, q, (q + 1.0) / (q - 1.0), (float)e, (float)(e - (double)(float)e));

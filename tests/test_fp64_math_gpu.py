@@ -81,6 +81,15 @@ def test_near_div_of_any_operand(probe):
         np.testing.assert_array_equal(np.signbit(probe(0, a, b))[~np.isnan(a / b)], np.signbit(a / b)[~np.isnan(a / b)])
 
 
+@pytest.mark.parametrize("lo,hi", [(-1, 1), (-20, 20), (-60, 60)])
+def test_ghost_quotient_is_the_ieee_quotient(probe, lo, hi):
+    """FP32: the error of the reciprocal, 2^-23, squared by the residual step: 2^-46 before the last rounding, so that one
+    pair in 2^21 may differ"""
+    rng = np.random.default_rng(6)
+    a, b = numbers(rng, lo, hi).astype(np.float32), numbers(rng, lo, hi).astype(np.float32)
+    nearly_ieee(probe(5, a, b).astype(np.float32), a / b, 4)
+
+
 @pytest.mark.parametrize("lo,hi", [(-1, 1), (-30, 30), (-1000, 1000)])
 def test_fast_sqrt_is_the_ieee_root(probe, lo, hi):
     a = numbers(np.random.default_rng(2), lo, hi)
