@@ -78,17 +78,12 @@ struct KP {
 
 // Programmatic dependent launch: wait until the preceding grid of the stream has
 // completed and its writes are visible (returns at once for a launch without a
-// programmatic dependency), then allow the next grid of the stream to be
-// scheduled, so its launch overlaps this grid instead of following it.
+// programmatic dependency)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() {
-    pdl_wait();
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
 
-// The same where the next grid is large and bound by its fullest SM: released early only from a grid of a
-// few blocks, as blocks placed beside running ones are spread unevenly over the SMs (spherical 63^3, FP64: 194 us
-// an iteration with early release throughout, 125 with this).
+// ... then allow the next grid of the stream to be scheduled, so its launch overlaps this grid instead of following it:
+// only from a grid of a few blocks, as blocks placed beside running ones are spread unevenly over the SMs (spherical
+// 63^3, FP64: 194 us an iteration with early release throughout, 125 with this).
 __device__ __forceinline__ void pdl_enter_small() {
     pdl_wait();
     if (gridDim.x * gridDim.y * gridDim.z <= 64u) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

@@ -14,9 +14,7 @@
 
 namespace sph {
 
-// division of the stress / pseudo-step updates: IEEE in FP64, the fast
-// intrinsic in FP32 (operands are O(1)-scaled viscosities and steps)
-__device__ __forceinline__ double pdiv(double a, double b) { return a / b; }
+// FP32 division of the stress / pseudo-step updates: the fast intrinsic (FP64: mid_div, near_div of sph_math.cuh)
 __device__ __forceinline__ float pdiv(float a, float b) { return __fdividef(a, b); }
 
 template <typename T>

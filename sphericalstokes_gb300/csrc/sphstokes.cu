@@ -125,12 +125,11 @@ struct Ctx {
     float* map_key[4][2] = {};           // V1 and η buffers of the arrangement a set was built for
     int* d_err = nullptr;                // set by a kernel whose bounded wait ran out
     bool use_tma = true;
-    bool use_pdl = true;  // sweep and BC kernels launched with a programmatic dependency (pdl_enter)
+    bool use_pdl = true;  // sweep and BC kernels launched with a programmatic dependency (pdl_wait)
     bool fused = true;   // FP32 sweeps use the fused kernel
     int fused_chunk = 0; // planes per block of the fused sweep (0: chosen by fused_chunk())
     bool chunk_fixed = false;  // by SPH_FUSED_CHUNK: in batches too
     int sms = 152;
-    int fused_slots = 0; // resident blocks of the fused TMA sweep on the device (SMs x blocks per SM)
     double* adj = nullptr;  // adjoint arrays (AJ_STATE slots of the box), allocated on first use
     // per-launch timing of the fused sweep kernel (sph_sweep_profile): event pairs
     // recorded around each launch while prof_next < prof_ev.size()/2
@@ -248,7 +247,7 @@ KP<T> make_kp(Ctx& c, State<T>& s) {
 dim3 blk2d() { return dim3(32, 8, 1); }
 
 // launch with a programmatic dependency on the preceding grid of the stream (the
-// kernel starts with pdl_enter()); a plain launch when PDL is switched off
+// kernel waits, pdl_wait, before it touches what an earlier grid writes or reads); a plain launch when PDL is switched off
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -1922,11 +1921,8 @@ int sph_create(const sph_params* prm, void** out) {
     }
     if ((rc = set_fused_attrs())) return cleanup(rc);
     {
-        int dev = 0, sms = 0, per_sm = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<SPH, 1, false>, SW_NT, sweep_smem_bytes()) == cudaSuccess)
-            c->fused_slots = sms * per_sm;
-        if (sms > 0) c->sms = sms;
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) c->sms = sms;
         cudaGetLastError();
     }
     if (const char* e = std::getenv("SPH_NO_GRAPHS")) c->use_graphs = std::atoi(e) == 0;
