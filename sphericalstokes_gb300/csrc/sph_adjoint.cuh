@@ -13,9 +13,10 @@
 // λ_V with Eᵀ μ: the coupling products are the transposes of the forward ones.
 //
 // Every kernel gathers: a thread owns the entries it writes and reads the adjoints that reach them, so
-// there are no atomics and no clearing of accumulators.  The kernels march along x3 like those of
+// there are no atomics and no clearing of accumulators; but for the transposed stress ghosts
+// (k_bc_adjoint, BC_STRESS), which scatter to neighbours with FP64 atomics.  The kernels march along x3 like those of
 // sph_march.cuh and are bound the same way, by FP64 instructions; the factors that stay fixed
-// during a solve (rates, stiffnesses, the state's strain rates over the viscosity, the law's
+// during a solve (rates, stiffnesses, the state's strain rates, the law's
 // derivative) are made once by k_adj_setup.
 //   k_adj_stress   λ_V -> adjoint of σ, τ (cells, edges), of P; MEM: μ and λ_P updated
 //   k_adj_eta      per cell λᵀ ∂R/∂η (and, for the law, that times dη_t/dε̇)

@@ -9,8 +9,8 @@
 //   k_nodes    compute_V!                        :267-329   (sph_march.cuh)
 //   k_bc       BC_R! / BC_θ! / BC_φ! and the cyl/cart BC kernels, all stages
 // All three coordinate systems share the kernels; the metric terms come from
-// the template parameter G and the 1D tables in Geo.  The FP32 fused sweep in
-// sph_fused.cuh implements the same arithmetic with shared-memory tiling.
+// the template parameter G and the 1D tables in Geo.  The FP32 fused sweeps in
+// sph_sweep.cuh and sph_fused.cuh implement the same arithmetic with shared-memory tiling.
 #pragma once
 #include "sph_core.cuh"
 

@@ -18,14 +18,15 @@
 // * Issue slots.  A thread owns a pair of points, so arithmetic is FFMA2 / FADD2 /
 //   FMUL2, shared-memory and global accesses are 8 bytes wide, and the per-plane
 //   bookkeeping is shared by two cells.  A difference a - b is one FFMA2 with the
-//   constant -1 (a paired add cannot negate an operand).  What plane K+1 contributes
-//   to the stencils of plane K is what plane K+1 needs of itself at the next step:
-//   13 pairs (face velocities, sums of η and ηSM over two cells) are carried in
-//   registers and each input plane is read from shared memory once.
-// * Copies in flight.  Because of the carry an input slot is free as soon as stage 1
-//   of a plane is done, so two slots keep one to two planes (40 KB each) in flight;
-//   the warp that computes the halo points has no velocities to update and issues
-//   them (7 four-dimensional boxes per plane: fields of a slab are equally spaced).
+//   constant -1 (a paired add cannot negate an operand).  Of η and ηSM, what plane K+1
+//   contributes to the stencils of plane K is what it needs of itself at the next step:
+//   the pair's values and their sums over two cells (6 pairs) are carried in registers, with
+//   the stresses of plane K that the velocities of plane K+1 want, and each plane of η and
+//   ηSM is read from shared memory once; the velocities of a plane are read at both steps.
+// * Copies in flight.  Stage 1 of plane K reads the input slots of planes K and K+1, so that
+//   three slots (12.5 KB each) keep one to two planes in flight, with the old state and the
+//   right-hand sides in two (22 KB each); the warp that computes the halo points has no velocities to
+//   update and issues them (7 four-dimensional boxes per plane: fields of a slab are equally spaced).
 // * 14 rows, because 7 warps of owned points and one of halo points (31 pairs) make four
 //   warps per scheduler at two blocks per SM, which leaves 128 registers to each thread:
 //   16 rows need a ninth warp, five warps on some schedulers, 96 registers and spills.
@@ -37,7 +38,7 @@
 // Measured on a GB300, us per sweep with its boundary velocities (before: one cell per
 // thread, 32 x 8 tiles, 30 warps per SM, x2 / x3 ghosts by two to four BC launches):
 // 255^3 304 (375; 5.7 TB/s of the algorithmic bytes, 0.85 of the copy rate),
-// 511 x 255 x 255 with a free surface 607 (732), 131 x 117 x 101 44.5 (65.0),
+// 511 x 255 x 255 with a free surface 607 (732), 131 x 117 x 101 44.1 (65.0),
 // 63^3 11.8 (19.1), 47 x 31 x 39 Cartesian 6.2 (14.5).  At 255^3 300 warp instructions
 // per 32 cells (608).  The same copies and stores without the arithmetic take 285 us
 // (the tiles' halos and 10 + 10 streams cost 10 % of the copy rate): memory bound there.  The
@@ -237,8 +238,7 @@ __device__ __forceinline__ SweepCoef sweep_coef(const Geo<float>& geo, float d2,
     return c;
 }
 
-// Boundary work of the sweep, out of line: few points run it and the march stays small.
-//
+// Boundary work of the sweep, which few points run:
 // the divergence-free ghosts (smask) of cell (x, y, k) among its six face velocities v; the cell's
 // metric from its sweep coefficients (exact: they are powers of two times the metric factors)
 template <int G>

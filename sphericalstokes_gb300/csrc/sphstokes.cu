@@ -229,9 +229,13 @@ KP<T> make_kp(Ctx& c, State<T>& s) {
     p.g = T(q.g);
     p.tau_C = T(q.tau_C); p.n_exp = T(c.cur_n); p.relax = T(q.relax); p.edot_bg = T(q.edot_bg);
     const bool ed = q.rheology == SPH_RHEO_EDOT_POWER_RELAX;
-    p.law_i2 = T(ed ? 1.0 / (q.edot_bg * q.edot_bg) : 1.0 / (q.tau_C * q.tau_C));
+    // a scale whose square leaves the range: squared ratios of zero, which the laws take from the ratio itself
+    const double scale = ed ? q.edot_bg : q.tau_C;
+    const bool square = std::fabs(scale) > 0x1p-500 && std::fabs(scale) < 0x1p500;
+    p.law_i2 = square ? T(1.0 / (scale * scale)) : T(0);
     p.law_ex = T(0.5 * (c.cur_n - 1.0) / (ed ? c.cur_n : 1.0));
     power_form(ed, c.cur_n, &p.law_p, &p.law_q);
+    if (!square) p.law_p = p.law_q = 0;
     p.law_i1 = T(1.0 / q.tau_C);
     p.law_e = (float)p.law_ex; p.law_el = (float)(0.5 * (c.cur_n - 1.0) / (ed ? c.cur_n : 1.0) - p.law_e);
     p.law_rho = p.law_q > 1 ? T(p.law_q + 1) / T(p.law_q - 1) : T(0);

@@ -76,7 +76,7 @@ def velocities(rng, scale):
 
 @pytest.mark.parametrize("relax", [0.3, 0.5, 1.0])
 @pytest.mark.parametrize("n_exp", [1.0, 1.7, 2.0, 3.0, 4.0, 5.0, 6.0])
-@pytest.mark.parametrize("edot_bg", [0.25, 1e-15, 1e20])
+@pytest.mark.parametrize("edot_bg", [0.25, 1e-15, 1e20, 1e-158, 1e160])
 def test_strain_rates_over_the_range(n_exp, relax, edot_bg):
     rng = np.random.default_rng(1)
     p = edot_params(n_exp, relax, edot_bg)
@@ -105,7 +105,8 @@ def test_old_and_target_viscosity_far_apart(n_exp, relax, pair):
 
 
 @pytest.mark.parametrize("n_exp", [1.5, 2.0, 2.5, 3.0])
-@pytest.mark.parametrize("scale,tau_C", [(0.0, 1.3), (1e-130, 1e30), (1e-130, 1.0), (1.0, 1.3), (1e130, 1.3), (1e130, 1e-30)])
+@pytest.mark.parametrize("scale,tau_C", [(0.0, 1.3), (1e-130, 1e30), (1e-130, 1.0), (1.0, 1.3), (1e130, 1.3), (1e130, 1e-30),
+                                         (0.0, 1e-170), (0.0, 1e170), (1e-130, 1e-170), (1e-140, 1e-160), (1e140, 1e160), (1e150, 1e156)])
 def test_stresses_over_the_range(n_exp, scale, tau_C):
     rng = np.random.default_rng(3)
     p = S.default_params("spherical", n1=N[0], n2=N[1], n3=N[2], rheology="tau_power", n_exp=n_exp, tau_C=tau_C, init="none")
@@ -122,3 +123,22 @@ def test_stresses_over_the_range(n_exp, scale, tau_C):
     # (power_law! takes 1/eta_PL: infinite, and eta zero, where eta_PL = eta_ini / power is below 1 / the largest double)
     gone = power / ini > X(np.finfo(np.float64).max)
     check(got, np.where(gone, X(0), X(2) * ini.astype(X) / (X(1) + power)))
+
+
+@pytest.mark.parametrize("n_exp", [2.0, 2.5, 3.0, 5.0])
+@pytest.mark.parametrize("scale,tau_C", [(1.0, 1.3), (1e-130, 1e-160), (1e140, 1e158), (1e150, 1e156)])
+def test_relaxed_stresses_over_the_range(n_exp, scale, tau_C):
+    rng = np.random.default_rng(4)
+    relax = 0.3
+    p = S.default_params("cylindrical", n1=N[0], n2=N[1], n3=N[2], rheology="tau_power_relax", n_exp=n_exp, relax=relax, tau_C=tau_C, init="none")
+    with S.Solver(p) as sv:
+        for f in ("TAU11", "TAU22", "TAU33", "TAU12", "TAU13", "TAU23"):
+            sv.set(f, scale * rng.standard_normal(sv.dims(f)))
+        ini, old = (np.exp(rng.standard_normal(N)) for _ in range(2))
+        for f, a in (("ETA", ini), ("ETA_INI", ini), ("ETA_PL", old), ("PHASE", np.zeros(N))):
+            sv.set(f, a)
+        sv.power_law()
+        tii, got, pl = sv.get("TII"), sv.get("ETA"), sv.get("ETA_PL")
+    want = (ini.astype(X) * (tii.astype(X) / X(tau_C)) ** (X(1) - X(n_exp))) ** X(relax) * old.astype(X) ** (X(1) - X(relax))
+    check(pl, want)
+    check(got, X(2) / (X(1) / ini.astype(X) + X(1) / want))
