@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(MC_NT, cells_blocks(WHAT)) k_cells(const __gri
     // whether the quotients of this column may be formed by mid_div: its steps, and η and ηSM of the plane below
     bool steps = true, below = true;
     if (PT) {
-        MidRange<T, 60> m;
+        MidRange<T, 100> m;
         m.add(p.gsc); m.add(p.kbc); m.add(p.vpdt2);
         steps = m.ok();
     }
