@@ -22,8 +22,8 @@
 //   k_adj_eta      per cell λᵀ ∂R/∂η (and, for the law, that times dη_t/dε̇)
 //   k_adj_collect, k_adj_law   the law's dependence on V added to the adjoints of the strain rates
 //   k_adj_strain   adjoints of strain rates and div V -> V (all entries)
-// Measured on a GB300, 63^3 sector under the strain-rate law: 114 us per transposed iteration (820 with
-// scatters by FP64 atomics and coefficients evaluated as stencils of unit vectors), the FP64 units 63 - 78 %
+// Measured on a GB300, 63^3 sector under the strain-rate law: 118 us per transposed iteration (820 with
+// scatters by FP64 atomics and coefficients evaluated as stencils of unit vectors), the FP64 units 56 - 77 %
 // busy in the cell and node kernels; the rest is the five BC stages and launches.
 #pragma once
 #include "sph_march.cuh"

@@ -16,9 +16,9 @@
 // direct: neighbours come from L1, and their issue slots are free beside FP64 at 1/16 of a warp
 // instruction per clock.
 // Measured on a GB300, 127^3 sector, strain-rate law, us (FP64 operations per cell): k_cells with the strain
-// rates kept 379 (97), k_edot 208 (54, before the roots of root_pow), k_nodes 205 (52), each with the FP64 units
-// 86 - 88 % busy; one point per thread, with separate strain-rate kernel and CUDA's pow, exp and log: compute_P! 537,
-// strain rates 223, law 642, compute_V! 310.  An iteration 757 (2071); Cartesian 207^3, relaxed stress law 3085 (7030).
+// rates kept 385 (98), k_nodes_law 352 (93), both with the FP64 units 87 % busy (spherical 63^3 73 and 84 %); one point per
+// thread, with separate strain-rate kernel and CUDA's pow, exp and log: compute_P! 537, strain rates 223, law 642,
+// compute_V! 310.  An iteration 765 (2071); Cartesian 207^3, relaxed stress law 3118 (7030).
 #pragma once
 #include "sph_math.cuh"
 

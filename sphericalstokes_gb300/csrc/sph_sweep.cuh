@@ -39,7 +39,7 @@
 // thread, 32 x 8 tiles, 30 warps per SM, x2 / x3 ghosts by two to four BC launches):
 // 255^3 304 (375; 5.7 TB/s of the algorithmic bytes, 0.85 of the copy rate),
 // 511 x 255 x 255 with a free surface 607 (732), 131 x 117 x 101 44.1 (65.0),
-// 63^3 11.8 (19.1), 47 x 31 x 39 Cartesian 6.2 (14.5).  At 255^3 300 warp instructions
+// 63^3 11.8 (19.1), 47 x 31 x 39 Cartesian 6.2 (14.5).  At 255^3 316 warp instructions
 // per 32 cells (608).  The same copies and stores without the arithmetic take 285 us
 // (the tiles' halos and 10 + 10 streams cost 10 % of the copy rate): memory bound there.  The
 // smallest grids are one wave of blocks: the latency of a few planes and the launch.
