@@ -295,16 +295,20 @@ __device__ __forceinline__ void edot_body(const KP<double>& p, int chunk, int by
         const double ei = p.eta_ini[c], eo = RELAXED ? p.eta[c] : ei, w = x * p.law_i2;
         const bool lin = p.phase && p.phase[c], half = p.relax == 0.5;
         double et = ei;
+        const bool rest = __double_as_longlong(x) == 0, root = root_range(w);
         MidRange<double, 400> mid;
         mid.add(ei); mid.add(eo);
-        if (p.law_q && (half || !RELAXED) && mid.ok() && root_range(w)) {  // (every intermediate value is a normal number)
-            if (!lin) et = mid_div(ei + ei, 1.0 + root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el));
+        if (p.law_q && (half || !RELAXED) && mid.ok() && (root || rest)) {  // (every intermediate value is a normal number, or zero)
+            double f = 0.0;
+            if (root) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
+            if (!lin) et = mid_div(ei + ei, 1.0 + f);
             if (RELAXED) et = mid_sqrt(eo * et);
         } else {
             if (!lin) {
                 double f;
-                if (p.law_q && root_range(w)) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
+                if (p.law_q && root) f = root_pow(w, p.law_p, p.law_q, p.law_rho, p.law_e, p.law_el);
                 else if (normal_pos(w)) f = fast_pow(tab, w, p.law_ex);
+                else if (rest && p.law_ex > 0.0) f = 0.0;
                 else f = pow(sqrt(x) / p.edot_bg, 2.0 * p.law_ex);  // (the square of the ratio leaves the range first)
                 et = near_div(ei + ei, 1.0 + f);
             }
@@ -371,7 +375,10 @@ __device__ __forceinline__ void rheo_body(const KP<double>& p, int faces_only, i
         const double w = p.law_q ? small_pow(tii * p.law_i1, x, lin ? 0 : p.law_p) : 0.0;
         if (!RELAX) {
             double f = w;
-            if (!p.law_q) f = normal_pos(x) ? fast_pow(tab, x, cx) : pow(tii / p.tau_C, 2.0 * cx);  // (as in edot_body)
+            if (!p.law_q) {  // (as in edot_body)
+                if (normal_pos(x)) f = fast_pow(tab, x, cx);
+                else f = __double_as_longlong(t2) == 0 && cx > 0.0 ? 0.0 : pow(tii / p.tau_C, 2.0 * cx);
+            }
             p.eta[c] = near_div(ei + ei, 1.0 + f);
         } else {
             const double po = p.eta_pl[c];
